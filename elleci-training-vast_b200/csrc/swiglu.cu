@@ -24,7 +24,8 @@ using namespace rowio;
 
 // e^t in float32 for the sigmoid: t clamped to [-87, 87] (beyond it 1 + e^t no longer changes, or the sigmoid is below
 // 2e-38), n = round-half-even(t*log2(e)) taken by adding and subtracting 1.5*2^23 (its low mantissa bits are n as an
-// integer), r = t - n*ln2 in two fused steps, degree-7 Taylor polynomial in Horner form with fused multiply-adds, times
+// integer), r = t - n*ln2 in two fused steps (ln2 in the two parts that
+// Moshier's Cephes library uses), degree-7 Taylor polynomial in Horner form with fused multiply-adds, times
 // 2^n built in the exponent field.  About 1 ulp.  A NaN argument is clamped away (fmaxf returns the other operand); the
 // callers multiply by the argument afterwards, which brings the NaN back.
 __device__ __forceinline__ float exp_fixed(float t) {
@@ -46,18 +47,18 @@ __device__ __forceinline__ float exp_fixed(float t) {
     return __fmul_rn(p, scale);
 }
 
-// 1/d correctly rounded for a d whose reciprocal is a normal number (here d = 1 + e^t lies in [1, 2^126]): the hardware
-// approximation and one Newton step in two fused multiply-adds - the general-purpose reciprocal is this sequence plus a
-// check and a branch for the arguments that cannot occur here.
-__device__ __forceinline__ float rcp_normal(float d) {
-    float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
-    const float e = __fmaf_rn(-d, r, 1.0f);
-    return __fmaf_rn(r, e, r);
+// 1/d correctly rounded for d in [1, 2^126] (here d = 1 + e^t): with r0 the hardware approximation and e = 1 - d*r0 (exact
+// in one fused multiply-add up to the last place), 1/d = r0/(1 - e) = r0*(1 + e + e^2 + ...), the geometric series; its
+// first three terms leave an error of e^3 < 2^-66.  Compared with __frcp_rn over every mantissa and every exponent of that range.
+__device__ __forceinline__ float rcp_series(float d) {
+    float r0;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"(d));
+    const float e = __fmaf_rn(-d, r0, 1.0f);
+    return __fmaf_rn(r0, __fmaf_rn(e, e, e), r0);
 }
 
 // sigmoid(g) = 1 / (1 + e^-g)
-__device__ __forceinline__ float sigmoid_fixed(float g) { return rcp_normal(__fadd_rn(1.0f, exp_fixed(-g))); }
+__device__ __forceinline__ float sigmoid_fixed(float g) { return rcp_series(__fadd_rn(1.0f, exp_fixed(-g))); }
 
 // Eight elements of the gate: sig = sigmoid(g), s = io(g * sig), h = io(s * u) - silu rounded to the I/O type, then the
 // product rounded to the I/O type, as the two tensor operations of the reference round them.
