@@ -19,7 +19,7 @@
 // 128 output columns k per CTA).  DX expands without the final byte interleave (decode16_deint), which permutes the
 // output columns inside groups of 16; the epilogue undoes that while the sums are in registers.
 // The leader commits each stage to the "empty" barriers of both CTAs and each tile to both "tmem_full" barriers; no
-// cluster-multicast load or commit is used.  Every mbarrier wait is bounded (tc_ptx.cuh).
+// cluster-multicast load is used.  Every mbarrier wait is bounded (tc_ptx.cuh).
 #include "common.cuh"
 #include "epilogue.cuh"
 #include "tc_ptx.cuh"
@@ -110,11 +110,13 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     //   full   (leader's copy is used) one phase = both CTAs' A tiles landed (transaction bytes) + both halves expanded
     //          (one arrival per CTA's transform warp) + the leader producer's expect-arrival
     //   empty  (local) the MMAs that read stage s have completed
-    // With every data movement and every MMA removed, the handshakes of this kernel alone took more than half of its time
-    // when the MMA-issuing thread waited on two barriers and made four commits per block; it now waits on ONE barrier and
-    // makes TWO commits per block (one per CTA).  Passing the peer's release through the leader's producer instead of a
-    // second commit was tried and lost a third of the throughput: the handshake chain is latency-bound, and the relay
-    // added a hop to it.
+    // The kernel is bound by the latency of this handshake chain, so the MMA-issuing thread waits on ONE barrier and makes
+    // ONE commit per block, which arrives on both CTAs' "empty" barriers, and arrivals across the pair carry no wider memory
+    // ordering than they need (tc_ptx.cuh).  Passing the peer's release through the leader's producer was tried and lost a
+    // third of the throughput: the relay added a hop to the chain.
+    // 4096 tokens, 4096 -> 11008 / 11008 -> 4096, bf16 out, L2 flushed: forward 157 / 173 us with two commits, cluster-scope
+    // arrivals and block coordinates divided out per block; 137 / 140 us now
+    // (2700 / 2640 TOP/s); dX 169 / 155 -> 138 / 134 us.  (Two boxes; the faster one gave 133 / 136 and 136 / 131.)
     auto bar_full = [&](int s) { return bars + 8u * s; };
     auto bar_empty = [&](int s) { return bars + 8u * (DA + s); };
     static_assert(DA == DB, "the A and B rings advance in lockstep");
@@ -198,16 +200,12 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                             const uint64_t db = (MODE == MODE_FWD) ? make_desc(b_addr + k * 32, 16) : make_desc(b_addr + k * 4096, 16384);
                             umma_i8_pair(d_tmem, da, db, idesc, (kb | k) != 0);
                         }
-                        umma_commit_pair(mapa_u32(bar_empty(s), 0));
-                        umma_commit_pair(mapa_u32(bar_empty(s), 1));
+                        umma_commit_pair(bar_empty(s));
                     }
                     __syncwarp();
                     if (++s == DA) { s = 0; ph ^= 1u; }
                 }
-                if (!failed && lane == 0) {
-                    umma_commit_pair(mapa_u32(bar_tfull(acc), 0));
-                    umma_commit_pair(mapa_u32(bar_tfull(acc), 1));
-                }
+                if (!failed && lane == 0) umma_commit_pair(bar_tfull(acc));
                 __syncwarp();
             }
         }
@@ -331,12 +329,21 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         const int my_items = (num_items > pair) ? (num_items - pair + num_pairs - 1) / num_pairs : 0;
         const long long total = (long long)my_items * p.kbp;
         const uint4 zero_codes = make_uint4(0x55555555u, 0x55555555u, 0x55555555u, 0x55555555u);     // sixteen weights 0 per word
-        auto load_block = [&](long long g, uint4 (&pk)[8]) {
-            const int i = (int)(g / p.kbp);
-            int trow, tcol, part, kb0;
-            item_coords(pair + i * num_pairs, num_tiles, p, trow, tcol, part, kb0);
-            const int kb = kb0 + (int)(g - (long long)i * p.kbp);
-            const int c0 = tcol * BN + (int)rank * 128;             // this CTA's 128 output columns
+        // The loads run through this warp's blocks in order, six reduction blocks apart: the item and the block inside it are
+        // carried forward, so that only a new item costs divisions.
+        int ld_item = pair, ld_kb = xw, ld_kb0 = 0, ld_c0 = 0;
+        auto set_item = [&]() {
+            while (ld_kb >= p.kbp) { ld_kb -= p.kbp; ld_item += num_pairs; }
+            if (ld_item < num_items) {
+                int trow, tcol, part;
+                item_coords(ld_item, num_tiles, p, trow, tcol, part, ld_kb0);
+                ld_c0 = tcol * BN + (int)rank * 128;                // this CTA's 128 output columns
+            }
+        };
+        set_item();
+        auto load_next = [&](uint4 (&pk)[8]) {
+            const int kb = ld_kb0 + ld_kb, c0 = ld_c0;
+            ld_kb += NUM_XF_WARPS;
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
                 const int item = lane + 32 * j, row = item >> 1, seg = item & 1;
@@ -351,17 +358,18 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                 }
                 pk[j] = ok ? __ldg(reinterpret_cast<const uint4*>(src)) : zero_codes;
             }
+            if (ld_kb >= p.kbp) set_item();
         };
         uint4 cur[8], nxt[8];
-        if (xw < total) load_block(xw, cur);
-        for (long long g = xw; g < total && !failed; g += NUM_XF_WARPS) {
+        uint32_t phb = 0;                   // phase of this warp's slot: one block after the other
+        if (xw < total) load_next(cur);
+        for (long long g = xw; g < total && !failed; g += NUM_XF_WARPS, phb ^= 1u) {
             // Block g uses this warp's own B slot (g % 6 == xw).  A barrier only tells the parity of its phase, so a
             // waiter must never be two phases away from it: with one slot per warp the previous use of the slot was this
             // warp's previous block (g-6).
             const bool more = g + NUM_XF_WARPS < total;
-            if (!LEAN && more) load_block(g + NUM_XF_WARPS, nxt);        // a whole block ahead, into the second image
+            if (!LEAN && more) load_next(nxt);        // a whole block ahead, into the second image
             const int sb_i = xw;
-            const uint32_t phb = (uint32_t)(g / DB) & 1u;
             if (!mbar_wait_warp(bar_empty(sb_i), phb ^ 1u, p.status, 28)) { failed = true; break; }
             uint8_t* sb = smem_gen + DA * A_BYTES + sb_i * B_BYTES;
 #pragma unroll
@@ -380,7 +388,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             }
             if (LEAN) {
                 asm volatile("" ::: "memory");  // keeps the compiler from starting the next loads while `cur` is still needed
-                if (more) load_block(g + NUM_XF_WARPS, cur);        // into the one image, as soon as it is free
+                if (more) load_next(cur);        // into the one image, as soon as it is free
             }
             fence_async_smem();
             __syncwarp();
