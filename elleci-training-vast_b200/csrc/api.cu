@@ -20,6 +20,8 @@ int launch_quantize_grad(const void* dY, int dt, long long ld, const float* xa, 
 int launch_hysteresis(const float* dW, uint8_t* Wp, uint8_t* Hp, const HystParams& p, int N, int K, uint32_t idx_base,
                       cudaStream_t st);
 int launch_gemm_simple(int mode, const int8_t* A, const void* B, int R, int C, int D, const EpiParams& epi, cudaStream_t st);
+bool gemm_skinny_fits(int mode, const void* A, const void* B, int R, int C, int D, const EpiParams& epi);
+int launch_gemm_skinny(int mode, const int8_t* A, const void* B, int R, int C, int D, const EpiParams& epi, cudaStream_t st);
 int gemm_tc_eligible(int mode, const void* A, const void* B, int R, int C, int D);
 int launch_gemm_tc(int mode, const int8_t* A, const void* B, int R, int C, int D, const EpiParams& epi, int32_t* status,
                    cudaStream_t st);
@@ -154,6 +156,9 @@ static int gemm_dispatch(int mode, const int8_t* A, const void* B, int R, int C,
     // once, which the CUDA-core kernel takes twenty times longer for.
     if (elig == EL_OK && (R >= 32 || (long long)C * D >= (1ll << 18)))
         return launch_tc(mode, R <= 128, A, B, R, C, D, epi, status, st, ws, ws_bytes, lean);
+    // layers of 16, 32 or 48 inputs: streaming kernels (see gemm_skinny.cu for both sides' times); a column count that no vector
+    // store takes, an odd reduction or unaligned operands stay with the CUDA-core kernel
+    if (elig != EL_OK && gemm_skinny_fits(mode, A, B, R, C, D, epi)) return launch_gemm_skinny(mode, A, B, R, C, D, epi, st);
     return launch_gemm_simple(mode, A, B, R, C, D, epi, st);
 }
 
