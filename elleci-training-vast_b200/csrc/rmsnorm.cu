@@ -151,9 +151,9 @@ rmsnorm_quantize_rows_kernel(const T* __restrict__ x, long long ldx, const float
 // weight rounded once and kept in registers.  A thread owns 64 bytes of every row, so that the warp reductions and the scalar
 // arithmetic of a row are spread over many elements, and several CTAs share an SM, so that one's barriers hide behind the
 // others' work.  Products of two values of a 16-bit I/O type are taken packed (one rounding, the same result), and the
-// quantiser rounds by adding 1.5*2^23 instead of converting.  What bounds it: about 15 instructions per element and one
+// quantiser rounds by adding 1.5*2^23 instead of converting.  What bounds it: about 20 instructions per element and one
 // float64 conversion; memory 3 bytes per element (bf16).
-// 4096 tokens x 11008, bf16: 76 us in the one-CTA-per-row form, 55 us in this one; x 4096: 27 -> 22.5 us (events around
+// 4096 tokens x 11008, bf16: 76 us in the one-CTA-per-row form, 47 us in this one; x 4096: 27 -> 20.5 us (events around
 // the call, L2 flushed).
 constexpr int FW_STAGES = 2;
 template <typename T> constexpr int FW_VECS = 8 / (int)sizeof(T);        // vectors of 8 per thread: 4, float32: 2
@@ -169,12 +169,13 @@ rmsnorm_quantize_stream_kernel(const T* __restrict__ x, long long ldx, const flo
     __shared__ double red_d[2][MAX_RED];
     __shared__ uint32_t red_u[2][MAX_RED];
     __shared__ uint32_t red_f[2][MAX_RED];
-    const Slots<T, V> slots{ring};
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, TT = blockDim.x;
+    const Slots<T, FW_STAGES, V> slots(ring);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const f32x2 nz = negative_zeros();
     typename Io<T>::Raw w[V];
 #pragma unroll
     for (int c = 0; c < V; ++c) {
-        const int k = (tid + c * TT) * 8;
+        const int k = column_of<V>(c);
         float wv[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
         if (k < K) load8_w(weight + k, wv);
         w[c] = Io<T>::pack(wv);                      // rounds to the I/O type
@@ -183,7 +184,7 @@ rmsnorm_quantize_stream_kernel(const T* __restrict__ x, long long ldx, const flo
         if (m < M) {
 #pragma unroll
             for (int c = 0; c < V; ++c) {
-                const int k = (tid + c * TT) * 8;
+                const int k = column_of<V>(c);
                 if (k < K) slots.fetch(stage, c, x + (size_t)m * ldx + k);
             }
         }
@@ -201,16 +202,10 @@ rmsnorm_quantize_stream_kernel(const T* __restrict__ x, long long ldx, const flo
         double ss = 0.0;
 #pragma unroll
         for (int c = 0; c < V; ++c) {
-            row[c] = (tid + c * TT) * 8 < K ? slots.read(stage, c) : raw_zero<T>();
-            float v[8];
-            Io<T>::unpack(row[c], v);
-            double a = 0.0, b = 0.0;
-#pragma unroll
-            for (int i = 0; i < 8; i += 2) {
-                a += (double)__fmul_rn(v[i], v[i]);
-                b += (double)__fmul_rn(v[i + 1], v[i + 1]);
-            }
-            ss += a + b;
+            row[c] = column_of<V>(c) < K ? slots.read(stage, c) : raw_zero<T>();
+            f32x2 v[4];
+            unpack2<T>(row[c], v);
+            ss += dot8(v, v);
         }
         ss = warp_sum(ss);
         if (lane == 0) red_d[stage][warp] = ss;
@@ -221,14 +216,15 @@ rmsnorm_quantize_stream_kernel(const T* __restrict__ x, long long ldx, const flo
         const float r = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(ms, norm_eps)));
         // ---- y = io(io(x*r) * io(w)) and its largest magnitude ------------------------------------------------------------
         uint32_t top = 0u;
+        const f32x2 r2 = pair(r, r);
 #pragma unroll
         for (int c = 0; c < V; ++c) {
-            float v[8];
-            Io<T>::unpack(row[c], v);
+            f32x2 v[4];
+            unpack2<T>(row[c], v);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) v[i] = __fmul_rn(v[i], r);
-            row[c] = mul_raw(Io<T>::pack(v), w[c]);
-            if ((tid + c * TT) * 8 < K) top = max_bits(top, row[c]);
+            for (int i = 0; i < 4; ++i) v[i] = mul2(v[i], r2);
+            row[c] = mul_raw(pack2<T>(v), w[c]);
+            if (column_of<V>(c) < K) top = max_bits(top, row[c]);
         }
         top = __reduce_max_sync(0xffffffffu, magnitude_bits<T>(top));
         if (lane == 0) red_u[stage][warp] = top;
@@ -242,7 +238,7 @@ rmsnorm_quantize_stream_kernel(const T* __restrict__ x, long long ldx, const flo
             for (int c = 0; c < V; ++c) {
                 float y[8];
                 Io<T>::unpack(row[c], y);
-                if ((tid + c * TT) * 8 < K) {
+                if (column_of<V>(c) < K) {
 #pragma unroll
                     for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(finite_or_zero(y[i])));
                 }
@@ -262,11 +258,9 @@ rmsnorm_quantize_stream_kernel(const T* __restrict__ x, long long ldx, const flo
         const bool fast = row_finite && s <= 3.402823466e38f;
 #pragma unroll
         for (int c = 0; c < V; ++c) {
-            const int k = (tid + c * TT) * 8;
+            const int k = column_of<V>(c);
             if (k < K) {
-                float y[8];
-                Io<T>::unpack(row[c], y);
-                *reinterpret_cast<uint2*>(q + (size_t)m * K + k) = fast ? quantise8<true>(y, s) : quantise8<false>(y, s);
+                *reinterpret_cast<uint2*>(q + (size_t)m * K + k) = fast ? quantise8<T, true>(row[c], s, nz) : quantise8<T, false>(row[c], s, nz);
             }
         }
     }
@@ -338,9 +332,9 @@ rmsnorm_backward_kernel(const T* __restrict__ g, const T* __restrict__ x, const 
 // Streaming form of the same: one CTA walks over the tokens with three rows per thread-owned slot set (row_stream.cuh), the
 // column sums stay in registers, and the row sum of the NEXT token is formed before the gradient of the current one, so that
 // its exchange between the warps hides behind the gradient and a token costs one barrier.
-// What bounds it: a token is 22 instructions and two float64 conversions per element; memory 6 bytes per element (bf16).
+// What bounds it: a token is about 30 instructions and two float64 conversions per element; memory 6 bytes per element (bf16).
 // 4096 tokens x 11008, bf16: 230 us with one token at a time, column sums in shared memory at a 64-byte stride (four-way bank
-// conflicts) and both passes reading the rows from L2/HBM; 91 us in this form; x 4096: 83 -> 42 us (events around the call, L2 flushed, the
+// conflicts) and both passes reading the rows from L2/HBM; 83 us in this form; x 4096: 83 -> 40 us (events around the call, L2 flushed, the
 // dweight kernel included).
 // V: vectors of 8 columns per thread; THREADS: the largest CTA (sets the register budget).
 constexpr int BW_STAGES = 3;
@@ -350,13 +344,14 @@ rmsnorm_backward_stream_kernel(const T* __restrict__ g, const T* __restrict__ x,
                                const float* __restrict__ rstd, T* __restrict__ dx, double* __restrict__ partial, int M, int K) {
     extern __shared__ uint4 ring[];
     __shared__ double red[2][MAX_RED];
-    const Slots<T, 2 * V> slots{ring};
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, TT = blockDim.x;
+    const Slots<T, BW_STAGES, 2 * V> slots(ring);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const f32x2 nz = negative_zeros();
     typename Io<T>::Raw w[V];
     double col[V][8];
 #pragma unroll
     for (int c = 0; c < V; ++c) {
-        const int k = (tid + c * TT) * 8;
+        const int k = column_of<V>(c);
         float wv[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
         if (k < K) load8_w(weight + k, wv);
         w[c] = Io<T>::pack(wv);                      // rounds to the I/O type
@@ -367,7 +362,7 @@ rmsnorm_backward_stream_kernel(const T* __restrict__ g, const T* __restrict__ x,
         if (m < M) {
 #pragma unroll
             for (int c = 0; c < V; ++c) {
-                const int k = (tid + c * TT) * 8;
+                const int k = column_of<V>(c);
                 if (k < K) {
                     slots.fetch(stage, 2 * c, g + (size_t)m * K + k);
                     slots.fetch(stage, 2 * c + 1, x + (size_t)m * K + k);
@@ -381,17 +376,11 @@ rmsnorm_backward_stream_kernel(const T* __restrict__ g, const T* __restrict__ x,
         double s = 0.0;
 #pragma unroll
         for (int c = 0; c < V; ++c) {
-            if ((tid + c * TT) * 8 < K) {
-                float gn[8], xv[8];
-                Io<T>::unpack(mul_raw(slots.read(stage, 2 * c), w[c]), gn);
-                Io<T>::unpack(slots.read(stage, 2 * c + 1), xv);
-                double a = 0.0, b = 0.0;
-#pragma unroll
-                for (int i = 0; i < 8; i += 2) {
-                    a += (double)__fmul_rn(gn[i], xv[i]);
-                    b += (double)__fmul_rn(gn[i + 1], xv[i + 1]);
-                }
-                s += a + b;
+            if (column_of<V>(c) < K) {
+                f32x2 gn[4], xv[4];
+                unpack2<T>(mul_raw(slots.read(stage, 2 * c), w[c]), gn);
+                unpack2<T>(slots.read(stage, 2 * c + 1), xv);
+                s += dot8(gn, xv);
             }
         }
         return s;
@@ -416,24 +405,29 @@ rmsnorm_backward_stream_kernel(const T* __restrict__ g, const T* __restrict__ x,
         const float r = rstd[m];
         const float r3 = __fmul_rn(__fmul_rn(r, r), r);
         const float coef = __fdiv_rn(__fmul_rn(r3, (float)csum), (float)K);
+        const f32x2 r2 = pair(r, r), coef2 = pair(coef, coef);
 #pragma unroll
         for (int c = 0; c < V; ++c) {
-            const int k = (tid + c * TT) * 8;
+            const int k = column_of<V>(c);
             if (k < K) {
                 const typename Io<T>::Raw graw = slots.read(stage, 2 * c);
-                float gv[8], gn[8], xv[8], xn[8], o[8];
-                Io<T>::unpack(graw, gv);
-                Io<T>::unpack(mul_raw(graw, w[c]), gn);
-                Io<T>::unpack(slots.read(stage, 2 * c + 1), xv);
+                f32x2 v[4], xv[4], o[4];
+                unpack2<T>(mul_raw(graw, w[c]), v);                              // gn = io(g*io(w))
+                unpack2<T>(slots.read(stage, 2 * c + 1), xv);
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    xn[i] = __fmul_rn(xv[i], r);
-                    o[i] = __fsub_rn(__fmul_rn(gn[i], r), __fmul_rn(xv[i], coef));
+                for (int i = 0; i < 4; ++i) {
+                    o[i] = sub2(mul2_exact(v[i], r2, nz), mul2_exact(xv[i], coef2, nz));
+                    xv[i] = mul2(xv[i], r2);
                 }
-                Io<T>::store8(dx + (size_t)m * K + k, o);
-                Io<T>::round8(xn);
+                *reinterpret_cast<typename Io<T>::Raw*>(dx + (size_t)m * K + k) = pack2<T>(o);
+                unpack2<T>(graw, v);
+                unpack2<T>(pack2<T>(xv), xv);                                    // io(x*r)
 #pragma unroll
-                for (int i = 0; i < 8; ++i) col[c][i] += (double)__fmul_rn(gv[i], xn[i]);
+                for (int i = 0; i < 4; ++i) {
+                    const f32x2 t = mul2(v[i], xv[i]);
+                    col[c][2 * i] += (double)lo_of(t);
+                    col[c][2 * i + 1] += (double)hi_of(t);
+                }
             }
         }
         fetch(stage, m + BW_STAGES * G);             // into the slots just read, by the thread that read them
@@ -444,7 +438,7 @@ rmsnorm_backward_stream_kernel(const T* __restrict__ g, const T* __restrict__ x,
     double* out = partial + (size_t)blockIdx.x * K;
 #pragma unroll
     for (int c = 0; c < V; ++c) {
-        const int k = (tid + c * TT) * 8;
+        const int k = column_of<V>(c);
         if (k < K) {
 #pragma unroll
             for (int i = 0; i < 8; i += 2) *reinterpret_cast<double2*>(out + k + i) = make_double2(col[c][i], col[c][i + 1]);

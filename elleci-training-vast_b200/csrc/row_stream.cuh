@@ -18,14 +18,19 @@ template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile(
 // 16-byte pieces of 8 elements of T
 template <typename T> constexpr int PIECES = (int)sizeof(T) / 2;
 
-// A thread's slots: piece p of vector c of stage s lies at ((s*VECS + c)*PIECES + p)*blockDim.x + threadIdx.x, so the lanes of
-// a warp touch consecutive 16-byte words.
-template <typename T, int VECS>
+// Thread t of a CTA owns, with V vectors per thread, the vectors (t/32)*32*V + t%32 + 32*c (c < V) of every row: a warp reads
+// and writes runs of 512 bytes, and from one vector to the next all offsets, in memory and in the slots, are constants.
+template <int V> __device__ __forceinline__ int column_of(int c) {
+    return (((int)threadIdx.x >> 5) * 32 * V + ((int)threadIdx.x & 31) + 32 * c) * 8;
+}
+
+// A thread's slots: each warp has its own region of STAGES x VECS x PIECES runs of 32 16-byte words, one word per lane.
+template <typename T, int STAGES, int VECS>
 struct Slots {
     uint4* base;
-    __device__ __forceinline__ uint4* at(int s, int c, int p) const {
-        return base + ((size_t)(s * VECS + c) * PIECES<T> + p) * blockDim.x + threadIdx.x;
-    }
+    __device__ __forceinline__ explicit Slots(uint4* ring)
+        : base(ring + (threadIdx.x >> 5) * (STAGES * VECS * PIECES<T> * 32) + (threadIdx.x & 31)) {}
+    __device__ __forceinline__ uint4* at(int s, int c, int p) const { return base + ((s * VECS + c) * PIECES<T> + p) * 32; }
     __device__ __forceinline__ void fetch(int s, int c, const T* src) const {
 #pragma unroll
         for (int p = 0; p < PIECES<T>; ++p) cp_async16(at(s, c, p), reinterpret_cast<const uint4*>(src) + p);
@@ -37,7 +42,80 @@ struct Slots {
         for (int p = 0; p < PIECES<T>; ++p) d[p] = *at(s, c, p);
         return r;
     }
+    __device__ __forceinline__ void write(int s, int c, const typename Io<T>::Raw& r) const {
+        const uint4* d = reinterpret_cast<const uint4*>(&r);
+#pragma unroll
+        for (int p = 0; p < PIECES<T>; ++p) *at(s, c, p) = d[p];
+    }
 };
+
+// Two float32 values as one operand: sm_100 multiplies and adds such pairs in one instruction, each value rounded on its own, so
+// the results are those of the two scalar instructions at half the issue slots (which is what bounds these kernels).
+// A product whose result is added or subtracted next goes through mul2_exact: the assembler contracts mul.rn.f32x2 and
+// add.rn.f32x2 into one fused operation (seen as int8 values that differ at ties), which a product formed as a*b + nz, nz = -0
+// unknown at compile time, does not allow; adding -0 changes no value and no sign.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pair(float lo, float hi) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float lo_of(f32x2 v) {
+    float a, b;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+    return a;
+}
+__device__ __forceinline__ float hi_of(f32x2 v) {
+    float a, b;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+    return b;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 negative_zeros() {      // grids of these kernels are one-dimensional: blockIdx.z is 0
+    const float z = __uint_as_float(0x80000000u + blockIdx.z);
+    return pair(z, z);
+}
+__device__ __forceinline__ f32x2 mul2_exact(f32x2 a, f32x2 b, f32x2 nz) { return fma2(a, b, nz); }
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+template <typename T> __device__ __forceinline__ void unpack2(const typename Io<T>::Raw& r, f32x2 v[4]) {
+    float f[8];
+    Io<T>::unpack(r, f);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] = pair(f[2 * i], f[2 * i + 1]);
+}
+template <typename T> __device__ __forceinline__ typename Io<T>::Raw pack2(const f32x2 v[4]) {       // rounds to the I/O type
+    const float f[8] = {lo_of(v[0]), hi_of(v[0]), lo_of(v[1]), hi_of(v[1]), lo_of(v[2]), hi_of(v[2]), lo_of(v[3]), hi_of(v[3])};
+    return Io<T>::pack(f);
+}
+// sum of the 8 float32 products a*b as float64 terms
+__device__ __forceinline__ double dot8(const f32x2 a[4], const f32x2 b[4]) {
+    double s = 0.0, t = 0.0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const f32x2 p = mul2(a[i], b[i]);
+        s += (double)lo_of(p);
+        t += (double)hi_of(p);
+    }
+    return s + t;
+}
 template <typename T> __device__ __forceinline__ typename Io<T>::Raw raw_zero() {
     float z[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     return Io<T>::pack(z);
@@ -88,26 +166,23 @@ template <> __device__ __forceinline__ float magnitude<__nv_bfloat16>(uint32_t b
 template <> __device__ __forceinline__ float magnitude<__half>(uint32_t bits) { return __half2float(__ushort_as_half((unsigned short)bits)); }
 template <> __device__ __forceinline__ float magnitude<float>(uint32_t bits) { return __uint_as_float(bits); }
 
-// CTA-wide sum of doubles and maximum of words with one barrier each: the caller alternates between two `red` buffers of one
-// entry per warp from row to row, so that a buffer is rewritten only after the barrier of the row in between.
+// CTA-wide sum of doubles and maximum of words with one barrier between the two halves: one entry of `red` per warp, then every
+// warp joins the entries itself (the same operations in every warp, so all threads hold the same bits).  The caller alternates
+// between two `red` buffers from row to row, so that a buffer is rewritten only after the barrier of the row in between.
+constexpr int MAX_RED = 32;
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
 }
-__device__ __forceinline__ double sum_red(const double* red) {      // same order in every thread
-    const int nw = blockDim.x >> 5;
-    double t = red[0];
-    for (int i = 1; i < nw; ++i) t += red[i];
-    return t;
+__device__ __forceinline__ double sum_red(const double* red) {
+    const int lane = threadIdx.x & 31;
+    return warp_sum(lane < (int)(blockDim.x >> 5) ? red[lane] : 0.0);
 }
 __device__ __forceinline__ uint32_t max_red(const uint32_t* red) {
-    const int nw = blockDim.x >> 5;
-    uint32_t t = red[0];
-    for (int i = 1; i < nw; ++i) t = max(t, red[i]);
-    return t;
+    const int lane = threadIdx.x & 31;
+    return __reduce_max_sync(0xffffffffu, lane < (int)(blockDim.x >> 5) ? red[lane] : 0u);
 }
-constexpr int MAX_RED = 32;
 
 // Threads of a streaming CTA for rows of K elements, VECS vectors of 8 per thread: whole warps.
 inline int stream_threads(int K, int vecs) { return ((K + 8 * vecs - 1) / (8 * vecs) + 31) & ~31; }
@@ -115,15 +190,29 @@ inline int stream_threads(int K, int vecs) { return ((K + 8 * vecs - 1) / (8 * v
 
 }  // namespace rowio
 
-// Tokens' int8 rows: shared by the streaming norm and gate kernels.  y*s for a row whose largest magnitude gives
-// s = 127/absmax: adding 1.5*2^23 rounds |y*s| <= 127 to the nearest even integer and leaves it in the low mantissa bits (no
-// trip through the conversion unit); rows with a non-finite value take the saturating conversion, NaN -> 0.
-template <bool FAST>
-__device__ __forceinline__ uint2 quantise8(const float y[8], float s) {
+// The int8 row of a token, 8 elements.  FAST, for a row whose largest magnitude gives s = 127/absmax: adding 1.5*2^23 rounds
+// |y*s| <= 127 to the nearest even integer and leaves it in the low mantissa bits (no trip through the conversion unit); a row
+// with a non-finite value takes the saturating conversion, NaN -> 0.
+template <typename T, bool FAST>
+__device__ __forceinline__ uint2 quantise8(const typename rowio::Io<T>::Raw& raw, float s, rowio::f32x2 nz) {
+    using namespace rowio;
     int qi[8];
+    if (FAST) {
+        f32x2 y[4];
+        unpack2<T>(raw, y);
+        const f32x2 ss = pair(s, s), magic = pair(12582912.0f, 12582912.0f);
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
-        qi[i] = FAST ? __float_as_int(__fadd_rn(__fmul_rn(y[i], s), 12582912.0f)) : q8_sat(__fmul_rn(finite_or_nan(y[i]), s));
+        for (int i = 0; i < 4; ++i) {
+            const f32x2 r = add2(mul2_exact(y[i], ss, nz), magic);
+            qi[2 * i] = __float_as_int(lo_of(r));
+            qi[2 * i + 1] = __float_as_int(hi_of(r));
+        }
+    } else {
+        float y[8];
+        Io<T>::unpack(raw, y);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) qi[i] = q8_sat(__fmul_rn(finite_or_nan(y[i]), s));
+    }
     return make_uint2(pack4_s8(qi[0], qi[1], qi[2], qi[3]), pack4_s8(qi[4], qi[5], qi[6], qi[7]));
 }
 

@@ -11,7 +11,9 @@
 // Every float32 step is a single correctly rounded operation in a fixed order (the exponential is a fixed polynomial
 // evaluated with fused multiply-adds, row sums are accumulated in float64), so the CPU oracle reproduces the kernels
 // bit for bit.
-#include "row_io.cuh"
+#include <type_traits>
+
+#include "row_stream.cuh"
 
 namespace el {
 
@@ -59,6 +61,33 @@ __device__ __forceinline__ float rcp_series(float d) {
 
 // sigmoid(g) = 1 / (1 + e^-g)
 __device__ __forceinline__ float sigmoid_fixed(float g) { return rcp_series(__fadd_rn(1.0f, exp_fixed(-g))); }
+
+// The same for two values at once (paired instructions: the same operations on each value in the same order).  1/d is formed
+// from nd = -d, so that e = 1 - d*r0 = fma(nd, r0, 1).
+__device__ __forceinline__ f32x2 both(float v) { return pair(v, v); }
+__device__ __forceinline__ f32x2 sigmoid_fixed2(f32x2 g, f32x2 nz) {
+    const f32x2 t = pair(fminf(fmaxf(-lo_of(g), -87.0f), 87.0f), fminf(fmaxf(-hi_of(g), -87.0f), 87.0f));
+    const f32x2 nm = add2(mul2_exact(t, both(1.44269504088896341f), nz), both(12582912.0f));
+    const f32x2 n = sub2(nm, both(12582912.0f));
+    f32x2 r = fma2(n, both(-0.693145751953125f), t);
+    r = fma2(n, both(-1.42860682030941723e-6f), r);
+    f32x2 p = both(1.0f / 5040.0f);
+    p = fma2(p, r, both(1.0f / 720.0f));
+    p = fma2(p, r, both(1.0f / 120.0f));
+    p = fma2(p, r, both(1.0f / 24.0f));
+    p = fma2(p, r, both(1.0f / 6.0f));
+    p = fma2(p, r, both(0.5f));
+    p = fma2(p, r, both(1.0f));
+    p = fma2(p, r, both(1.0f));
+    const f32x2 scale = pair(__int_as_float((__float_as_int(lo_of(nm)) + 127) << 23), __int_as_float((__float_as_int(hi_of(nm)) + 127) << 23));
+    const f32x2 nd = sub2(both(-1.0f), mul2_exact(p, scale, nz));          // -(1 + e^t)
+    float r0, r1;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"(-lo_of(nd)));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r1) : "f"(-hi_of(nd)));
+    const f32x2 q = pair(r0, r1);
+    const f32x2 e = fma2(nd, q, both(1.0f));
+    return fma2(q, fma2(e, e, e), q);
+}
 
 // Eight elements of the gate: sig = sigmoid(g), s = io(g * sig), h = io(s * u) - silu rounded to the I/O type, then the
 // product rounded to the I/O type, as the two tensor operations of the reference round them.
@@ -219,6 +248,139 @@ swiglu_quantize_rows_kernel(const T* __restrict__ gate, const T* __restrict__ up
     }
 }
 
+// Streaming form (see rmsnorm_quantize_stream_kernel): two rows of gate and up ahead in thread-owned slots, the weight rounded
+// once, packed products.  What bounds it: about 36 instructions per element, 22 of them the fixed sigmoid; memory 5 bytes.
+// 4096 tokens x 11008, bf16: 111 us in the one-CTA-per-row form, 80 us in this one (L2 flushed).
+constexpr int SF_STAGES = 2;
+constexpr int SF_VECS = 4;                            // vectors of 8 per thread
+
+template <typename T, bool NORM>
+__global__ void __maxnreg__(80)
+swiglu_quantize_stream_kernel(const T* __restrict__ gate, const T* __restrict__ up, long long ld, const float* __restrict__ weight,
+                              int8_t* __restrict__ q, float* __restrict__ row_absmax, float* __restrict__ rstd_out, int M, int H,
+                              float norm_eps, float quant_eps) {
+    constexpr int V = SF_VECS;
+    constexpr uint32_t INF_BITS = sizeof(T) == 4 ? 0x7f800000u : (std::is_same<T, __half>::value ? 0x7c00u : 0x7f80u);
+    extern __shared__ uint4 ring[];
+    __shared__ double red_d[2][MAX_RED];
+    __shared__ uint32_t red_u[2][MAX_RED];
+    __shared__ uint32_t red_f[2][MAX_RED];
+    const Slots<T, SF_STAGES, 2 * V> slots(ring);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const f32x2 nz = negative_zeros();
+    typename Io<T>::Raw w[V];
+    if (NORM) {
+#pragma unroll
+        for (int c = 0; c < V; ++c) {
+            const int k = column_of<V>(c);
+            float wv[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+            if (k < H) load8_w(weight + k, wv);
+            w[c] = Io<T>::pack(wv);                  // rounds to the I/O type
+        }
+    }
+    auto fetch = [&](int stage, int m) {
+        if (m < M) {
+#pragma unroll
+            for (int c = 0; c < V; ++c) {
+                const int k = column_of<V>(c);
+                if (k < H) {
+                    slots.fetch(stage, 2 * c, gate + (size_t)m * ld + k);
+                    slots.fetch(stage, 2 * c + 1, up + (size_t)m * ld + k);
+                }
+            }
+        }
+        cp_async_commit();
+    };
+    const int G = gridDim.x;
+#pragma unroll
+    for (int s = 0; s < SF_STAGES; ++s) fetch(s, blockIdx.x + s * G);
+    int stage = 0;
+    for (int m = blockIdx.x; m < M; m += G, stage ^= 1) {
+        static_assert(SF_STAGES == 2, "stage doubles as the parity of the reduction buffers");
+        cp_async_wait<SF_STAGES - 1>();
+        // ---- h = io(io(g*sig(g))*u), and its mean of squares -> rstd -----------------------------------------------------------
+        typename Io<T>::Raw row[V];
+        double ss = 0.0;
+#pragma unroll
+        for (int c = 0; c < V; ++c) {
+            row[c] = raw_zero<T>();
+            if (column_of<V>(c) < H) {
+                f32x2 g[4];
+                unpack2<T>(slots.read(stage, 2 * c), g);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) g[i] = mul2(g[i], sigmoid_fixed2(g[i], nz));
+                row[c] = mul_raw(pack2<T>(g), slots.read(stage, 2 * c + 1));
+                if (NORM) {
+                    unpack2<T>(row[c], g);
+                    ss += dot8(g, g);
+                }
+            }
+        }
+        fetch(stage, m + SF_STAGES * G);             // into the slots just read, by the thread that read them
+        float r = 1.0f;
+        if (NORM) {
+            ss = warp_sum(ss);
+            if (lane == 0) red_d[stage][warp] = ss;
+            __syncthreads();
+            ss = sum_red(red_d[stage]);
+            const float ms = __fdiv_rn((float)ss, (float)H);
+            r = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(ms, norm_eps)));
+        }
+        // ---- y = io(io(h*r) * io(w)), or h itself, and its largest magnitude -----------------------------------------------------
+        uint32_t top = 0u;
+#pragma unroll
+        for (int c = 0; c < V; ++c) {
+            if (column_of<V>(c) < H) {
+                if (NORM) {
+                    f32x2 v[4];
+                    unpack2<T>(row[c], v);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) v[i] = mul2(v[i], both(r));
+                    row[c] = mul_raw(pack2<T>(v), w[c]);
+                }
+                top = max_bits(top, row[c]);
+            }
+        }
+        top = __reduce_max_sync(0xffffffffu, magnitude_bits<T>(top));
+        if (lane == 0) red_u[stage][warp] = top;
+        __syncthreads();
+        top = max_red(red_u[stage]);
+        float amax = magnitude<T>(top);
+        const bool row_finite = top < INF_BITS;      // same answer in every thread of the CTA
+        if (!row_finite) {        // the row holds an infinity or a NaN: the maximum over its finite values only
+            amax = 0.0f;
+#pragma unroll
+            for (int c = 0; c < V; ++c) {
+                float y[8];
+                Io<T>::unpack(row[c], y);
+                if (column_of<V>(c) < H) {
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(finite_or_zero(y[i])));
+                }
+            }
+            const uint32_t b = __reduce_max_sync(0xffffffffu, __float_as_uint(amax));
+            if (lane == 0) red_f[stage][warp] = b;
+            __syncthreads();
+            amax = __uint_as_float(max_red(red_f[stage]));
+        }
+        const float a = fmaxf(amax, quant_eps);
+        const float s = __fdiv_rn(127.0f, a);
+        if (tid == 0) {
+            row_absmax[m] = a;
+            if (NORM) rstd_out[m] = r;
+        }
+        // ---- quantise ---------------------------------------------------------------------------------------------------------------
+        const bool fast = row_finite && s <= 3.402823466e38f;
+#pragma unroll
+        for (int c = 0; c < V; ++c) {
+            const int k = column_of<V>(c);
+            if (k < H) {
+                *reinterpret_cast<uint2*>(q + (size_t)m * H + k) = fast ? quantise8<T, true>(row[c], s, nz) : quantise8<T, false>(row[c], s, nz);
+            }
+        }
+    }
+}
+
 // Backward.  Upstream gradient gy [M,H] with respect to the normalised product y (or to h itself when `weight` is
 // null).  Follows autograd through the reference's tensor operations, each intermediate rounded where a tensor of the
 // I/O type would hold it:
@@ -354,24 +516,156 @@ swiglu_backward_kernel(const T* __restrict__ gy, const T* __restrict__ gate, con
     }
 }
 
+// Streaming form, with the norm: one CTA walks over the tokens with up to three rows of gy, gate and up ahead in thread-owned
+// slots (row_stream.cuh), the column sums of dweight and the row's sigmoids in registers, products of two 16-bit values
+// packed.  What bounds it: about 55 instructions per element, 22 of them the fixed sigmoid, and two float64 conversions;
+// memory 10 bytes.  (The one barrier of a token is a tenth of its time, so the next token's row sum is not pulled ahead as
+// in rmsnorm_backward_stream_kernel; its sigmoids would not fit in the registers either.)
+// 4096 tokens x 11008, bf16: 228 us with column sums in shared memory at a 64-byte stride (four-way bank conflicts) and
+// every row read twice from memory; 163 us in this form (L2 flushed, the dweight kernel
+// included).
+// W_SLOTS: the rounded weights lie in slots of their own instead of registers (rows of up to 11264 16-bit elements leave room;
+// with all of it in registers 150 bytes per thread spill).
+constexpr int SB_STAGES = 3;
+template <typename T, int V, int THREADS, bool W_SLOTS>
+__global__ void __launch_bounds__(THREADS, 1)
+swiglu_backward_stream_kernel(const T* __restrict__ gy, const T* __restrict__ gate, const T* __restrict__ up, long long ld,
+                              const float* __restrict__ weight, const float* __restrict__ rstd, T* __restrict__ d_gate,
+                              T* __restrict__ d_up, long long ld_d, double* __restrict__ partial, int M, int H) {
+    extern __shared__ uint4 ring[];
+    __shared__ double red[2][MAX_RED];
+    const Slots<T, SB_STAGES, 3 * V> slots(ring);
+    const Slots<T, 1, V> w_slots(ring + SB_STAGES * 3 * V * PIECES<T> * blockDim.x);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const f32x2 nz = negative_zeros();
+    typename Io<T>::Raw w[W_SLOTS ? 1 : V];
+    double col[V][8];
+#pragma unroll
+    for (int c = 0; c < V; ++c) {
+        const int k = column_of<V>(c);
+        float wv[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        if (k < H) load8_w(weight + k, wv);
+        const typename Io<T>::Raw wr = Io<T>::pack(wv);      // rounds to the I/O type
+        if (W_SLOTS) w_slots.write(0, c, wr);
+        else w[W_SLOTS ? 0 : c] = wr;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) col[c][i] = 0.0;
+    }
+    auto weight_of = [&](int c) -> typename Io<T>::Raw { return W_SLOTS ? w_slots.read(0, c) : w[W_SLOTS ? 0 : c]; };
+    auto fetch = [&](int stage, int m) {
+        if (m < M) {
+#pragma unroll
+            for (int c = 0; c < V; ++c) {
+                const int k = column_of<V>(c);
+                if (k < H) {
+                    slots.fetch(stage, 3 * c, gy + (size_t)m * H + k);
+                    slots.fetch(stage, 3 * c + 1, gate + (size_t)m * ld + k);
+                    slots.fetch(stage, 3 * c + 2, up + (size_t)m * ld + k);
+                }
+            }
+        }
+        cp_async_commit();
+    };
+    const int G = gridDim.x;
+#pragma unroll
+    for (int s = 0; s < SB_STAGES; ++s) fetch(s, blockIdx.x + s * G);
+    int stage = 0, par = 0;
+    for (int m = blockIdx.x; m < M; m += G, par ^= 1) {
+        cp_async_wait<SB_STAGES - 1>();
+        const float r = rstd[m];
+        // ---- c = sum of io(gy*io(w)) * h; the sigmoids stay in registers ------------------------------------------------------------
+        f32x2 sig[V][4];
+        double dot = 0.0;
+#pragma unroll
+        for (int c = 0; c < V; ++c) {
+            if (column_of<V>(c) < H) {
+                f32x2 g[4], gn[4];
+                unpack2<T>(slots.read(stage, 3 * c + 1), g);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    sig[c][i] = sigmoid_fixed2(g[i], nz);
+                    g[i] = mul2(g[i], sig[c][i]);
+                }
+                unpack2<T>(mul_raw(pack2<T>(g), slots.read(stage, 3 * c + 2)), g);           // h
+                unpack2<T>(mul_raw(slots.read(stage, 3 * c), weight_of(c)), gn);
+                dot += dot8(gn, g);
+            }
+        }
+        dot = warp_sum(dot);
+        if (lane == 0) red[par][warp] = dot;
+        __syncthreads();
+        dot = sum_red(red[par]);
+        const float r3 = __fmul_rn(__fmul_rn(r, r), r);
+        const float coef = __fdiv_rn(__fmul_rn(r3, (float)dot), (float)H);
+        // ---- the gradients --------------------------------------------------------------------------------------------------------------
+#pragma unroll
+        for (int c = 0; c < V; ++c) {
+            const int k = column_of<V>(c);
+            if (k < H) {
+                const typename Io<T>::Raw yr = slots.read(stage, 3 * c), ur = slots.read(stage, 3 * c + 2);
+                f32x2 g[4], h[4], t[4];
+                unpack2<T>(slots.read(stage, 3 * c + 1), g);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) t[i] = mul2(g[i], sig[c][i]);
+                const typename Io<T>::Raw sr = pack2<T>(t);                       // s = io(g*sig)
+                unpack2<T>(mul_raw(sr, ur), h);                                   // h = io(s*u)
+                {
+                    f32x2 yv[4];
+                    unpack2<T>(yr, yv);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) t[i] = mul2(h[i], both(r));
+                    unpack2<T>(pack2<T>(t), t);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const f32x2 d = mul2(yv[i], t[i]);
+                        col[c][2 * i] += (double)lo_of(d);
+                        col[c][2 * i + 1] += (double)hi_of(d);
+                    }
+                }
+                unpack2<T>(mul_raw(yr, weight_of(c)), t);                                 // gn = io(gy*io(w))
+#pragma unroll
+                for (int i = 0; i < 4; ++i) t[i] = sub2(mul2_exact(t[i], both(r), nz), mul2_exact(h[i], both(coef), nz));
+                const typename Io<T>::Raw dh = pack2<T>(t);
+                *reinterpret_cast<typename Io<T>::Raw*>(d_up + (size_t)m * ld_d + k) = mul_raw(dh, sr);
+                unpack2<T>(mul_raw(dh, ur), t);                                   // ds = io(dh*u)
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    t[i] = mul2(mul2(t[i], sig[c][i]), add2(both(1.0f), mul2_exact(g[i], sub2(both(1.0f), sig[c][i]), nz)));
+                *reinterpret_cast<typename Io<T>::Raw*>(d_gate + (size_t)m * ld_d + k) = pack2<T>(t);
+            }
+        }
+        fetch(stage, m + SB_STAGES * G);             // into the slots just read, by the thread that read them
+        stage = stage + 1 == SB_STAGES ? 0 : stage + 1;
+    }
+    double* out = partial + (size_t)blockIdx.x * H;
+#pragma unroll
+    for (int c = 0; c < V; ++c) {
+        const int k = column_of<V>(c);
+        if (k < H) {
+#pragma unroll
+            for (int i = 0; i < 8; i += 2) *reinterpret_cast<double2*>(out + k + i) = make_double2(col[c][i], col[c][i + 1]);
+        }
+    }
+}
+
 // dweight[k] = float(sum of the CTAs' partial sums), in a fixed order of additions for any grid (32 columns per CTA, the
-// eight warps each add every eighth partial in order, warp 0 adds the eight results in order).
-__global__ void __launch_bounds__(256)
+// 32 warps each add every 32nd partial in order, warp 0 adds their results in order).
+__global__ void __launch_bounds__(1024)
 swiglu_dweight_kernel(const double* __restrict__ partial, int n_parts, float* __restrict__ dweight, int H) {
-    __shared__ double part[8][32];
+    __shared__ double part[32][32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int k = blockIdx.x * 32 + lane;
     double s = 0.0;
     if (k < H) {
-#pragma unroll 4
-        for (int p = warp; p < n_parts; p += 8) s += partial[(size_t)p * H + k];
+#pragma unroll 8
+        for (int p = warp; p < n_parts; p += 32) s += partial[(size_t)p * H + k];
     }
     part[warp][lane] = s;
     __syncthreads();
     if (warp == 0 && k < H) {
         double t = 0.0;
 #pragma unroll
-        for (int w = 0; w < 8; ++w) t += part[w][lane];
+        for (int w = 0; w < 32; ++w) t += part[w][lane];
         dweight[k] = (float)t;
     }
 }
@@ -487,6 +781,48 @@ int launch_sigmoid_fixed(const float* g, float* sig, long long n, cudaStream_t s
     return check_launch();
 }
 
+template <typename T, bool NORM>
+static int launch_quantize_stream(const T* gate, const T* up, long long ld, const float* weight, float norm_eps, int8_t* q,
+                                  float* row_absmax, float* rstd, int M, int H, float quant_eps, cudaStream_t st) {
+    static DeviceOnce attr_once;
+    int dev = 0, sms = 0;
+    EL_CUDA_TRY(cudaGetDevice(&dev));
+    const int rc = device_sm_count(&sms);
+    if (rc != EL_OK) return rc;
+    if (!attr_once.is_done(dev)) {
+        EL_CUDA_TRY(cudaFuncSetAttribute(swiglu_quantize_stream_kernel<T, NORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+        attr_once.mark(dev);
+    }
+    const int threads = stream_threads(H, SF_VECS);
+    const size_t smem = (size_t)SF_STAGES * 2 * 64 * threads;
+    int per_sm = 768 / threads;                      // 80 registers per thread
+    const int by_smem = (int)((200u * 1024u) / (smem + 1024));
+    per_sm = per_sm < by_smem ? per_sm : by_smem;
+    per_sm = per_sm < 1 ? 1 : (per_sm > 24 ? 24 : per_sm);
+    const int grid = M < sms * per_sm ? M : sms * per_sm;
+    swiglu_quantize_stream_kernel<T, NORM><<<grid, threads, smem, st>>>(gate, up, ld, weight, q, row_absmax, rstd, M, H, norm_eps, quant_eps);
+    return check_launch();
+}
+
+// 16-bit rows of up to 16384 elements (two stages of gate and up then fit in shared memory) stream; longer ones and float32,
+// whose row takes twice the slots for the same arithmetic, run the one-CTA-per-row kernel (float32, 1000 tokens x 4096: 18.4 us there,
+// 22.6 us streaming).
+template <typename T>
+static int launch_quantize_t(const T* gate, const T* up, long long ld, const float* weight, float norm_eps, int8_t* q, float* row_absmax,
+                             float* rstd, int M, int H, float quant_eps, cudaStream_t st) {
+    if constexpr (sizeof(T) == 2) {
+        if (H <= 16384) {
+            if (weight) return launch_quantize_stream<T, true>(gate, up, ld, weight, norm_eps, q, row_absmax, rstd, M, H, quant_eps, st);
+            return launch_quantize_stream<T, false>(gate, up, ld, weight, norm_eps, q, row_absmax, rstd, M, H, quant_eps, st);
+        }
+    }
+    if (sizeof(T) == 4 && H <= 4096)
+        swiglu_quantize_rows_kernel<T, 2><<<M, RN_THREADS, 0, st>>>(gate, up, ld, weight, q, row_absmax, rstd, H, norm_eps, quant_eps);
+    else
+        swiglu_quantize_rows_kernel<T, 6><<<M, RN_THREADS, 0, st>>>(gate, up, ld, weight, q, row_absmax, rstd, H, norm_eps, quant_eps);
+    return check_launch();
+}
+
 int launch_swiglu_quantize_rows(const void* gate, const void* up, int dt, long long ld, const float* weight, float norm_eps,
                                 int8_t* q, float* row_absmax, float* rstd, int M, int H, float quant_eps, cudaStream_t st) {
     if (M == 0) return EL_OK;
@@ -495,15 +831,12 @@ int launch_swiglu_quantize_rows(const void* gate, const void* up, int dt, long l
     if ((reinterpret_cast<uintptr_t>(gate) & 15) || (reinterpret_cast<uintptr_t>(up) & 15) || ((size_t)ld * esz) % 16 != 0 ||
         (reinterpret_cast<uintptr_t>(weight) & 15) || (reinterpret_cast<uintptr_t>(q) & 7))
         return EL_ERR_ALIGNMENT;
-#define EL_SGQ(T, NC) swiglu_quantize_rows_kernel<T, NC><<<M, RN_THREADS, 0, st>>>((const T*)gate, (const T*)up, ld, weight, q, row_absmax, rstd, H, norm_eps, quant_eps)
     switch (dt) {
-        case EL_BF16: if (H <= 4096) EL_SGQ(__nv_bfloat16, 2); else EL_SGQ(__nv_bfloat16, 6); break;
-        case EL_F16: if (H <= 4096) EL_SGQ(__half, 2); else EL_SGQ(__half, 6); break;
-        case EL_F32: if (H <= 4096) EL_SGQ(float, 2); else EL_SGQ(float, 6); break;
+        case EL_BF16: return launch_quantize_t((const __nv_bfloat16*)gate, (const __nv_bfloat16*)up, ld, weight, norm_eps, q, row_absmax, rstd, M, H, quant_eps, st);
+        case EL_F16: return launch_quantize_t((const __half*)gate, (const __half*)up, ld, weight, norm_eps, q, row_absmax, rstd, M, H, quant_eps, st);
+        case EL_F32: return launch_quantize_t((const float*)gate, (const float*)up, ld, weight, norm_eps, q, row_absmax, rstd, M, H, quant_eps, st);
         default: return EL_ERR_INVALID_ARG;
     }
-#undef EL_SGQ
-    return check_launch();
 }
 
 template <typename T, int SIG_CACHE>
@@ -524,7 +857,35 @@ static int launch_swiglu_backward_norm(const T* gy, const T* gate, const T* up, 
                                                                                partial, M, H);
     int rc = check_launch();
     if (rc != EL_OK) return rc;
-    swiglu_dweight_kernel<<<(H + 31) / 32, 256, 0, st>>>(partial, grid, dweight, H);
+    swiglu_dweight_kernel<<<(H + 31) / 32, 1024, 0, st>>>(partial, grid, dweight, H);
+    return check_launch();
+}
+
+template <typename T, int THREADS, bool W_SLOTS>
+static int launch_backward_stream(const T* gy, const T* gate, const T* up, long long ld, const float* weight, const float* rstd,
+                                  T* d_gate, T* d_up, long long ld_d, float* dweight, double* partial, int M, int H, cudaStream_t st) {
+    static DeviceOnce attr_once;
+    int dev = 0, sms = 0;
+    EL_CUDA_TRY(cudaGetDevice(&dev));
+    int rc = device_sm_count(&sms);
+    if (rc != EL_OK) return rc;
+    if (!attr_once.is_done(dev)) {
+        EL_CUDA_TRY(cudaFuncSetAttribute(swiglu_backward_stream_kernel<T, 2, THREADS, W_SLOTS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         226 * 1024));
+        attr_once.mark(dev);
+    }
+    const int threads = stream_threads(H, 2);
+    const size_t smem = (size_t)(SB_STAGES * 3 + (W_SLOTS ? 1 : 0)) * 2 * PIECES<T> * sizeof(uint4) * threads;
+    // resident CTAs per SM by registers and shared memory, at most the four per SM that the workspace holds partials for
+    int per_sm = THREADS / threads;
+    const int by_smem = (int)((226u * 1024u) / smem);
+    per_sm = per_sm < by_smem ? per_sm : by_smem;
+    per_sm = per_sm < 1 ? 1 : (per_sm > 4 ? 4 : per_sm);
+    const int grid = M < sms * per_sm ? M : sms * per_sm;
+    swiglu_backward_stream_kernel<T, 2, THREADS, W_SLOTS><<<grid, threads, smem, st>>>(gy, gate, up, ld, weight, rstd, d_gate, d_up, ld_d, partial, M, H);
+    rc = check_launch();
+    if (rc != EL_OK) return rc;
+    swiglu_dweight_kernel<<<(H + 31) / 32, 1024, 0, st>>>(partial, grid, dweight, H);
     return check_launch();
 }
 
@@ -538,8 +899,18 @@ static int launch_swiglu_backward_t(const T* gy, const T* gate, const T* up, lon
                                                                          nullptr, M, H);
         return check_launch();
     }
-    // registers per thread that cost no occupancy: rows up to 4096 elements run four CTAs per SM, longer rows two or one
-    if (H <= 4096) return launch_swiglu_backward_norm<T, 2>(gy, gate, up, ld, weight, rstd, d_gate, d_up, ld_d, dweight, partial, M, H, st);
+    // Rows whose three stages of gy, gate and up fit in shared memory stream (16-bit types: 12288 columns, float32: 6144).
+    // Two vectors per thread: 80 registers at 768 threads.
+    const int threads = stream_threads(H, 2);
+#define EL_SGB(THREADS, W_SLOTS) return launch_backward_stream<T, THREADS, W_SLOTS>(gy, gate, up, ld, weight, rstd, d_gate, d_up, ld_d, dweight, partial, M, H, st)
+    if constexpr (sizeof(T) == 2) {
+        if (threads <= 704) EL_SGB(704, true);
+        if (threads <= 768) EL_SGB(768, false);
+    } else {
+        if (threads <= 352) EL_SGB(384, true);
+        if (threads <= 384) EL_SGB(384, false);
+    }
+#undef EL_SGB
     return launch_swiglu_backward_norm<T, 6>(gy, gate, up, ld, weight, rstd, d_gate, d_up, ld_d, dweight, partial, M, H, st);
 }
 
