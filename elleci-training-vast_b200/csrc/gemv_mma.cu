@@ -217,15 +217,14 @@ gemv_mma_kernel(const T* __restrict__ x, const int8_t* xq, const float* amax_in,
                     }
                 }
             }
-            // partial sums of this warp's blocks -> the CTA's accumulator for this row group
+            // partial sums of this warp's blocks -> the CTA's accumulator for this row group, in the lanes' own order: 32 different
+            // banks per instruction.  (As a [16][MT] matrix, eight rows met in the same banks from 32 tokens on: 4096 -> 11008 with
+            // 32 tokens 18.6 us, 64 tokens 34.2 us; 13.2 and 23.6 us in this order.)
             int* acc = acc_sm + (gi & 1) * 16 * MT;
 #pragma unroll
             for (int t = 0; t < NT; ++t) {
-                const int col = t * 8 + seg * 2;
-                atomicAdd(&acc[r8 * MT + col], d[t][0]);
-                atomicAdd(&acc[r8 * MT + col + 1], d[t][1]);
-                atomicAdd(&acc[(r8 + 8) * MT + col], d[t][2]);
-                atomicAdd(&acc[(r8 + 8) * MT + col + 1], d[t][3]);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) atomicAdd(&acc[(t * 4 + i) * 32 + lane], d[t][i]);
             }
         }
         __syncthreads();
@@ -234,8 +233,10 @@ gemv_mma_kernel(const T* __restrict__ x, const int8_t* xq, const float* amax_in,
         for (int i = tid; i < 16 * MT; i += GM_THREADS) {
             const int m = i >> 4, row = i & 15;
             const int n = g * 16 + row;
-            const int v = acc[row * MT + m];
-            acc[row * MT + m] = 0;
+            // sum i of lane l of token group t: row (l>>2) + 8*(i>>1), token 8*t + 2*(l&3) + (i&1)
+            int* slot = &acc[((m >> 3) * 4 + ((row >> 3) << 1) + (m & 1)) * 32 + (row & 7) * 4 + ((m & 7) >> 1)];
+            const int v = *slot;
+            *slot = 0;
             if (m < M && n < N) {
                 const float sc = __fmul_rn(__fdiv_rn(s_amax[m], 127.0f), epi.alpha);
                 epi_store_one(epi, m, n, v, sc);
