@@ -8,8 +8,6 @@
 //
 // Row sums (of squares, and in the backward pass) are accumulated in float64, so that their float32 value does not
 // depend on the order of the additions: the result is the one the CPU oracle defines, bit for bit.
-#include <type_traits>
-
 #include "row_stream.cuh"
 
 namespace el {
@@ -334,7 +332,7 @@ rmsnorm_backward_kernel(const T* __restrict__ g, const T* __restrict__ x, const 
 // its exchange between the warps hides behind the gradient and a token costs one barrier.
 // What bounds it: a token is about 30 instructions and two float64 conversions per element; memory 6 bytes per element (bf16).
 // 4096 tokens x 11008, bf16: 230 us with one token at a time, column sums in shared memory at a 64-byte stride (four-way bank
-// conflicts) and both passes reading the rows from L2/HBM; 83 us in this form; x 4096: 83 -> 40 us (events around the call, L2 flushed, the
+// conflicts) and both passes reading the rows from L2/HBM; 77 us in this form; x 4096: 83 -> 40 us (events around the call, L2 flushed, the
 // dweight kernel included).
 // V: vectors of 8 columns per thread; THREADS: the largest CTA (sets the register budget).
 constexpr int BW_STAGES = 3;
@@ -395,6 +393,7 @@ rmsnorm_backward_stream_kernel(const T* __restrict__ g, const T* __restrict__ x,
     __syncthreads();
     csum = sum_red(red[0]);
     int par = 1;
+    float r = m < M ? rstd[m] : 0.0f;
     for (; m < M; m += G, par ^= 1) {
         const int next = stage + 1 == BW_STAGES ? 0 : stage + 1;
         cp_async_wait<BW_STAGES - 2>();
@@ -402,7 +401,7 @@ rmsnorm_backward_stream_kernel(const T* __restrict__ g, const T* __restrict__ x,
             const double s = warp_sum(row_dot(next));
             if (lane == 0) red[par][warp] = s;
         }
-        const float r = rstd[m];
+        const float r_next = m + G < M ? __ldg(rstd + m + G) : 0.0f;
         const float r3 = __fmul_rn(__fmul_rn(r, r), r);
         const float coef = __fdiv_rn(__fmul_rn(r3, (float)csum), (float)K);
         const f32x2 r2 = pair(r, r), coef2 = pair(coef, coef);
@@ -434,6 +433,7 @@ rmsnorm_backward_stream_kernel(const T* __restrict__ g, const T* __restrict__ x,
         __syncthreads();
         csum = sum_red(red[par]);
         stage = next;
+        r = r_next;
     }
     double* out = partial + (size_t)blockIdx.x * K;
 #pragma unroll
@@ -446,27 +446,33 @@ rmsnorm_backward_stream_kernel(const T* __restrict__ g, const T* __restrict__ x,
     }
 }
 
-// dweight[k] = float(sum of the CTAs' partial sums).  A CTA covers 32 columns (one per lane); its 32 warps each add every
-// 32nd partial in order, and warp 0 adds the 32 results in order: a fixed order of additions for any grid.
-// (Eight warps per CTA: 10.9 us for 592 partials of 16 columns, a chain of dependent loads; 3.8 us with 32.)
+// dweight[k] = float(sum of the CTAs' partial sums).  A CTA covers 32 columns (one per lane); its W warps (8 or 32) each add
+// every W-th partial in order, and warp 0 adds their results in order: a fixed order of additions for a given width.
+// Few columns take 32 warps: 592 partials of 16 columns on 8 warps are a chain of dependent loads (10.9 us, 3.8 us with 32); where
+// the columns fill the SMs, 8 warps per CTA are enough and start sooner.
 __global__ void __launch_bounds__(1024)
 rmsnorm_dweight_kernel(const double* __restrict__ partial, int n_parts, float* __restrict__ dweight, int K) {
     __shared__ double part[32][32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
     const int k = blockIdx.x * 32 + lane;
     double s = 0.0;
     if (k < K) {
 #pragma unroll 8
-        for (int p = warp; p < n_parts; p += 32) s += partial[(size_t)p * K + k];
+        for (int p = warp; p < n_parts; p += warps) s += partial[(size_t)p * K + k];
     }
     part[warp][lane] = s;
     __syncthreads();
     if (warp == 0 && k < K) {
         double t = 0.0;
-#pragma unroll
-        for (int w = 0; w < 32; ++w) t += part[w][lane];
+        for (int w = 0; w < warps; ++w) t += part[w][lane];
         dweight[k] = (float)t;
     }
+}
+
+int dweight_threads(int columns) {
+    int sms = 148;
+    device_sm_count(&sms);
+    return (columns + 31) / 32 <= sms ? 1024 : 256;
 }
 
 int backward_grid(int M, int K) {
@@ -575,7 +581,7 @@ static int launch_rmsnorm_backward_t(const T* g, const T* x, const float* weight
         if (stream_threads(K, 2) <= MAX_V2) rc = launch_backward_stream<T, 2, MAX_V2>(g, x, weight, rstd, dx, partial, M, K, &grid, st);
         else if constexpr (sizeof(T) == 2) rc = launch_backward_stream<T, 4, 512>(g, x, weight, rstd, dx, partial, M, K, &grid, st);
         if (rc != EL_OK) return rc;
-        rmsnorm_dweight_kernel<<<(K + 31) / 32, 1024, 0, st>>>(partial, grid, dweight, K);
+        rmsnorm_dweight_kernel<<<(K + 31) / 32, dweight_threads(K), 0, st>>>(partial, grid, dweight, K);
         return check_launch();
     }
     const size_t smem = (size_t)K * sizeof(double);
@@ -589,7 +595,7 @@ static int launch_rmsnorm_backward_t(const T* g, const T* x, const float* weight
     rmsnorm_backward_kernel<T><<<grid, RN_THREADS, smem, st>>>(g, x, weight, rstd, dx, partial, M, K);
     rc = check_launch();
     if (rc != EL_OK) return rc;
-    rmsnorm_dweight_kernel<<<(K + 31) / 32, 1024, 0, st>>>(partial, grid, dweight, K);
+    rmsnorm_dweight_kernel<<<(K + 31) / 32, dweight_threads(K), 0, st>>>(partial, grid, dweight, K);
     return check_launch();
 }
 

@@ -3,6 +3,8 @@
 // asynchronous 16-byte copies, so the rows ahead cost neither registers nor barriers: the thread that waits is the thread
 // that issued, and no other thread reads its slots.
 #pragma once
+#include <type_traits>
+
 #include "row_io.cuh"
 
 namespace el {
@@ -142,6 +144,44 @@ __device__ __forceinline__ Io<float>::Raw mul_raw(const Io<float>::Raw& a, const
     r.a = make_float4(__fmul_rn(a.a.x, b.a.x), __fmul_rn(a.a.y, b.a.y), __fmul_rn(a.a.z, b.a.z), __fmul_rn(a.a.w, b.a.w));
     r.b = make_float4(__fmul_rn(a.b.x, b.b.x), __fmul_rn(a.b.y, b.b.y), __fmul_rn(a.b.z, b.b.z), __fmul_rn(a.b.w, b.b.w));
     return r;
+}
+
+// Half of such a vector: 4 elements, for loops that would not fit in the registers eight at a time.
+template <typename T> struct Quad { uint2 a; };
+template <> struct Quad<float> { float4 a; };
+template <typename T> __device__ __forceinline__ Quad<T> quad_of(const typename Io<T>::Raw& r, int half) {
+    Quad<T> q;
+    if constexpr (sizeof(T) == 2) q.a = half ? make_uint2(r.a.z, r.a.w) : make_uint2(r.a.x, r.a.y);
+    else q.a = half ? r.b : r.a;
+    return q;
+}
+template <typename T> __device__ __forceinline__ void unpack2(const Quad<T>& q, f32x2 v[2]) {
+    if constexpr (std::is_same<T, float>::value) {
+        v[0] = pair(q.a.x, q.a.y);
+        v[1] = pair(q.a.z, q.a.w);
+    } else if constexpr (std::is_same<T, __half>::value) {
+        const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&q.a.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&q.a.y));
+        v[0] = pair(a.x, a.y);
+        v[1] = pair(b.x, b.y);
+    } else {
+        v[0] = pair(__uint_as_float(q.a.x << 16), __uint_as_float(q.a.x & 0xFFFF0000u));
+        v[1] = pair(__uint_as_float(q.a.y << 16), __uint_as_float(q.a.y & 0xFFFF0000u));
+    }
+}
+template <typename T> __device__ __forceinline__ Quad<T> pack2(f32x2 v0, f32x2 v1) {       // rounds to the I/O type
+    Quad<T> q;
+    if constexpr (std::is_same<T, float>::value) q.a = make_float4(lo_of(v0), hi_of(v0), lo_of(v1), hi_of(v1));
+    else if constexpr (std::is_same<T, __half>::value) q.a = make_uint2(pack_f16x2(lo_of(v0), hi_of(v0)), pack_f16x2(lo_of(v1), hi_of(v1)));
+    else q.a = make_uint2(pack_bf16x2(lo_of(v0), hi_of(v0)), pack_bf16x2(lo_of(v1), hi_of(v1)));
+    return q;
+}
+template <typename T> __device__ __forceinline__ Quad<T> mul_quad(const Quad<T>& a, const Quad<T>& b) {       // io(a*b)
+    Quad<T> q;
+    if constexpr (std::is_same<T, float>::value)
+        q.a = make_float4(__fmul_rn(a.a.x, b.a.x), __fmul_rn(a.a.y, b.a.y), __fmul_rn(a.a.z, b.a.z), __fmul_rn(a.a.w, b.a.w));
+    else if constexpr (std::is_same<T, __half>::value) q.a = make_uint2(mul_f16x2(a.a.x, b.a.x), mul_f16x2(a.a.y, b.a.y));
+    else q.a = make_uint2(mul_bf16x2(a.a.x, b.a.x), mul_bf16x2(a.a.y, b.a.y));
+    return q;
 }
 
 // Running maximum of |value| on bit patterns: the order of finite values is the order of their bits, and infinities and NaN

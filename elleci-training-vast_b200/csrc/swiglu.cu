@@ -11,8 +11,6 @@
 // Every float32 step is a single correctly rounded operation in a fixed order (the exponential is a fixed polynomial
 // evaluated with fused multiply-adds, row sums are accumulated in float64), so the CPU oracle reproduces the kernels
 // bit for bit.
-#include <type_traits>
-
 #include "row_stream.cuh"
 
 namespace el {
@@ -522,10 +520,10 @@ swiglu_backward_kernel(const T* __restrict__ gy, const T* __restrict__ gate, con
 // memory 10 bytes.  (The one barrier of a token is a tenth of its time, so the next token's row sum is not pulled ahead as
 // in rmsnorm_backward_stream_kernel; its sigmoids would not fit in the registers either.)
 // 4096 tokens x 11008, bf16: 228 us with column sums in shared memory at a 64-byte stride (four-way bank conflicts) and
-// every row read twice from memory; 163 us in this form (L2 flushed, the dweight kernel
+// every row read twice from memory; 142 us in this form (L2 flushed, the dweight kernel
 // included).
 // W_SLOTS: the rounded weights lie in slots of their own instead of registers (rows of up to 11264 16-bit elements leave room;
-// with all of it in registers 150 bytes per thread spill).
+// with all of it in registers 150 bytes per thread spill, and with shared memory this full the spills go to L2: 163 us).
 constexpr int SB_STAGES = 3;
 template <typename T, int V, int THREADS, bool W_SLOTS>
 __global__ void __launch_bounds__(THREADS, 1)
@@ -602,36 +600,36 @@ swiglu_backward_stream_kernel(const T* __restrict__ gy, const T* __restrict__ ga
         for (int c = 0; c < V; ++c) {
             const int k = column_of<V>(c);
             if (k < H) {
-                const typename Io<T>::Raw yr = slots.read(stage, 3 * c), ur = slots.read(stage, 3 * c + 2);
-                f32x2 g[4], h[4], t[4];
-                unpack2<T>(slots.read(stage, 3 * c + 1), g);
+                const typename Io<T>::Raw yr = slots.read(stage, 3 * c), gr = slots.read(stage, 3 * c + 1), ur = slots.read(stage, 3 * c + 2);
+                const typename Io<T>::Raw wr = weight_of(c);
 #pragma unroll
-                for (int i = 0; i < 4; ++i) t[i] = mul2(g[i], sig[c][i]);
-                const typename Io<T>::Raw sr = pack2<T>(t);                       // s = io(g*sig)
-                unpack2<T>(mul_raw(sr, ur), h);                                   // h = io(s*u)
-                {
-                    f32x2 yv[4];
-                    unpack2<T>(yr, yv);
+                for (int half = 0; half < 2; ++half) {       // four elements at a time: eight spill
+                    const Quad<T> yq = quad_of<T>(yr, half), uq = quad_of<T>(ur, half);
+                    f32x2 g[2], h[2], t[2];
+                    unpack2<T>(quad_of<T>(gr, half), g);
+                    const f32x2 s0 = sig[c][2 * half], s1 = sig[c][2 * half + 1];
+                    const Quad<T> sq = pack2<T>(mul2(g[0], s0), mul2(g[1], s1));             // s = io(g*sig)
+                    unpack2<T>(mul_quad<T>(sq, uq), h);                                      // h = io(s*u)
+                    f32x2 yv[2];
+                    unpack2<T>(yq, yv);
+                    unpack2<T>(pack2<T>(mul2(h[0], both(r)), mul2(h[1], both(r))), t);
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) t[i] = mul2(h[i], both(r));
-                    unpack2<T>(pack2<T>(t), t);
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
+                    for (int i = 0; i < 2; ++i) {
                         const f32x2 d = mul2(yv[i], t[i]);
-                        col[c][2 * i] += (double)lo_of(d);
-                        col[c][2 * i + 1] += (double)hi_of(d);
+                        col[c][4 * half + 2 * i] += (double)lo_of(d);
+                        col[c][4 * half + 2 * i + 1] += (double)hi_of(d);
                     }
+                    unpack2<T>(mul_quad<T>(yq, quad_of<T>(wr, half)), t);                    // gn = io(gy*io(w))
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) t[i] = sub2(mul2_exact(t[i], both(r), nz), mul2_exact(h[i], both(coef), nz));
+                    const Quad<T> dh = pack2<T>(t[0], t[1]);
+                    *reinterpret_cast<Quad<T>*>(d_up + (size_t)m * ld_d + k + 4 * half) = mul_quad<T>(dh, sq);
+                    unpack2<T>(mul_quad<T>(dh, uq), t);                                      // ds = io(dh*u)
+                    t[0] = mul2(mul2(t[0], s0), add2(both(1.0f), mul2_exact(g[0], sub2(both(1.0f), s0), nz)));
+                    t[1] = mul2(mul2(t[1], s1), add2(both(1.0f), mul2_exact(g[1], sub2(both(1.0f), s1), nz)));
+                    *reinterpret_cast<Quad<T>*>(d_gate + (size_t)m * ld_d + k + 4 * half) = pack2<T>(t[0], t[1]);
+                    asm volatile("" ::: "memory");
                 }
-                unpack2<T>(mul_raw(yr, weight_of(c)), t);                                 // gn = io(gy*io(w))
-#pragma unroll
-                for (int i = 0; i < 4; ++i) t[i] = sub2(mul2_exact(t[i], both(r), nz), mul2_exact(h[i], both(coef), nz));
-                const typename Io<T>::Raw dh = pack2<T>(t);
-                *reinterpret_cast<typename Io<T>::Raw*>(d_up + (size_t)m * ld_d + k) = mul_raw(dh, sr);
-                unpack2<T>(mul_raw(dh, ur), t);                                   // ds = io(dh*u)
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-                    t[i] = mul2(mul2(t[i], sig[c][i]), add2(both(1.0f), mul2_exact(g[i], sub2(both(1.0f), sig[c][i]), nz)));
-                *reinterpret_cast<typename Io<T>::Raw*>(d_gate + (size_t)m * ld_d + k) = pack2<T>(t);
             }
         }
         fetch(stage, m + SB_STAGES * G);             // into the slots just read, by the thread that read them
@@ -648,26 +646,33 @@ swiglu_backward_stream_kernel(const T* __restrict__ gy, const T* __restrict__ ga
     }
 }
 
-// dweight[k] = float(sum of the CTAs' partial sums), in a fixed order of additions for any grid (32 columns per CTA, the
-// 32 warps each add every 32nd partial in order, warp 0 adds their results in order).
+// dweight[k] = float(sum of the CTAs' partial sums).  A CTA covers 32 columns (one per lane); its W warps (8 or 32) each add
+// every W-th partial in order, and warp 0 adds their results in order: a fixed order of additions for a given width.
+// Few columns take 32 warps: 592 partials of 16 columns on 8 warps are a chain of dependent loads (10.9 us, 3.8 us with 32); where
+// the columns fill the SMs, 8 warps per CTA are enough and start sooner.
 __global__ void __launch_bounds__(1024)
 swiglu_dweight_kernel(const double* __restrict__ partial, int n_parts, float* __restrict__ dweight, int H) {
     __shared__ double part[32][32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
     const int k = blockIdx.x * 32 + lane;
     double s = 0.0;
     if (k < H) {
 #pragma unroll 8
-        for (int p = warp; p < n_parts; p += 32) s += partial[(size_t)p * H + k];
+        for (int p = warp; p < n_parts; p += warps) s += partial[(size_t)p * H + k];
     }
     part[warp][lane] = s;
     __syncthreads();
     if (warp == 0 && k < H) {
         double t = 0.0;
-#pragma unroll
-        for (int w = 0; w < 32; ++w) t += part[w][lane];
+        for (int w = 0; w < warps; ++w) t += part[w][lane];
         dweight[k] = (float)t;
     }
+}
+
+int dweight_threads(int columns) {
+    int sms = 148;
+    device_sm_count(&sms);
+    return (columns + 31) / 32 <= sms ? 1024 : 256;
 }
 
 int backward_grid(int M, int H, bool norm) {
@@ -857,7 +862,7 @@ static int launch_swiglu_backward_norm(const T* gy, const T* gate, const T* up, 
                                                                                partial, M, H);
     int rc = check_launch();
     if (rc != EL_OK) return rc;
-    swiglu_dweight_kernel<<<(H + 31) / 32, 1024, 0, st>>>(partial, grid, dweight, H);
+    swiglu_dweight_kernel<<<(H + 31) / 32, dweight_threads(H), 0, st>>>(partial, grid, dweight, H);
     return check_launch();
 }
 
@@ -885,7 +890,7 @@ static int launch_backward_stream(const T* gy, const T* gate, const T* up, long 
     swiglu_backward_stream_kernel<T, 2, THREADS, W_SLOTS><<<grid, threads, smem, st>>>(gy, gate, up, ld, weight, rstd, d_gate, d_up, ld_d, partial, M, H);
     rc = check_launch();
     if (rc != EL_OK) return rc;
-    swiglu_dweight_kernel<<<(H + 31) / 32, 1024, 0, st>>>(partial, grid, dweight, H);
+    swiglu_dweight_kernel<<<(H + 31) / 32, dweight_threads(H), 0, st>>>(partial, grid, dweight, H);
     return check_launch();
 }
 
