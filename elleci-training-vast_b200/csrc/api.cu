@@ -29,6 +29,7 @@ int launch_gemm_tc2(int mode, const int8_t* A, const void* B, int R, int C, int 
                     cudaStream_t st, void* const* dst, int n_dst, long long ld_total, long long col_offset, int rows_per_dst,
                     int first_dst, void* workspace, size_t workspace_bytes, bool lean);
 int gemm_tc2_k_split(int R, int C, int D);
+bool gemm_tc_narrow(int R, int C);
 int launch_reduce_scale_gather(const int* parts, int n_parts, void* const* out_all, int n_ranks, long long row_offset,
                                long long rows_total, const EpiParams& epi, int Mr, int C, cudaStream_t st);
 int launch_dw_hysteresis_tc(const int8_t* Gq, const int8_t* Xq, const float* g_absmax, uint8_t* Wp, uint8_t* Hp,
@@ -154,8 +155,13 @@ static int gemm_dispatch(int mode, const int8_t* A, const void* B, int R, int C,
     // auto: the tensor-core tiles are 128 rows deep; very small problems go to the CUDA-core kernel.  A few rows against a
     // large weight matrix still belong on the tensor-core kernel: the call is then the time to stream the packed weights
     // once, which the CUDA-core kernel takes twenty times longer for.
-    if (elig == EL_OK && (R >= 32 || (long long)C * D >= (1ll << 18)))
-        return launch_tc(mode, R <= 128, A, B, R, C, D, epi, status, st, ws, ws_bytes, lean);
+    if (elig == EL_OK && (R >= 32 || (long long)C * D >= (1ll << 18))) {
+        // Single CTAs for up to 128 rows and for problems with few tiles (figures at gemm_tc_narrow), unless the pair kernel splits
+        // the reduction of those (the caller's workspace) or is asked for in its register-lean form.
+        const bool split = mode != MODE_DW && ws != nullptr && gemm_tc2_k_split(R, C, D) > 1;
+        const bool single = R <= 128 || (!lean && !split && gemm_tc_narrow(R, C));
+        return launch_tc(mode, single, A, B, R, C, D, epi, status, st, ws, ws_bytes, lean);
+    }
     // layers of 16, 32 or 48 inputs: streaming kernels (see gemm_skinny.cu for both sides' times); a column count that no vector
     // store takes, an odd reduction or unaligned operands stay with the CUDA-core kernel
     if (elig != EL_OK && gemm_skinny_fits(mode, A, B, R, C, D, epi)) return launch_gemm_skinny(mode, A, B, R, C, D, epi, st);

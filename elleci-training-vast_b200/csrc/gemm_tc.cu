@@ -400,6 +400,19 @@ int gemm_tc_eligible(int mode, const void* A, const void* B, int R, int C, int D
     }
 }
 
+// 128-column tiles where 256-column ones would leave half of the SMs without a tile.  Forward and dX of such problems run on
+// single CTAs too: a pair covers 256 x 256 outputs, and with few tiles the time is the number of blocks each SM works through, not
+// the expansion work that pairs halve.  Measured (CUDA graph, 8 weight buffers), forward on pairs / here, us: 1024 tokens 1536 ->
+// 1536 13.7 / 10.5, 4096 tokens 4096 -> 512 20.9 / 18.0, 512 tokens 4096 -> 4096 20.9 / 17.9, 1024 tokens 1024 -> 1024 11.8 / 8.0;
+// one step beyond the rule, 2048 tokens 2048 -> 2048 15.7 / 16.0.  128 rows (always single CTAs) 4096 -> 11008: 27.2 us with
+// 256-column tiles, 18.4 with these.  Fused weight gradient, 256- / 128-column tiles: 1024 tokens 1536 -> 1536 16.9 / 10.8, 4096
+// tokens 4096 -> 512 23.9 / 17.5.
+bool gemm_tc_narrow(int R, int C) {
+    int sms = 0;
+    if (device_sm_count(&sms) != EL_OK) return false;
+    return 2LL * ((R + tc::BM - 1) / tc::BM) * ((C + 255) / 256) <= sms;
+}
+
 int launch_gemm_tc(int mode, const int8_t* A, const void* B, int R, int C, int D, const EpiParams& epi, int32_t* status,
                    cudaStream_t st) {
     int rc = gemm_tc_eligible(mode, A, B, R, C, D);
@@ -413,19 +426,20 @@ int launch_gemm_tc(int mode, const int8_t* A, const void* B, int R, int C, int D
     const int esz = (epi.out_dtype == EL_BF16 || epi.out_dtype == EL_F16) ? 2 : 4;
     p.vec_ok = ((reinterpret_cast<uintptr_t>(epi.out) & 15) == 0) && ((epi.ldo * esz) % 16 == 0);
     CUtensorMap tmA, tmB;
-    constexpr int BN = 256;
+    const bool narrow = gemm_tc_narrow(R, C);
+    const int BN = narrow ? 128 : 256;
     if (mode == MODE_FWD) {
         if ((rc = tc::make_map(&tmA, A, D, R, D, 128, 128, true)) != EL_OK) return rc;
         if ((rc = tc::make_map(&tmB, B, D / 4, C, D / 4, 32, BN, false)) != EL_OK) return rc;
-        return tc::launch_t<MODE_FWD, BN, EPI_SCALE>(tmA, tmB, p, st);
+        return narrow ? tc::launch_t<MODE_FWD, 128, EPI_SCALE>(tmA, tmB, p, st) : tc::launch_t<MODE_FWD, 256, EPI_SCALE>(tmA, tmB, p, st);
     } else if (mode == MODE_DX) {
         if ((rc = tc::make_map(&tmA, A, D, R, D, 128, 128, true)) != EL_OK) return rc;
         if ((rc = tc::make_map(&tmB, B, C / 4, D, C / 4, BN / 4, 128, false)) != EL_OK) return rc;
-        return tc::launch_t<MODE_DX, BN, EPI_SCALE>(tmA, tmB, p, st);
+        return narrow ? tc::launch_t<MODE_DX, 128, EPI_SCALE>(tmA, tmB, p, st) : tc::launch_t<MODE_DX, 256, EPI_SCALE>(tmA, tmB, p, st);
     } else {
         if ((rc = tc::make_map(&tmA, A, R, D, R, 128, 128, true)) != EL_OK) return rc;
         if ((rc = tc::make_map(&tmB, B, C, D, C, 128, 128, true)) != EL_OK) return rc;
-        return tc::launch_t<MODE_DW, BN, EPI_SCALE>(tmA, tmB, p, st);
+        return narrow ? tc::launch_t<MODE_DW, 128, EPI_SCALE>(tmA, tmB, p, st) : tc::launch_t<MODE_DW, 256, EPI_SCALE>(tmA, tmB, p, st);
     }
 }
 
@@ -446,6 +460,7 @@ int launch_dw_hysteresis_tc(const int8_t* Gq, const int8_t* Xq, const float* g_a
     CUtensorMap tmA, tmB;
     if ((rc = tc::make_map(&tmA, Gq, N, M, N, 128, 128, true)) != EL_OK) return rc;
     if ((rc = tc::make_map(&tmB, Xq, K, M, K, 128, 128, true)) != EL_OK) return rc;
+    if (gemm_tc_narrow(N, K)) return tc::launch_t<MODE_DW, 128, EPI_HYST>(tmA, tmB, p, st);
     return tc::launch_t<MODE_DW, 256, EPI_HYST>(tmA, tmB, p, st);
 }
 
