@@ -1,8 +1,9 @@
-"""Builds libelleci_int2.so (the C-ABI CUDA library) in-tree for sm_100a with nvcc.
+"""Builds libelleci_int2.so (the C-ABI CUDA library) in-tree for sm_100a with nvcc, and elleci_host_ops.so (the operators' host
+side, against the installed torch) with the C++ compiler.
 
     python elleci-training-vast_b200/build.py [--force]
 
-The output, lib/libelleci_int2.so, is git-ignored; it is rebuilt when a source file is newer.
+The outputs, lib/libelleci_int2.so and lib/elleci_host_ops.so, are git-ignored; they are rebuilt when a source file is newer.
 """
 from __future__ import annotations
 
@@ -15,6 +16,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB_DIR = os.path.join(HERE, "lib")
 LIB_PATH = os.path.join(LIB_DIR, "libelleci_int2.so")
+HOST_PATH = os.path.join(LIB_DIR, "elleci_host_ops.so")
 SOURCES = ["api.cu", "pack_quant.cu", "hysteresis.cu", "gemm_simple.cu", "gemm_skinny.cu", "gemm_tc.cu", "gemm_tc2.cu", "decode_tc.cu", "gemv_small.cu", "gemv_mma.cu", "rmsnorm.cu", "swiglu.cu", "peer_sync.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -29,9 +31,9 @@ def _nvcc() -> str:
 
 
 def _stale() -> bool:
-    if not os.path.exists(LIB_PATH):
+    if not os.path.exists(LIB_PATH) or not os.path.exists(HOST_PATH):
         return True
-    t = os.path.getmtime(LIB_PATH)
+    t = min(os.path.getmtime(LIB_PATH), os.path.getmtime(HOST_PATH))
     deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC)] + [os.path.join(HERE, "..", "include", "elleci_int2.h"),
                                                                  os.path.abspath(__file__)]
     return any(os.path.getmtime(d) > t for d in deps)
@@ -61,7 +63,26 @@ def build(force: bool = False, verbose: bool = False) -> str:
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"link failed:\n{r.stderr}")
+    build_host_ops()
     return LIB_PATH
+
+
+def build_host_ops() -> str:
+    """The extension module of csrc/host_ops.cpp: host code against the installed torch's headers, no CUDA code."""
+    import sysconfig
+
+    import torch
+    root = os.path.dirname(torch.__file__)
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f"-I{root}/include",
+           f"-I{root}/include/torch/csrc/api/include", f"-I{sysconfig.get_paths()['include']}", f"-I{cuda}/include",
+           os.path.join(CSRC, "host_ops.cpp"), "-o", HOST_PATH, f"-L{root}/lib", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch",
+           "-ltorch_python", "-ldl"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"building host_ops.cpp failed:\n{r.stderr}")
+    return HOST_PATH
 
 
 if __name__ == "__main__":

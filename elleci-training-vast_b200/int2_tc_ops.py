@@ -17,6 +17,7 @@ from typing import Optional, Tuple
 import torch
 
 from . import _lib
+from ._lib import host_ops
 from ._lib import EL_BF16, EL_F16, EL_F32, EL_FLAG_LEAN, EL_I32, EL_PATH_AUTO, EL_PATH_SIMPLE, EL_PATH_TC, ElleciError, call
 
 _DT = {torch.float16: EL_F16, torch.bfloat16: EL_BF16, torch.float32: EL_F32, torch.int32: EL_I32}
@@ -80,14 +81,7 @@ def quantize_activation_async(input: torch.Tensor, d_global_max: torch.Tensor) -
     (tc_quantize_activation_async, kernels/int2/int2_tc_ops.cpp:343-371).  `d_global_max` is accepted for
     signature compatibility; the absmax is accumulated in the returned scale tensor, so concurrent
     streams do not share scratch."""
-    _cuda(input, "Input")
-    _cuda(d_global_max, "d_global_max")
-    _require(input.dtype in (torch.float16, torch.bfloat16, torch.float32), "Input must be float16")
-    x = input.contiguous()
-    out = torch.empty(x.shape, dtype=torch.int8, device=x.device)
-    scale = torch.empty(1, dtype=torch.float32, device=x.device)
-    call("el_quantize_tensor", x.data_ptr(), _DT[x.dtype], out.data_ptr(), scale.data_ptr(), x.numel(), _stream())
-    return out, scale
+    return host_ops().quantize_tensor(input, d_global_max)
 
 
 def quantize_activation(input: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
@@ -108,78 +102,16 @@ def dequantize_activation(input_int8: torch.Tensor, scale: torch.Tensor, dtype: 
     return out
 
 
-_gemm_ws: dict = {}
-
-
-def _gemm_workspace(device: torch.device, mode: int, M: int, N: int, K: int):
-    """(pointer, bytes) of the scratch a GEMM with few output tiles uses to split its reduction over idle CTA pairs, or
-    (None, 0) when the shape is not split.  One buffer per device and stream, grown on demand; calls on one stream are
-    ordered, so they can share it."""
-    need = _lib.lib().el_gemm_workspace_bytes(mode, M, N, K)
-    if need == 0:
-        return None, 0
-    key = (device.index if device.index is not None else torch.cuda.current_device(), _stream())
-    buf = _gemm_ws.get(key)
-    if buf is None or buf.numel() < need:
-        buf = torch.empty(need, dtype=torch.uint8, device=device)
-        _gemm_ws[key] = buf
-    return buf.data_ptr(), buf.numel()
-
-
-def _gemm_fwd(Xq, W_packed, absmax, stride, gamma, out_dtype, path=EL_PATH_AUTO):
-    _cuda(Xq, "X_int8"); _cuda(W_packed, "W_packed"); _cuda(absmax, "d_scale_x")
-    _require(Xq.dtype == torch.int8, "X_int8 must be int8")
-    _require(W_packed.dtype == torch.uint8, "W_packed must be uint8")
-    _require(absmax.dtype == torch.float32, "d_scale_x must be float32")
-    _require(W_packed.dim() == 2, "W_packed must be 2-D [N, ceil(K/4)]")
-    N, pK = W_packed.shape
-    K = Xq.shape[-1]
-    _require((K + 3) // 4 == pK, f"Dimension mismatch: X has {K} features but W_packed has packed_K={pK} "
-                                 f"(expected ceil(K/4)={(K + 3) // 4})")
-    Xf = Xq.contiguous().view(-1, K)
-    M = Xf.shape[0]
-    _require(stride == 0 or absmax.numel() == M, "one absmax per token expected")
-    Wc = W_packed.contiguous()
-    Y = torch.empty(M, N, dtype=out_dtype, device=Xq.device)
-    st = device_status(Xq.device)
-    ws, ws_bytes = _gemm_workspace(Xq.device, 0, M, N, K) if (path & ~EL_FLAG_LEAN) in (EL_PATH_AUTO, EL_PATH_TC) else (None, 0)
-    call("el_gemm_fwd_ws", Xf.data_ptr(), Wc.data_ptr(), Y.data_ptr(), _DT[out_dtype], absmax.data_ptr(), stride,
-         float(gamma), M, N, K, path, ws, ws_bytes, st.data_ptr(), _stream())
-    _maybe_check(Xq.device)
-    return Y.view(*Xq.shape[:-1], N)
-
-
-def _gemm_dx(dYq, W_packed, absmax, stride, gamma, K, out_dtype, path=EL_PATH_AUTO):
-    _cuda(dYq, "dY_int8"); _cuda(W_packed, "W_packed"); _cuda(absmax, "d_scale_dy")
-    _require(dYq.dtype == torch.int8, "dY_int8 must be int8")
-    _require(W_packed.dtype == torch.uint8, "W_packed must be uint8")
-    _require(absmax.dtype == torch.float32, "d_scale_dy must be float32")
-    N, pK = W_packed.shape
-    _require(dYq.shape[-1] == N, f"dY has {dYq.shape[-1]} features but W_packed has {N} rows")
-    _require((K + 3) // 4 == pK, f"K={K} does not match W_packed's packed_K={pK}")
-    Yf = dYq.contiguous().view(-1, N)
-    M = Yf.shape[0]
-    _require(stride == 0 or absmax.numel() == M, "one absmax per token expected")
-    Wc = W_packed.contiguous()
-    dX = torch.empty(M, K, dtype=out_dtype, device=dYq.device)
-    st = device_status(dYq.device)
-    ws, ws_bytes = _gemm_workspace(dYq.device, 1, M, N, int(K)) if (path & ~EL_FLAG_LEAN) in (EL_PATH_AUTO, EL_PATH_TC) else (None, 0)
-    call("el_gemm_dx_ws", Yf.data_ptr(), Wc.data_ptr(), dX.data_ptr(), _DT[out_dtype], absmax.data_ptr(), stride,
-         float(gamma), M, N, int(K), path, ws, ws_bytes, st.data_ptr(), _stream())
-    _maybe_check(dYq.device)
-    return dX.view(*dYq.shape[:-1], K)
-
-
 def matmul_int8(X_int8: torch.Tensor, W_packed: torch.Tensor, d_scale_x: torch.Tensor, gamma: float,
                 out_dtype: torch.dtype = torch.float16, path: int = EL_PATH_AUTO) -> torch.Tensor:
     """Y = X_int8 @ W^T * (scale_x/127) * gamma, fp16 out (tc_matmul_int8, kernels/int2/int2_tc_ops.cpp:381-425)."""
-    return _gemm_fwd(X_int8, W_packed, d_scale_x, 0, gamma, out_dtype, path)
+    return host_ops().gemm_fwd(X_int8, W_packed, d_scale_x, 0, gamma, out_dtype, path)
 
 
 def backward_input_int8(dY_int8: torch.Tensor, W_packed: torch.Tensor, d_scale_dy: torch.Tensor, gamma: float, K: int,
                         out_dtype: torch.dtype = torch.float16, path: int = EL_PATH_AUTO) -> torch.Tensor:
     """dX = dY_int8 @ W * (scale_dy/127) * gamma (tc_backward_input_int8, kernels/int2/int2_tc_ops.cpp:435-470)."""
-    return _gemm_dx(dY_int8, W_packed, d_scale_dy, 0, gamma, K, out_dtype, path)
+    return host_ops().gemm_dx(dY_int8, W_packed, d_scale_dy, 0, gamma, int(K), out_dtype, path)
 
 
 def hysteresis_step_v2(dW: torch.Tensor, W_packed: torch.Tensor, H_packed: torch.Tensor, lr: float, lr_scale: float,
@@ -265,34 +197,10 @@ def quantize_rows(x: torch.Tensor, eps: float = ACT_EPS, fold_absmax: Optional[t
     maxima found elsewhere (reduced over the ranks of a column-sharded tensor); it is floored at eps in place
     and returned as the absmax.  A 2-D column window `x[:, a:b]` is read in place.  `out` (contiguous int8, M*K
     elements: a row block of a larger buffer, say) receives the quantised rows instead of a new tensor."""
-    _cuda(x, "x")
-    _require(x.dtype in _DT and x.dtype != torch.int32, "x must be float16, bfloat16 or float32")
-    xv, M, K, ld = _rows_view(x)
-    if out is None:
-        q = torch.empty(*x.shape[:-1], K, dtype=torch.int8, device=x.device)
-    else:
-        _require(out.is_cuda and out.dtype == torch.int8 and out.is_contiguous() and out.numel() == M * K,
-                 "out must be a contiguous int8 CUDA tensor of M*K elements")
-        q = out
-    if raw_absmax is None:
-        a = torch.empty(M, dtype=torch.float32, device=x.device)
-        mode = _lib.EL_QUANT_FULL
-    else:
-        _require(raw_absmax.dtype == torch.float32 and raw_absmax.numel() == M and raw_absmax.is_contiguous(),
-                 "raw_absmax must be a contiguous float32 [M]")
-        a = raw_absmax
-        mode = _lib.EL_QUANT_WITH_ABSMAX
-    fold_max = None
-    if fold_absmax is not None:
-        _require(fold_absmax.dtype == torch.float32 and fold_absmax.numel() == M, "fold_absmax must be float32 [M]")
-        fold_max = torch.zeros(1, dtype=torch.float32, device=x.device)
-    call("el_quantize_rows", xv.data_ptr(), _DT[xv.dtype], ld, q.data_ptr(), a.data_ptr(), M, K, float(eps), mode,
-         _ptr(fold_absmax), _ptr(fold_max), _stream())
-    return (q, a) if fold_absmax is None else (q, a, fold_max)
+    return host_ops().quantize_rows(x, eps, fold_absmax, raw_absmax, out)
 
 
 NORM_EPS = 1e-6            # default eps of the reference's pre-linear RMSNorm (core/bitnet/bitnet_int2_optimized.py:78)
-_norm_ws: dict = {}
 
 
 def rmsnorm_supported(x: torch.Tensor) -> bool:
@@ -307,50 +215,13 @@ def rmsnorm_quantize_rows(x: torch.Tensor, weight: torch.Tensor, norm_eps: float
     """The reference's pre-linear RMSNorm (`_ExtraRMSNorm`, core/bitnet/bitnet_int2_optimized.py:72-86) followed by
     the per-token quantiser, in one pass over x.  `weight` is the float32 norm weight [K].  Returns
     (q int8 like x, absmax float32 [M], rstd float32 [M]); q and absmax equal quantize_rows(norm(x))."""
-    _cuda(x, "x"); _cuda(weight, "weight")
-    _require(x.dtype in (torch.float16, torch.bfloat16, torch.float32), "x must be float16, bfloat16 or float32")
-    xv, M, K, ld = _rows_view(x)
-    _require(weight.dtype == torch.float32 and weight.numel() == K and weight.is_contiguous(), "weight must be a contiguous float32 [K]")
-    q = torch.empty(*x.shape[:-1], K, dtype=torch.int8, device=x.device)
-    a = torch.empty(M, dtype=torch.float32, device=x.device)
-    rstd = torch.empty(M, dtype=torch.float32, device=x.device)
-    call("el_rmsnorm_quantize_rows", xv.data_ptr(), _DT[xv.dtype], ld, weight.data_ptr(), float(norm_eps), q.data_ptr(),
-         a.data_ptr(), rstd.data_ptr(), M, K, float(quant_eps), _stream())
-    return q, a, rstd
+    return host_ops().rmsnorm_quantize_rows(x, weight, norm_eps, quant_eps)
 
 
 def rmsnorm_backward(g: torch.Tensor, x: torch.Tensor, weight: torch.Tensor, rstd: torch.Tensor):
     """Backward of the pre-linear RMSNorm for the gradient g with respect to its output (same shape and dtype as x).
     Returns (dx like x, dweight float32 [K])."""
-    _cuda(g, "g"); _cuda(x, "x")
-    _require(g.dtype == x.dtype and g.shape == x.shape, "g and x must have the same shape and dtype")
-    K = x.shape[-1]
-    gc, xc = g.contiguous(), x.contiguous()
-    M = xc.numel() // K if K else 0
-    _require(weight.dtype == torch.float32 and weight.numel() == K, "weight must be float32 [K]")
-    _require(rstd.dtype == torch.float32 and rstd.numel() == M, "rstd must be float32 [M]")
-    need = _lib.lib().el_rmsnorm_backward_workspace_bytes(K)
-    key = (x.device.index, _stream(), K)       # one scratch buffer per stream: calls on different streams may overlap
-    ws = _norm_ws.get(key)
-    if ws is None:
-        ws = torch.empty(need, dtype=torch.uint8, device=x.device)
-        _norm_ws[key] = ws
-    dx = torch.empty_like(xc)
-    dw = torch.empty(K, dtype=torch.float32, device=x.device)
-    call("el_rmsnorm_backward", gc.data_ptr(), xc.data_ptr(), _DT[xc.dtype], weight.contiguous().data_ptr(), rstd.data_ptr(),
-         dx.data_ptr(), dw.data_ptr(), ws.data_ptr(), need, M, K, _stream())
-    return dx.view_as(x), dw
-
-
-def _gate_up_views(gate: torch.Tensor, up: torch.Tensor):
-    """2-D views of gate and up with one common row pitch (the two halves of a [M, 2H] matrix qualify)."""
-    _require(gate.dtype == up.dtype and gate.shape == up.shape, "gate and up must have the same shape and dtype")
-    _require(gate.dtype in (torch.float16, torch.bfloat16, torch.float32), "gate and up must be float16, bfloat16 or float32")
-    gv, M, H, ld = _rows_view(gate)
-    uv, _, _, ld_u = _rows_view(up)
-    if ld_u != ld:
-        gv, uv, ld = gv.contiguous(), uv.contiguous(), H
-    return gv, uv, M, H, ld
+    return host_ops().rmsnorm_backward(g, x, weight, rstd)
 
 
 def swiglu_supported(gate: torch.Tensor) -> bool:
@@ -373,21 +244,7 @@ def prelinear_rows(x: torch.Tensor, up: Optional[torch.Tensor] = None, norm_weig
                    norm_eps: float = NORM_EPS) -> torch.Tensor:
     """The input of an INT2 layer as the fused training kernels form it (`silu(x) * up` when `up` is given, then the
     pre-linear RMSNorm when `norm_weight` is given), written out in x's dtype: what `linear_decode` is fed at inference."""
-    _cuda(x, "x")
-    if up is not None:
-        _cuda(up, "up")
-        xv, uv, M, K, ld = _gate_up_views(x, up)
-    else:
-        _require(x.dtype in (torch.float16, torch.bfloat16, torch.float32), "x must be float16, bfloat16 or float32")
-        xv, M, K, ld = _rows_view(x)
-        uv = None
-    if norm_weight is not None:
-        _require(norm_weight.dtype == torch.float32 and norm_weight.numel() == K and norm_weight.is_contiguous(),
-                 "norm_weight must be a contiguous float32 [K]")
-    y = torch.empty(*x.shape[:-1], K, dtype=xv.dtype, device=x.device)
-    call("el_prelinear_rows", xv.data_ptr(), _ptr(uv), _DT[xv.dtype], ld, _ptr(norm_weight), float(norm_eps), y.data_ptr(), M, K,
-         _stream())
-    return y
+    return host_ops().prelinear_rows(x, up, norm_weight, norm_eps)
 
 
 def swiglu_quantize_rows(gate: torch.Tensor, up: torch.Tensor, norm_weight: Optional[torch.Tensor] = None,
@@ -395,17 +252,7 @@ def swiglu_quantize_rows(gate: torch.Tensor, up: torch.Tensor, norm_weight: Opti
     """`F.silu(gate) * up` of the reference's feed-forward block (model/model.py:107-108), the pre-linear RMSNorm of the
     INT2 layer that consumes it (core/bitnet/bitnet_int2_optimized.py:201-204; skipped when `norm_weight` is None) and
     the per-token quantiser, in one pass.  Returns (q int8 like gate, absmax float32 [M], rstd float32 [M] or None)."""
-    _cuda(gate, "gate"); _cuda(up, "up")
-    gv, uv, M, H, ld = _gate_up_views(gate, up)
-    if norm_weight is not None:
-        _require(norm_weight.dtype == torch.float32 and norm_weight.numel() == H and norm_weight.is_contiguous(),
-                 "norm_weight must be a contiguous float32 [H]")
-    q = torch.empty(*gate.shape[:-1], H, dtype=torch.int8, device=gate.device)
-    a = torch.empty(M, dtype=torch.float32, device=gate.device)
-    rstd = torch.empty(M, dtype=torch.float32, device=gate.device) if norm_weight is not None else None
-    call("el_swiglu_quantize_rows", gv.data_ptr(), uv.data_ptr(), _DT[gv.dtype], ld, _ptr(norm_weight), float(norm_eps),
-         q.data_ptr(), a.data_ptr(), _ptr(rstd), M, H, float(quant_eps), _stream())
-    return q, a, rstd
+    return host_ops().swiglu_quantize_rows(gate, up, norm_weight, norm_eps, quant_eps)
 
 
 def swiglu_backward(gy: torch.Tensor, gate: torch.Tensor, up: torch.Tensor, norm_weight: Optional[torch.Tensor] = None,
@@ -413,32 +260,7 @@ def swiglu_backward(gy: torch.Tensor, gate: torch.Tensor, up: torch.Tensor, norm
     """Backward of swiglu_quantize_rows for the gradient gy with respect to the row that was quantised.  Returns
     (d_gate, d_up, d_norm_weight or None); with `out` (a [M, 2H] tensor of the I/O type) the two gradients are written
     into its halves (the gradient of a fused gate|up projection) and returned as views."""
-    _cuda(gy, "gy"); _cuda(gate, "gate"); _cuda(up, "up")
-    gv, uv, M, H, ld = _gate_up_views(gate, up)
-    _require(gy.dtype == gv.dtype and gy.numel() == M * H, "gy must have the shape and dtype of gate")
-    gyc = gy.contiguous()
-    if out is None:
-        d_gate, d_up, ld_d = torch.empty(M, H, dtype=gv.dtype, device=gv.device), torch.empty(M, H, dtype=gv.dtype, device=gv.device), H
-    else:
-        _require(out.dtype == gv.dtype and out.shape == (M, 2 * H) and out.is_contiguous(), "out must be a contiguous [M, 2H] tensor")
-        d_gate, d_up, ld_d = out[:, :H], out[:, H:], 2 * H
-    dw, ws, need = None, None, 0
-    if norm_weight is not None:
-        _require(norm_weight.dtype == torch.float32 and norm_weight.numel() == H, "norm_weight must be float32 [H]")
-        _require(rstd is not None and rstd.dtype == torch.float32 and rstd.numel() == M, "rstd must be float32 [M]")
-        need = _lib.lib().el_swiglu_backward_workspace_bytes(H)
-        key = (gv.device.index, _stream(), H)
-        ws = _norm_ws.get(key)
-        if ws is None:
-            ws = torch.empty(need, dtype=torch.uint8, device=gv.device)
-            _norm_ws[key] = ws
-        dw = torch.empty(H, dtype=torch.float32, device=gv.device)
-        norm_weight = norm_weight.contiguous()
-    call("el_swiglu_backward", gyc.data_ptr(), gv.data_ptr(), uv.data_ptr(), _DT[gv.dtype], ld, _ptr(norm_weight), _ptr(rstd),
-         d_gate.data_ptr(), d_up.data_ptr(), ld_d, _ptr(dw), _ptr(ws), need, M, H, _stream())
-    if out is None:
-        return d_gate.view_as(gate), d_up.view_as(up), dw
-    return d_gate, d_up, dw
+    return host_ops().swiglu_backward(gy, gate, up, norm_weight, rstd, out)
 
 
 def absmax_rows(x: torch.Tensor) -> torch.Tensor:
@@ -469,7 +291,7 @@ def scale_rows(acc: torch.Tensor, row_absmax: torch.Tensor, gamma: float, out_dt
 def matmul_rows(Xq: torch.Tensor, W_packed: torch.Tensor, row_absmax: torch.Tensor, gamma: float,
                 out_dtype: torch.dtype = torch.bfloat16, path: int = EL_PATH_AUTO) -> torch.Tensor:
     """Y[m,:] = (Xq[m,:] @ W^T) * (row_absmax[m]/127) * gamma: the forward GEMM with per-token scales."""
-    return _gemm_fwd(Xq, W_packed, row_absmax, 1, gamma, out_dtype, path)
+    return host_ops().gemm_fwd(Xq, W_packed, row_absmax, 1, gamma, out_dtype, path)
 
 
 def matmul_rows_gather(Xq: torch.Tensor, W_packed: torch.Tensor, row_absmax: torch.Tensor, gamma: float,
@@ -571,20 +393,13 @@ def counter_add(counter: torch.Tensor, delta: int = 1) -> None:
 def backward_input_rows(dYq: torch.Tensor, W_packed: torch.Tensor, row_absmax: torch.Tensor, gamma: float, K: int,
                         out_dtype: torch.dtype = torch.bfloat16, path: int = EL_PATH_AUTO) -> torch.Tensor:
     """dX[m,:] = (dYq[m,:] @ W) * (row_absmax[m]/127) * gamma: the dX GEMM with per-token scales."""
-    return _gemm_dx(dYq, W_packed, row_absmax, 1, gamma, K, out_dtype, path)
+    return host_ops().gemm_dx(dYq, W_packed, row_absmax, 1, gamma, int(K), out_dtype, path)
 
 
 def quantize_grad(dY: torch.Tensor, x_absmax: torch.Tensor, g_absmax: torch.Tensor) -> torch.Tensor:
     """Gq = int8 of (dY * x_absmax[m]/127) under the per-tensor maximum g_absmax[1]; a 2-D column window of a
     wider dY is read in place."""
-    _cuda(dY, "dY")
-    yv, M, N, ld = _rows_view(dY)
-    _require(x_absmax.dtype == torch.float32 and x_absmax.numel() == M, "x_absmax must be float32 [M]")
-    _require(g_absmax.dtype == torch.float32 and g_absmax.numel() == 1, "g_absmax must be float32 [1]")
-    Gq = torch.empty(*dY.shape[:-1], N, dtype=torch.int8, device=dY.device)
-    call("el_quantize_grad", yv.data_ptr(), _DT[yv.dtype], ld, x_absmax.data_ptr(), g_absmax.data_ptr(), Gq.data_ptr(), M, N,
-         _stream())
-    return Gq
+    return host_ops().quantize_grad(dY, x_absmax, g_absmax)
 
 
 def quantize_grad_scatter(dY: torch.Tensor, x_absmax: torch.Tensor, g_slots: torch.Tensor, recv_ptrs, row_offset: int,
@@ -647,6 +462,10 @@ def dw_hysteresis(Gq: torch.Tensor, Xq: torch.Tensor, g_absmax: torch.Tensor, W_
                   idx_base: int = 0) -> None:
     """Fused weight-gradient GEMM + hysteresis update, in place on W_packed / H_packed.  `step`: the step number, or an
     int32 [1] CUDA tensor that holds it (for launches recorded in a CUDA graph; see counter_add)."""
+    if not isinstance(step, torch.Tensor):
+        host_ops().dw_hysteresis(Gq, Xq, g_absmax, W_packed, H_packed, lr, lr_scale, int(threshold), decay, int(step) & 0xFFFFFFFF,
+                                 int(idx_base) & 0xFFFFFFFF)
+        return
     _cuda(Gq, "Gq"); _cuda(Xq, "Xq")
     _require(Gq.dtype == torch.int8 and Xq.dtype == torch.int8, "Gq and Xq must be int8")
     N, K = Gq.shape[-1], Xq.shape[-1]
@@ -657,19 +476,12 @@ def dw_hysteresis(Gq: torch.Tensor, Xq: torch.Tensor, g_absmax: torch.Tensor, W_
              "W_packed / H_packed shape mismatch")
     _require(W_packed.is_contiguous() and H_packed.is_contiguous(), "W_packed/H_packed must be contiguous")
     st = device_status(Gq.device)
-    if isinstance(step, torch.Tensor):          # the step number is read from device memory when the kernel runs
-        _cuda(step, "step")
-        _require(step.dtype == torch.int32 and step.numel() == 1, "a step tensor must be int32 [1]")
-        call("el_dw_hysteresis_step_ptr", G2.data_ptr(), X2.data_ptr(), g_absmax.data_ptr(), W_packed.data_ptr(),
-             H_packed.data_ptr(), float(lr), float(lr_scale), int(threshold), float(decay), step.data_ptr(),
-             int(idx_base) & 0xFFFFFFFF, M, N, K, st.data_ptr(), _stream())
-        return
-    step32 = int(step) & 0xFFFFFFFF
-    step_i = step32 - (1 << 32) if step32 >= (1 << 31) else step32
-    call("el_dw_hysteresis", G2.data_ptr(), X2.data_ptr(), g_absmax.data_ptr(), W_packed.data_ptr(), H_packed.data_ptr(),
-         float(lr), float(lr_scale), int(threshold), float(decay), step_i, int(idx_base) & 0xFFFFFFFF, M, N, K,
-         st.data_ptr(), _stream())
-    _maybe_check(Gq.device)
+    # the step number is read from device memory when the kernel runs
+    _cuda(step, "step")
+    _require(step.dtype == torch.int32 and step.numel() == 1, "a step tensor must be int32 [1]")
+    call("el_dw_hysteresis_step_ptr", G2.data_ptr(), X2.data_ptr(), g_absmax.data_ptr(), W_packed.data_ptr(),
+         H_packed.data_ptr(), float(lr), float(lr_scale), int(threshold), float(decay), step.data_ptr(),
+         int(idx_base) & 0xFFFFFFFF, M, N, K, st.data_ptr(), _stream())
 
 
 _decode_ws: dict = {}
@@ -680,33 +492,7 @@ def linear_decode(x: torch.Tensor, W_packed: torch.Tensor, gamma: float, out_dty
     """Small-M layer call (1 <= M <= 64 tokens): per-token quantisation + the weight-streaming tensor-core kernel.
     Same integers and rounding as quantize_rows + matmul_rows.  `workspace` (uint8, zero before first use, left
     zero) defaults to a cached buffer per device, stream and N, so calls on different streams never share one."""
-    _cuda(x, "x"); _cuda(W_packed, "W_packed")
-    _require(x.dtype in (torch.float16, torch.bfloat16, torch.float32), "x must be float16, bfloat16 or float32")
-    _require(W_packed.dtype == torch.uint8 and W_packed.dim() == 2, "W_packed must be uint8 [N, ceil(K/4)]")
-    N, pK = W_packed.shape
-    K = x.shape[-1]
-    _require((K + 3) // 4 == pK, f"x has {K} features but W_packed has packed_K={pK}")
-    xc = x.contiguous().view(-1, K)
-    M = xc.shape[0]
-    _require(1 <= M <= 64, "linear_decode takes 1..64 tokens; use quantize_rows + matmul_rows beyond that")
-    out_dtype = out_dtype or x.dtype
-    need = _lib.lib().el_decode_workspace_bytes(N)
-    if workspace is None:
-        key = (x.device.index, _stream(), N)       # per stream: calls that share a workspace must be stream-ordered
-        workspace = _decode_ws.get(key)
-        if workspace is None:
-            workspace = torch.zeros(need, dtype=torch.uint8, device=x.device)
-            _decode_ws[key] = workspace
-    _require(workspace.is_cuda and workspace.numel() * workspace.element_size() >= need, "workspace too small")
-    xq = torch.empty(M, K, dtype=torch.int8, device=x.device)
-    a = torch.empty(M, dtype=torch.float32, device=x.device)
-    Y = torch.empty(M, N, dtype=out_dtype, device=x.device)
-    st = device_status(x.device)
-    call("el_linear_decode", xc.data_ptr(), _DT[xc.dtype], W_packed.contiguous().data_ptr(), Y.data_ptr(), _DT[out_dtype],
-         float(gamma), xq.data_ptr(), a.data_ptr(), workspace.data_ptr(), workspace.numel() * workspace.element_size(),
-         M, N, K, st.data_ptr(), _stream())
-    _maybe_check(x.device)
-    return Y.view(*x.shape[:-1], N)
+    return host_ops().linear_decode(x, W_packed, gamma, out_dtype, workspace)
 
 
 def set_decode_overlap(enable: bool) -> None:
