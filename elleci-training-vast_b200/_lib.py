@@ -65,6 +65,7 @@ SIGNATURES = {
     "el_peer_put": [_vp, _vp, _i, C.c_size_t, C.c_size_t, _i, _vp],
     "el_quantize_grad_scatter": [_vp, _i, _ll, _vp, _vp, _i, _vp, _vp, _i, _ll, _i, _i, _vp],
     "el_linear_decode": [_vp, _i, _vp, _vp, _i, _f, _vp, _vp, _vp, C.c_size_t, _i, _i, _i, _vp, _vp],
+    "el_prelinear_decode": [_vp, _vp, _i, _ll, _vp, _f, _vp, _vp, _i, _f, _vp, _vp, _vp, C.c_size_t, _i, _i, _i, _vp, _vp],
     "el_linear_decode_static": [_vp, _i, _vp, _vp, _i, _f, _i, _i, _i, _vp, _vp],
     "el_hysteresis_from_dw": [_vp, _vp, _vp, _f, _f, _i, _f, _i, _i, _i, _u32, _i, _vp],
     "el_dw_hysteresis": [_vp, _vp, _vp, _vp, _vp, _f, _f, _i, _f, _i, _u32, _i, _i, _i, _vp, _vp],

@@ -50,6 +50,8 @@ size_t swiglu_backward_workspace_bytes(int H);
 int launch_sigmoid_fixed(const float* g, float* sig, long long n, cudaStream_t st);
 int launch_prelinear_rows(const void* x, const void* up, int dt, long long ld, const float* weight, float norm_eps, void* y, int M,
                           int K, cudaStream_t st);
+int launch_prelinear_quantize_perm(const void* x, const void* up, int dt, long long ld, const float* weight, float norm_eps, int8_t* q,
+                                   float* row_absmax, int M, int K, float quant_eps, cudaStream_t st);
 int launch_swiglu_quantize_rows(const void* gate, const void* up, int dt, long long ld, const float* weight, float norm_eps,
                                 int8_t* q, float* row_absmax, float* rstd, int M, int H, float quant_eps, cudaStream_t st);
 int launch_swiglu_backward(const void* gy, const void* gate, const void* up, int dt, long long ld, const float* weight,
@@ -561,6 +563,26 @@ int el_linear_decode(const void* x, int x_dtype, const uint8_t* W_packed, void* 
     }
     int rc = launch_quantize_rows_perm(x, x_dtype, K, xq_scratch, absmax, M, K, 1e-5f, (cudaStream_t)stream);
     if (rc != EL_OK) return rc;
+    const EpiParams epi{Y, (long long)N, out_dtype, absmax, 1, gamma};
+    return launch_decode_tc(xq_scratch, W_packed, epi, workspace, M, N, K, dev_status, (cudaStream_t)stream);
+}
+
+int el_prelinear_decode(const void* x, const void* up, int x_dtype, long long ld, const float* norm_weight, float norm_eps,
+                        const uint8_t* W_packed, void* Y, int out_dtype, float gamma, int8_t* xq_scratch, float* absmax,
+                        void* workspace, size_t workspace_bytes, int M, int N, int K, int32_t* dev_status, el_stream_t stream) {
+    if (M < 0 || N < 0 || K < 0 || !float_dtype(x_dtype) || !float_dtype(out_dtype) || ld < K || (!up && !norm_weight)) return EL_ERR_INVALID_ARG;
+    if (M == 0 || N == 0) return EL_OK;
+    if (M > 64 || K == 0 || K % 64 != 0 || K > 16384) return EL_ERR_UNSUPPORTED_SHAPE;
+    if (!x || !W_packed || !Y || !xq_scratch || !absmax || !workspace) return EL_ERR_NULL_PTR;
+    if (workspace_bytes < decode_workspace_bytes(N)) return EL_ERR_INVALID_ARG;
+    int rc = require_sm100();
+    if (rc != EL_OK) return rc;
+    rc = launch_prelinear_quantize_perm(x, up, x_dtype, ld, norm_weight, norm_eps, xq_scratch, absmax, M, K, 1e-5f, (cudaStream_t)stream);
+    if (rc != EL_OK) return rc;
+    if (M <= decode_mma_max_tokens() && gemv_mma_preq_fits(M, K)) {
+        const EpiParams gepi{Y, (long long)N, out_dtype, nullptr, 0, gamma};
+        return launch_gemv_mma_preq(xq_scratch, absmax, W_packed, gepi, M, N, K, (cudaStream_t)stream);
+    }
     const EpiParams epi{Y, (long long)N, out_dtype, absmax, 1, gamma};
     return launch_decode_tc(xq_scratch, W_packed, epi, workspace, M, N, K, dev_status, (cudaStream_t)stream);
 }

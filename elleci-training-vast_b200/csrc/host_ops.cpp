@@ -35,7 +35,7 @@ PyObject* g_decode_ws = nullptr;        // dict (device index, stream, N) -> wor
     X(el_quantize_rows) X(el_quantize_grad) X(el_quantize_tensor) X(el_rmsnorm_quantize_rows)                          \
     X(el_rmsnorm_backward) X(el_rmsnorm_backward_workspace_bytes) X(el_swiglu_quantize_rows) X(el_swiglu_backward)     \
     X(el_swiglu_backward_workspace_bytes) X(el_prelinear_rows) X(el_gemm_workspace_bytes) X(el_gemm_fwd_ws)            \
-    X(el_gemm_dx_ws) X(el_dw_hysteresis) X(el_linear_decode) X(el_decode_workspace_bytes)
+    X(el_gemm_dx_ws) X(el_dw_hysteresis) X(el_linear_decode) X(el_prelinear_decode) X(el_decode_workspace_bytes)
 struct Library {
 #define X(name) decltype(&::name) name = nullptr;
     EL_FUNCTIONS(X)
@@ -491,15 +491,31 @@ Tensor decode_workspace(const Tensor& x, void* st, int64_t N, size_t need) {
     return ws;
 }
 
+// linear_decode(x, W_packed, gamma, out_dtype, workspace, up, norm_weight, norm_eps)
 PyObject* linear_decode(PyObject* const* a) {
     const Tensor &x = cuda_arg(a[0], "x"), &W = cuda_arg(a[1], "W_packed");
-    const float gamma = (float)float_arg(a[2]);
+    const float gamma = (float)float_arg(a[2]), neps = (float)float_arg(a[7]);
     EL_REQUIRE(float_type(x.scalar_type()), "x must be float16, bfloat16 or float32");
     EL_REQUIRE(W.scalar_type() == at::kByte && W.dim() == 2, "W_packed must be uint8 [N, ceil(K/4)]");
     const int64_t N = W.size(0), pK = W.size(1), K = x.size(-1);
     if ((K + 3) / 4 != pK) raise("x has " + std::to_string(K) + " features but W_packed has packed_K=" + std::to_string(pK));
-    Tensor xc = x.contiguous(), Wc = W.contiguous();
-    const int64_t M = K ? xc.numel() / K : 0;
+    const bool gated = !is_none(a[5]), normed = !is_none(a[6]);
+    Rows v, u;
+    Tensor w;
+    if (gated) {
+        gate_up(x, cuda_arg(a[5], "up"), v, u);
+    } else if (normed) {
+        v = rows_view(x);
+    } else {
+        Tensor xc = x.contiguous();
+        v = {xc, K ? xc.numel() / K : 0, K, K};
+    }
+    if (normed) {
+        w = tensor_arg(a[6], "norm_weight");
+        EL_REQUIRE(w.scalar_type() == at::kFloat && w.numel() == K && w.is_contiguous(), "norm_weight must be a contiguous float32 [K]");
+    }
+    const int64_t M = v.M;
+    Tensor Wc = W.contiguous();
     EL_REQUIRE(M >= 1 && M <= 64, "linear_decode takes 1..64 tokens; use quantize_rows + matmul_rows beyond that");
     const at::ScalarType out_dt = is_none(a[3]) ? x.scalar_type() : dtype_arg(a[3]);
     const int dt = code_of(out_dt);
@@ -511,12 +527,20 @@ PyObject* linear_decode(PyObject* const* a) {
     // one allocation for the quantised tokens and, on a 16-byte boundary behind them, their maxima
     const int64_t xq_bytes = (M * K + 15) & ~(int64_t)15;
     Tensor scratch = new_empty(x, {xq_bytes + M * 4}, at::kByte), Y = like_rows(x, N, out_dt);
+    int8_t* xq = (int8_t*)scratch.data_ptr();
+    float* amax = (float*)((char*)scratch.data_ptr() + xq_bytes);
     int32_t* word = status_word(x);
-    call("el_linear_decode", [&] {
-        return g_lib.el_linear_decode(xc.data_ptr(), code_of(x.scalar_type()), (const uint8_t*)Wc.data_ptr(), Y.data_ptr(), dt, gamma,
-                                (int8_t*)scratch.data_ptr(), (float*)((char*)scratch.data_ptr() + xq_bytes), ws.data_ptr(), have, (int)M, (int)N,
-                                (int)K, word, st);
-    });
+    if (gated || normed)
+        call("el_prelinear_decode", [&] {
+            return g_lib.el_prelinear_decode(v.t.data_ptr(), gated ? u.t.data_ptr() : nullptr, code_of(x.scalar_type()), v.ld,
+                                             normed ? (const float*)w.data_ptr() : nullptr, neps, (const uint8_t*)Wc.data_ptr(), Y.data_ptr(), dt,
+                                             gamma, xq, amax, ws.data_ptr(), have, (int)M, (int)N, (int)K, word, st);
+        });
+    else
+        call("el_linear_decode", [&] {
+            return g_lib.el_linear_decode(v.t.data_ptr(), code_of(x.scalar_type()), (const uint8_t*)Wc.data_ptr(), Y.data_ptr(), dt, gamma, xq, amax,
+                                          ws.data_ptr(), have, (int)M, (int)N, (int)K, word, st);
+        });
     maybe_check(x);
     return wrap(Y);
 }
@@ -560,7 +584,7 @@ PyObject* set_hooks(PyObject* const* a) {
 PyMethodDef methods[] = {
     EL_ENTRY(quantize_rows, 5), EL_ENTRY(quantize_grad, 3), EL_ENTRY(quantize_tensor, 2), EL_ENTRY(rmsnorm_quantize_rows, 4),
     EL_ENTRY(rmsnorm_backward, 4), EL_ENTRY(swiglu_quantize_rows, 5), EL_ENTRY(swiglu_backward, 6), EL_ENTRY(prelinear_rows, 4),
-    EL_ENTRY(gemm_fwd, 7), EL_ENTRY(gemm_dx, 8), EL_ENTRY(dw_hysteresis, 11), EL_ENTRY(linear_decode, 5), EL_ENTRY(set_hooks, 5),
+    EL_ENTRY(gemm_fwd, 7), EL_ENTRY(gemm_dx, 8), EL_ENTRY(dw_hysteresis, 11), EL_ENTRY(linear_decode, 8), EL_ENTRY(set_hooks, 5),
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "elleci_host_ops", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 

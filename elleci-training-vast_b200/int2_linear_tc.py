@@ -251,10 +251,14 @@ class Int2LinearTC(nn.Module):
             return None
         if up is not None and (up.dtype != x.dtype or up.shape != x.shape):
             return None
-        y = x
-        if pre_norm is not None or up is not None:
-            y = int2_tc_ops.prelinear_rows(x, up, None if pre_norm is None else pre_norm.weight,
-                                           1e-6 if pre_norm is None else pre_norm.eps)
+        if pre_norm is None and up is None:
+            return int2_tc_ops.linear_decode(x, self.W_packed, self._gamma_cached, x.dtype)
+        weight, eps = (None, 1e-6) if pre_norm is None else (pre_norm.weight, pre_norm.eps)
+        # one call forms, quantises and multiplies; a lone ungated token of a very long row is the exception: there the
+        # one-launch GEMV that quantises for itself is the faster second half (16384 -> 4096: 14.9 us against 15.6)
+        if K <= 12288 or (K <= 16384 and (M > 1 or up is not None)):
+            return int2_tc_ops.linear_decode(x, self.W_packed, self._gamma_cached, x.dtype, None, up, weight, eps)
+        y = int2_tc_ops.prelinear_rows(x, up, weight, eps)
         return int2_tc_ops.linear_decode(y, self.W_packed, self._gamma_cached, x.dtype)
 
     # ---- weight update -----------------------------------------------------------------------------------------

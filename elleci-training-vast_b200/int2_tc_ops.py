@@ -488,11 +488,13 @@ _decode_ws: dict = {}
 
 
 def linear_decode(x: torch.Tensor, W_packed: torch.Tensor, gamma: float, out_dtype: Optional[torch.dtype] = None,
-                  workspace: Optional[torch.Tensor] = None) -> torch.Tensor:
+                  workspace: Optional[torch.Tensor] = None, up: Optional[torch.Tensor] = None,
+                  norm_weight: Optional[torch.Tensor] = None, norm_eps: float = NORM_EPS) -> torch.Tensor:
     """Small-M layer call (1 <= M <= 64 tokens): per-token quantisation + the weight-streaming tensor-core kernel.
     Same integers and rounding as quantize_rows + matmul_rows.  `workspace` (uint8, zero before first use, left
-    zero) defaults to a cached buffer per device, stream and N, so calls on different streams never share one."""
-    return host_ops().linear_decode(x, W_packed, gamma, out_dtype, workspace)
+    zero) defaults to a cached buffer per device, stream and N, so calls on different streams never share one.
+    `up` and `norm_weight` as in prelinear_rows (K <= 16384): the layer input is formed from x first, without a tensor for it."""
+    return host_ops().linear_decode(x, W_packed, gamma, out_dtype, workspace, up, norm_weight, norm_eps)
 
 
 def set_decode_overlap(enable: bool) -> None:

@@ -377,6 +377,14 @@ EL_API int el_linear_decode(const void* x, int x_dtype, const uint8_t* W_packed,
                             int8_t* xq_scratch, float* absmax, void* workspace, size_t workspace_bytes, int M, int N,
                             int K, int32_t* dev_status, el_stream_t stream);
 
+/* el_prelinear_rows followed by el_linear_decode without the tensor between them: the layer input is formed from x (and
+ * `up`: a gate; and / or the float32 norm_weight [K] of the pre-linear RMSNorm; at least one of the two), quantised per token
+ * by one small kernel, and the weight-streaming kernels take the quantised tokens.  Same output, bit for bit.  x and up have row
+ * pitch ld; K % 64 == 0, K <= 16384, 1 <= M <= 64; scratch, workspace and alignment as for el_linear_decode. */
+EL_API int el_prelinear_decode(const void* x, const void* up, int x_dtype, long long ld, const float* norm_weight, float norm_eps,
+                               const uint8_t* W_packed, void* Y, int out_dtype, float gamma, int8_t* xq_scratch, float* absmax,
+                               void* workspace, size_t workspace_bytes, int M, int N, int K, int32_t* dev_status, el_stream_t stream);
+
 /* el_linear_decode for callers that cannot give the library any device memory (no counterpart in the reference).
  * Serving processes that forbid cudaMalloc after start-up, runtimes that own the whole memory pool and hosts at
  * their memory budget cannot supply the scratch buffers of el_linear_decode; here the quantised tokens, their
