@@ -58,6 +58,7 @@ template <int BN> struct Cfg {
 struct Params {
     int R, C, D;                    // output rows, output columns, reduction depth
     int tiles_r, tiles_c, k_blocks;
+    int band_rows;                  // row tiles per band of the tile order (see tile_coords)
     EpiParams epi;
     int vec_ok;                     // output rows keep 16-byte alignment
     int32_t* status;
@@ -68,6 +69,22 @@ struct Params {
     HystParams hp;
     uint32_t idx_base;
 };
+
+// Tile order: bands of `band_rows` row tiles; inside a band the column tiles follow one another and the band's row tiles run
+// fastest.  Forward and dX take one band (row-fastest: few weight tiles at a time).  The weight gradient streams BOTH operands along
+// its reduction, and the 148 tiles of a round walk the tokens together: 16 row tiles x 9.25 column tiles need 2048 + 2368 operand
+// columns per round where 148 tiles of one or two columns need all rows' columns, more than L2 holds from about 6000 tokens
+// on.  Fused launch, row-fastest / bands of 16, us: 6144 tokens 4096 -> 11008 223 / 208, 8192 tokens 318 / 294, 65536 tokens 4096 ->
+// 16384 3460 / 2800 (best of three; under the power cap); 4096 tokens and layers with fewer row tiles the same.
+constexpr int DW_BAND_ROWS = 16;
+__device__ __forceinline__ void tile_coords(int t, const Params& p, int& tr, int& tc) {
+    const int per_band = p.band_rows * p.tiles_c;
+    const int band = t / per_band, in = t - band * per_band;
+    const int first = band * p.band_rows;
+    const int rows_here = min(p.band_rows, p.tiles_r - first);
+    tc = in / rows_here;
+    tr = first + (in - tc * rows_here);
+}
 
 // ---- the kernel ----------------------------------------------------------------------------------------------
 
@@ -128,7 +145,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             int s = 0;
             uint32_t ph = 0;
             for (int t = blockIdx.x; t < num_tiles && !failed; t += gridDim.x) {
-                const int r0 = (t % p.tiles_r) * BM, c0 = (t / p.tiles_r) * BN;
+                int tr, tc;
+                tile_coords(t, p, tr, tc);
+                const int r0 = tr * BM, c0 = tc * BN;
                 for (int kb = 0; kb < p.k_blocks; ++kb) {
                     if (!mbar_wait(bar_empty(s), ph ^ 1u, p.status, 1)) { failed = true; break; }
                     const uint32_t sa = smem_base + s * STAGE_BYTES, sb = sa + A_BYTES, sp = sb + C::B_BYTES;
@@ -193,7 +212,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         if (EPI == EPI_HYST) hp = hyst_resolve_step(p.hp);
         int it = 0;
         for (int t = blockIdx.x; t < num_tiles && !failed; t += gridDim.x, ++it) {
-            const int r0 = (t % p.tiles_r) * BM, c0 = (t / p.tiles_r) * BN;
+            int tr, tc;
+            tile_coords(t, p, tr, tc);
+            const int r0 = tr * BM, c0 = tc * BN;
             const int acc = it & 1;
             const uint32_t acc_ph = (uint32_t)(it >> 1) & 1u;
             const int row = r0 + row_in_tile;
@@ -378,6 +399,7 @@ static int launch_t(const CUtensorMap& tmA, const CUtensorMap& tmB, Params& p, c
     p.tiles_r = (p.R + BM - 1) / BM;
     p.tiles_c = (p.C + BN - 1) / BN;
     p.k_blocks = (p.D + BK - 1) / BK;
+    p.band_rows = (MODE == MODE_DW && p.tiles_r > DW_BAND_ROWS) ? DW_BAND_ROWS : p.tiles_r;
     const long long tiles = (long long)p.tiles_r * p.tiles_c;
     if (tiles == 0) return EL_OK;
     if (p.k_blocks == 0) return EL_ERR_UNSUPPORTED_SHAPE;
