@@ -71,7 +71,7 @@ int launch_gemv_mma(const void* x, int x_dtype, const uint8_t* Wp, const EpiPara
 bool gemv_mma_fits(int M, int K);
 int launch_gemv_small(const void* x, int x_dtype, const uint8_t* Wp, const EpiParams& epi, int M, int N, int K, cudaStream_t st, bool overlap);
 int decode_gemv_max_tokens();
-bool gemv_mma_preq_fits(int M, int K);
+bool gemv_mma_preq_fits(int M, int N, int K);
 int launch_gemv_mma_preq(const int8_t* xq, const float* amax, const uint8_t* Wp, const EpiParams& epi, int M, int N, int K,
                          cudaStream_t st);
 
@@ -554,7 +554,7 @@ int el_linear_decode(const void* x, int x_dtype, const uint8_t* W_packed, void* 
         const EpiParams gepi{Y, (long long)N, out_dtype, nullptr, 0, gamma};
         return launch_gemv_mma(x, x_dtype, W_packed, gepi, M, N, K, (cudaStream_t)stream, decode_overlap());
     }
-    if (M <= decode_mma_max_tokens() && gemv_mma_preq_fits(M, K)) {
+    if (M <= decode_mma_max_tokens() && gemv_mma_preq_fits(M, N, K)) {
         // more tokens: quantise them once, then the warp-MMA kernel on the quantised tokens, 32 at a time
         int rc = launch_quantize_rows_perm(x, x_dtype, K, xq_scratch, absmax, M, K, 1e-5f, (cudaStream_t)stream);
         if (rc != EL_OK) return rc;
@@ -579,7 +579,7 @@ int el_prelinear_decode(const void* x, const void* up, int x_dtype, long long ld
     if (rc != EL_OK) return rc;
     rc = launch_prelinear_quantize_perm(x, up, x_dtype, ld, norm_weight, norm_eps, xq_scratch, absmax, M, K, 1e-5f, (cudaStream_t)stream);
     if (rc != EL_OK) return rc;
-    if (M <= decode_mma_max_tokens() && gemv_mma_preq_fits(M, K)) {
+    if (M <= decode_mma_max_tokens() && gemv_mma_preq_fits(M, N, K)) {
         const EpiParams gepi{Y, (long long)N, out_dtype, nullptr, 0, gamma};
         return launch_gemv_mma_preq(xq_scratch, absmax, W_packed, gepi, M, N, K, (cudaStream_t)stream);
     }

@@ -378,7 +378,7 @@ int launch_gemv_small(const void* x, int x_dtype, const uint8_t* Wp, const EpiPa
 int launch_gemv_mma(const void* x, int x_dtype, const uint8_t* Wp, const EpiParams& epi, int M, int N, int K, cudaStream_t st,
                     bool overlap);
 bool gemv_mma_fits(int M, int K);
-bool gemv_mma_preq_fits(int M, int K);
+bool gemv_mma_preq_fits(int M, int N, int K);
 int launch_gemv_mma_preq(const int8_t* xq, const float* amax, const uint8_t* Wp, const EpiParams& epi, int M, int N, int K,
                          cudaStream_t st);
 bool decode_overlap();
@@ -412,7 +412,7 @@ extern "C" EL_API int el_linear_decode_static(const void* x, int x_dtype, const 
     }
     int8_t* xq = reinterpret_cast<int8_t*>(base + STATIC_XQ_OFFSET);
     float* absmax = reinterpret_cast<float*>(base + STATIC_ABSMAX_OFFSET);
-    if (M <= decode_mma_max_tokens() && gemv_mma_preq_fits(M, K)) {      // the warp-MMA kernel on tokens quantised once
+    if (M <= decode_mma_max_tokens() && gemv_mma_preq_fits(M, N, K)) {      // the warp-MMA kernel on tokens quantised once
         rc = launch_quantize_rows_perm(x, x_dtype, K, xq, absmax, M, K, 1e-5f, st);
         if (rc != EL_OK) return rc;
         const EpiParams gepi{Y, (long long)N, out_dtype, nullptr, 0, gamma};

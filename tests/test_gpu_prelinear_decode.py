@@ -39,3 +39,16 @@ def test_prelinear_decode_refuses_what_it_cannot_run(ops, pkg):
     with pytest.raises(pkg.ElleciError) as e:
         ops.linear_decode(x, torch.zeros(16, 4112, dtype=torch.uint8, device=DEV), 1.0, norm_weight=torch.ones(16448, device=DEV))
     assert e.value.status == pkg._lib.EL_ERR_UNSUPPORTED_SHAPE
+
+
+@pytest.mark.parametrize("M,K,N", [(32, 6208, 100), (17, 8192, 5000), (33, 11008, 2400), (64, 16384, 2384), (16, 16384, 40), (9, 12800, 16)])
+def test_decode_of_tokens_that_exceed_shared_memory(ops, M, K, N):
+    """Rows too long for shared memory are multiplied a chunk of the reduction at a time: chunk ends inside and at a round of the
+    sixteen warps, one and several row groups per CTA, a remainder of tokens; the output is the prefill kernels' bit for bit."""
+    g = torch.Generator(device=DEV).manual_seed(M + K + N)
+    x = torch.randn(M, K, generator=g, device=DEV).bfloat16()
+    W = torch.randint(0, 256, (N, K // 4), generator=g, device=DEV, dtype=torch.uint8)
+    Xq, a = ops.quantize_rows(x)
+    want = ops.matmul_rows(Xq, W, a, 0.02)
+    assert torch.equal(ops.linear_decode(x, W, 0.02), want)
+    ops.check_device_status(torch.device(DEV))
