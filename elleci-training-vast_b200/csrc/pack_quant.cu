@@ -491,7 +491,9 @@ template <typename T, bool VEC>
 __global__ void __launch_bounds__(256)
 quantize_grad_kernel(const T* __restrict__ dY, long long ld, const float* __restrict__ x_absmax,
                      const float* __restrict__ g_absmax, int8_t* __restrict__ Gq, int N) {
-    const int m = blockIdx.x;
+    // Last row first: the launch before this one (the per-token quantiser with its fold) read the same rows in ascending order,
+    // and the last ones are still in L2.  4096 x 11008 bf16 behind it: 32 -> 28.7 us; 16384 x 4096: 45.1 -> 43.0 us.
+    const int m = gridDim.x - 1 - blockIdx.x;
     const float g = *g_absmax;
     const float inv = (g >= 1e-30f) ? __fdiv_rn(127.0f, g) : 0.0f;
     const float sx = __fdiv_rn(x_absmax[m], 127.0f);
