@@ -514,18 +514,17 @@ swiglu_backward_kernel(const T* __restrict__ gy, const T* __restrict__ gate, con
     }
 }
 
-// Streaming form, with the norm: one CTA walks over the tokens with up to three rows of gy, gate and up ahead in thread-owned
+// Streaming form, with the norm: one CTA walks over the tokens with up to two rows of gy, gate and up ahead in thread-owned
 // slots (row_stream.cuh), the column sums of dweight and the row's sigmoids in registers, products of two 16-bit values
 // packed.  What bounds it: about 55 instructions per element, 22 of them the fixed sigmoid, and two float64 conversions;
 // memory 10 bytes.  (The one barrier of a token is a tenth of its time, so the next token's row sum is not pulled ahead as
 // in rmsnorm_backward_stream_kernel; its sigmoids would not fit in the registers either.)
 // 4096 tokens x 11008, bf16: 228 us with column sums in shared memory at a 64-byte stride (four-way bank conflicts) and
-// every row read twice from memory; 142 us in this form (L2 flushed, the dweight kernel
-// included).
-// W_SLOTS: the rounded weights lie in slots of their own instead of registers (rows of up to 11264 16-bit elements leave room;
-// with all of it in registers 150 bytes per thread spill, and with shared memory this full the spills go to L2: 163 us).
-constexpr int SB_STAGES = 3;
-template <typename T, int V, int THREADS, bool W_SLOTS>
+// every row read twice from memory; 138 us in this form (L2 flushed, the dweight kernel included).
+// Two stages, not three: a row takes 5 us, five times the memory latency, and what shared memory does not take stays L1 for the
+// 32 bytes per thread that spill.  The rounded weights lie in slots of their own instead of registers (150 bytes would spill).
+constexpr int SB_STAGES = 2;
+template <typename T, int V, int THREADS>
 __global__ void __launch_bounds__(THREADS, 1)
 swiglu_backward_stream_kernel(const T* __restrict__ gy, const T* __restrict__ gate, const T* __restrict__ up, long long ld,
                               const float* __restrict__ weight, const float* __restrict__ rstd, T* __restrict__ d_gate,
@@ -536,20 +535,16 @@ swiglu_backward_stream_kernel(const T* __restrict__ gy, const T* __restrict__ ga
     const Slots<T, 1, V> w_slots(ring + SB_STAGES * 3 * V * PIECES<T> * blockDim.x);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const f32x2 nz = negative_zeros();
-    typename Io<T>::Raw w[W_SLOTS ? 1 : V];
     double col[V][8];
 #pragma unroll
     for (int c = 0; c < V; ++c) {
         const int k = column_of<V>(c);
         float wv[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
         if (k < H) load8_w(weight + k, wv);
-        const typename Io<T>::Raw wr = Io<T>::pack(wv);      // rounds to the I/O type
-        if (W_SLOTS) w_slots.write(0, c, wr);
-        else w[W_SLOTS ? 0 : c] = wr;
+        w_slots.write(0, c, Io<T>::pack(wv));        // rounds to the I/O type
 #pragma unroll
         for (int i = 0; i < 8; ++i) col[c][i] = 0.0;
     }
-    auto weight_of = [&](int c) -> typename Io<T>::Raw { return W_SLOTS ? w_slots.read(0, c) : w[W_SLOTS ? 0 : c]; };
     auto fetch = [&](int stage, int m) {
         if (m < M) {
 #pragma unroll
@@ -585,7 +580,7 @@ swiglu_backward_stream_kernel(const T* __restrict__ gy, const T* __restrict__ ga
                     g[i] = mul2(g[i], sig[c][i]);
                 }
                 unpack2<T>(mul_raw(pack2<T>(g), slots.read(stage, 3 * c + 2)), g);           // h
-                unpack2<T>(mul_raw(slots.read(stage, 3 * c), weight_of(c)), gn);
+                unpack2<T>(mul_raw(slots.read(stage, 3 * c), w_slots.read(0, c)), gn);
                 dot += dot8(gn, g);
             }
         }
@@ -601,7 +596,7 @@ swiglu_backward_stream_kernel(const T* __restrict__ gy, const T* __restrict__ ga
             const int k = column_of<V>(c);
             if (k < H) {
                 const typename Io<T>::Raw yr = slots.read(stage, 3 * c), gr = slots.read(stage, 3 * c + 1), ur = slots.read(stage, 3 * c + 2);
-                const typename Io<T>::Raw wr = weight_of(c);
+                const typename Io<T>::Raw wr = w_slots.read(0, c);
 #pragma unroll
                 for (int half = 0; half < 2; ++half) {       // four elements at a time: eight spill
                     const Quad<T> yq = quad_of<T>(yr, half), uq = quad_of<T>(ur, half);
@@ -985,7 +980,7 @@ static int launch_swiglu_backward_norm(const T* gy, const T* gate, const T* up, 
     return check_launch();
 }
 
-template <typename T, int THREADS, bool W_SLOTS>
+template <typename T, int THREADS>
 static int launch_backward_stream(const T* gy, const T* gate, const T* up, long long ld, const float* weight, const float* rstd,
                                   T* d_gate, T* d_up, long long ld_d, float* dweight, double* partial, int M, int H, cudaStream_t st) {
     static DeviceOnce attr_once;
@@ -994,19 +989,19 @@ static int launch_backward_stream(const T* gy, const T* gate, const T* up, long 
     int rc = device_sm_count(&sms);
     if (rc != EL_OK) return rc;
     if (!attr_once.is_done(dev)) {
-        EL_CUDA_TRY(cudaFuncSetAttribute(swiglu_backward_stream_kernel<T, 2, THREADS, W_SLOTS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        EL_CUDA_TRY(cudaFuncSetAttribute(swiglu_backward_stream_kernel<T, 2, THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          226 * 1024));
         attr_once.mark(dev);
     }
     const int threads = stream_threads(H, 2);
-    const size_t smem = (size_t)(SB_STAGES * 3 + (W_SLOTS ? 1 : 0)) * 2 * PIECES<T> * sizeof(uint4) * threads;
+    const size_t smem = (size_t)(SB_STAGES * 3 + 1) * 2 * PIECES<T> * sizeof(uint4) * threads;
     // resident CTAs per SM by registers and shared memory, at most the four per SM that the workspace holds partials for
     int per_sm = THREADS / threads;
     const int by_smem = (int)((226u * 1024u) / smem);
     per_sm = per_sm < by_smem ? per_sm : by_smem;
     per_sm = per_sm < 1 ? 1 : (per_sm > 4 ? 4 : per_sm);
     const int grid = M < sms * per_sm ? M : sms * per_sm;
-    swiglu_backward_stream_kernel<T, 2, THREADS, W_SLOTS><<<grid, threads, smem, st>>>(gy, gate, up, ld, weight, rstd, d_gate, d_up, ld_d, partial, M, H);
+    swiglu_backward_stream_kernel<T, 2, THREADS><<<grid, threads, smem, st>>>(gy, gate, up, ld, weight, rstd, d_gate, d_up, ld_d, partial, M, H);
     rc = check_launch();
     if (rc != EL_OK) return rc;
     swiglu_dweight_kernel<<<(H + 31) / 32, dweight_threads(H), 0, st>>>(partial, grid, dweight, H);
@@ -1023,18 +1018,11 @@ static int launch_swiglu_backward_t(const T* gy, const T* gate, const T* up, lon
                                                                          nullptr, M, H);
         return check_launch();
     }
-    // Rows whose three stages of gy, gate and up fit in shared memory stream (16-bit types: 12288 columns, float32: 6144).
-    // Two vectors per thread: 80 registers at 768 threads.
-    const int threads = stream_threads(H, 2);
-#define EL_SGB(THREADS, W_SLOTS) return launch_backward_stream<T, THREADS, W_SLOTS>(gy, gate, up, ld, weight, rstd, d_gate, d_up, ld_d, dweight, partial, M, H, st)
-    if constexpr (sizeof(T) == 2) {
-        if (threads <= 704) EL_SGB(704, true);
-        if (threads <= 768) EL_SGB(768, false);
-    } else {
-        if (threads <= 352) EL_SGB(384, true);
-        if (threads <= 384) EL_SGB(384, false);
-    }
-#undef EL_SGB
+    // Rows of up to 12288 16-bit or 8192 float32 elements stream: two vectors per thread, 80 registers at 768 threads (float32: 120
+    // at 512, where two stages fill the shared memory).
+    constexpr int MAX_T = sizeof(T) == 2 ? 768 : 512;
+    if (stream_threads(H, 2) <= MAX_T)
+        return launch_backward_stream<T, MAX_T>(gy, gate, up, ld, weight, rstd, d_gate, d_up, ld_d, dweight, partial, M, H, st);
     return launch_swiglu_backward_norm<T, 6>(gy, gate, up, ld, weight, rstd, d_gate, d_up, ld_d, dweight, partial, M, H, st);
 }
 
