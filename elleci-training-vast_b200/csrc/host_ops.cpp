@@ -97,13 +97,26 @@ int code_of(at::ScalarType t) {
 
 void* stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
 
-// Runs a C-ABI call without the GIL (a full launch queue may block in it) and raises for a status other than 0.
-template <typename F>
-void call(const char* name, F&& f) {
+// A tensor's data pointer, null for an undefined one.  Throws for a tensor without storage (a functorch wrapper, a fake tensor),
+// so the operators read the pointers of their inputs first: nothing has then been allocated or cached.
+template <typename T = void> T* ptr(const Tensor& t) { return t.defined() ? static_cast<T*>(t.data_ptr()) : nullptr; }
+
+struct ReleasedGil {                    // gives the GIL up and takes it back on every way out of the scope
+    PyThreadState* state = PyEval_SaveThread();
+    ReleasedGil() = default;
+    ReleasedGil(const ReleasedGil&) = delete;
+    ~ReleasedGil() noexcept(false) { PyEval_RestoreThread(state); }      // ends the thread if the interpreter is shutting down
+};
+
+// Makes a C-ABI call without the GIL (a full launch queue may block in it) and raises for a status other than 0.  The arguments
+// are values by then: nothing that can throw or touches Python runs without the GIL.
+template <typename... P, typename... A>
+void call(const char* name, int (*fn)(P...), A... args) {
     int status;
-    Py_BEGIN_ALLOW_THREADS
-    status = f();
-    Py_END_ALLOW_THREADS
+    {
+        const ReleasedGil released;
+        status = fn(static_cast<P>(args)...);
+    }
     if (status != EL_OK) {
         PyObject* r = PyObject_CallFunction(g_check, "si", name, status);
         Py_XDECREF(r);
@@ -176,6 +189,7 @@ PyObject* quantize_rows(PyObject* const* a) {
     EL_REQUIRE(float_type(x.scalar_type()), "x must be float16, bfloat16 or float32");
     const float eps = (float)float_arg(a[1]);
     const Rows v = rows_view(x);
+    const void* xp = ptr(v.t);
     Tensor q, amax, fold_max, fold;
     if (is_none(a[4])) {
         q = like_rows(x, v.cols, at::kChar);
@@ -198,12 +212,8 @@ PyObject* quantize_rows(PyObject* const* a) {
         EL_REQUIRE(fold.scalar_type() == at::kFloat && fold.numel() == v.M, "fold_absmax must be float32 [M]");
         fold_max = at::zeros({1}, at::TensorOptions().device(x.device()).dtype(at::kFloat));
     }
-    void* st = stream();
-    call("el_quantize_rows", [&] {
-        return g_lib.el_quantize_rows(v.t.data_ptr(), code_of(x.scalar_type()), v.ld, (int8_t*)q.data_ptr(), (float*)amax.data_ptr(), (int)v.M,
-                                (int)v.cols, eps, mode, fold.defined() ? (const float*)fold.data_ptr() : nullptr,
-                                fold.defined() ? (float*)fold_max.data_ptr() : nullptr, st);
-    });
+    call("el_quantize_rows", g_lib.el_quantize_rows, xp, code_of(x.scalar_type()), v.ld, ptr<int8_t>(q), ptr<float>(amax), v.M, v.cols, eps,
+         mode, ptr<float>(fold), ptr<float>(fold_max), stream());
     if (fold.defined()) return tuple_of(wrap(q), wrap(amax), wrap(fold_max));
     return tuple_of(wrap(q), wrap(amax));
 }
@@ -215,12 +225,10 @@ PyObject* quantize_grad(PyObject* const* a) {
     EL_REQUIRE(xa.scalar_type() == at::kFloat && xa.numel() == v.M, "x_absmax must be float32 [M]");
     EL_REQUIRE(ga.scalar_type() == at::kFloat && ga.numel() == 1, "g_absmax must be float32 [1]");
     const int dt = code_of(dY.scalar_type());
+    const void* yp = ptr(v.t);
+    const float *xap = ptr<float>(xa), *gap = ptr<float>(ga);
     Tensor Gq = like_rows(dY, v.cols, at::kChar);
-    void* st = stream();
-    call("el_quantize_grad", [&] {
-        return g_lib.el_quantize_grad(v.t.data_ptr(), dt, v.ld, (const float*)xa.data_ptr(), (const float*)ga.data_ptr(), (int8_t*)Gq.data_ptr(),
-                                (int)v.M, (int)v.cols, st);
-    });
+    call("el_quantize_grad", g_lib.el_quantize_grad, yp, dt, v.ld, xap, gap, ptr<int8_t>(Gq), v.M, v.cols, stream());
     return wrap(Gq);
 }
 
@@ -229,11 +237,9 @@ PyObject* quantize_tensor(PyObject* const* a) {
     cuda_arg(a[1], "d_global_max");
     EL_REQUIRE(float_type(in.scalar_type()), "Input must be float16");
     Tensor x = in.contiguous();
+    const void* xp = ptr(x);
     Tensor out = new_empty(x, x.sizes(), at::kChar), scale = new_empty(x, {1}, at::kFloat);
-    void* st = stream();
-    call("el_quantize_tensor", [&] {
-        return g_lib.el_quantize_tensor(x.data_ptr(), code_of(x.scalar_type()), (int8_t*)out.data_ptr(), (float*)scale.data_ptr(), x.numel(), st);
-    });
+    call("el_quantize_tensor", g_lib.el_quantize_tensor, xp, code_of(x.scalar_type()), ptr<int8_t>(out), ptr<float>(scale), x.numel(), stream());
     return tuple_of(wrap(out), wrap(scale));
 }
 
@@ -244,12 +250,11 @@ PyObject* rmsnorm_quantize_rows(PyObject* const* a) {
     EL_REQUIRE(float_type(x.scalar_type()), "x must be float16, bfloat16 or float32");
     const Rows v = rows_view(x);
     EL_REQUIRE(w.scalar_type() == at::kFloat && w.numel() == v.cols && w.is_contiguous(), "weight must be a contiguous float32 [K]");
+    const void* xp = ptr(v.t);
+    const float* wp = ptr<float>(w);
     Tensor q = like_rows(x, v.cols, at::kChar), amax = new_empty(x, {v.M}, at::kFloat), rstd = new_empty(x, {v.M}, at::kFloat);
-    void* st = stream();
-    call("el_rmsnorm_quantize_rows", [&] {
-        return g_lib.el_rmsnorm_quantize_rows(v.t.data_ptr(), code_of(x.scalar_type()), v.ld, (const float*)w.data_ptr(), neps, (int8_t*)q.data_ptr(),
-                                        (float*)amax.data_ptr(), (float*)rstd.data_ptr(), (int)v.M, (int)v.cols, qeps, st);
-    });
+    call("el_rmsnorm_quantize_rows", g_lib.el_rmsnorm_quantize_rows, xp, code_of(x.scalar_type()), v.ld, wp, neps, ptr<int8_t>(q), ptr<float>(amax),
+         ptr<float>(rstd), v.M, v.cols, qeps, stream());
     return tuple_of(wrap(q), wrap(amax), wrap(rstd));
 }
 
@@ -263,14 +268,13 @@ PyObject* rmsnorm_backward(PyObject* const* a) {
     EL_REQUIRE(w.scalar_type() == at::kFloat && w.numel() == K, "weight must be float32 [K]");
     EL_REQUIRE(rstd.scalar_type() == at::kFloat && rstd.numel() == M, "rstd must be float32 [M]");
     const int dt = code_of(xc.scalar_type());
+    Tensor wc = w.contiguous();
+    const void *gp = ptr(gc), *xp = ptr(xc);
+    const float *wp = ptr<float>(wc), *rp = ptr<float>(rstd);
     const size_t need = g_lib.el_rmsnorm_backward_workspace_bytes((int)K);
-    Tensor ws = new_empty(x, {(int64_t)need}, at::kByte), wc = w.contiguous();
+    Tensor ws = new_empty(x, {(int64_t)need}, at::kByte);
     Tensor dx = new_empty(x, xc.sizes(), xc.scalar_type()), dw = new_empty(x, {K}, at::kFloat);
-    void* st = stream();
-    call("el_rmsnorm_backward", [&] {
-        return g_lib.el_rmsnorm_backward(gc.data_ptr(), xc.data_ptr(), dt, (const float*)wc.data_ptr(), (const float*)rstd.data_ptr(), dx.data_ptr(),
-                                   (float*)dw.data_ptr(), ws.data_ptr(), need, (int)M, (int)K, st);
-    });
+    call("el_rmsnorm_backward", g_lib.el_rmsnorm_backward, gp, xp, dt, wp, rp, ptr(dx), ptr<float>(dw), ptr(ws), need, M, K, stream());
     return tuple_of(wrap(dx), wrap(dw));
 }
 
@@ -296,15 +300,13 @@ PyObject* swiglu_quantize_rows(PyObject* const* a) {
     if (!is_none(a[2])) {
         w = tensor_arg(a[2], "norm_weight");
         EL_REQUIRE(w.scalar_type() == at::kFloat && w.numel() == g.cols && w.is_contiguous(), "norm_weight must be a contiguous float32 [H]");
-        rstd = new_empty(gate, {g.M}, at::kFloat);
     }
+    const void *gp = ptr(g.t), *up_p = ptr(u.t);
+    const float* wp = ptr<float>(w);
+    if (w.defined()) rstd = new_empty(gate, {g.M}, at::kFloat);
     Tensor q = like_rows(gate, g.cols, at::kChar), amax = new_empty(gate, {g.M}, at::kFloat);
-    void* st = stream();
-    call("el_swiglu_quantize_rows", [&] {
-        return g_lib.el_swiglu_quantize_rows(g.t.data_ptr(), u.t.data_ptr(), code_of(gate.scalar_type()), g.ld,
-                                       w.defined() ? (const float*)w.data_ptr() : nullptr, neps, (int8_t*)q.data_ptr(), (float*)amax.data_ptr(),
-                                       w.defined() ? (float*)rstd.data_ptr() : nullptr, (int)g.M, (int)g.cols, qeps, st);
-    });
+    call("el_swiglu_quantize_rows", g_lib.el_swiglu_quantize_rows, gp, up_p, code_of(gate.scalar_type()), g.ld, wp, neps, ptr<int8_t>(q),
+         ptr<float>(amax), ptr<float>(rstd), g.M, g.cols, qeps, stream());
     return tuple_of(wrap(q), wrap(amax), w.defined() ? wrap(rstd) : none());
 }
 
@@ -315,6 +317,7 @@ PyObject* swiglu_backward(PyObject* const* a) {
     const int64_t M = g.M, H = g.cols;
     EL_REQUIRE(gy.scalar_type() == gate.scalar_type() && gy.numel() == M * H, "gy must have the shape and dtype of gate");
     Tensor gyc = gy.contiguous(), dg, du, dw, ws, w, rstd;
+    const void *yp = ptr(gyc), *gp = ptr(g.t), *up_p = ptr(u.t);
     int64_t ld_d = H;
     const bool own = is_none(a[5]);
     if (own) {
@@ -342,13 +345,8 @@ PyObject* swiglu_backward(PyObject* const* a) {
     }
     const bool norm = w.defined();
     if (!norm && !is_none(a[4])) rstd = tensor_arg(a[4], "rstd");
-    void* st = stream();
-    call("el_swiglu_backward", [&] {
-        return g_lib.el_swiglu_backward(gyc.data_ptr(), g.t.data_ptr(), u.t.data_ptr(), code_of(gate.scalar_type()), g.ld,
-                                  norm ? (const float*)w.data_ptr() : nullptr, rstd.defined() ? (const float*)rstd.data_ptr() : nullptr,
-                                  dg.data_ptr(), du.data_ptr(), ld_d, norm ? (float*)dw.data_ptr() : nullptr, norm ? ws.data_ptr() : nullptr,
-                                  need, (int)M, (int)H, st);
-    });
+    call("el_swiglu_backward", g_lib.el_swiglu_backward, yp, gp, up_p, code_of(gate.scalar_type()), g.ld, ptr<float>(w), ptr<float>(rstd), ptr(dg),
+         ptr(du), ld_d, ptr<float>(dw), ptr(ws), need, M, H, stream());
     return tuple_of(wrap(dg), wrap(du), norm ? wrap(dw) : none());
 }
 
@@ -368,12 +366,10 @@ PyObject* prelinear_rows(PyObject* const* a) {
         w = tensor_arg(a[2], "norm_weight");
         EL_REQUIRE(w.scalar_type() == at::kFloat && w.numel() == v.cols && w.is_contiguous(), "norm_weight must be a contiguous float32 [K]");
     }
+    const void *xp = ptr(v.t), *up_p = ptr(u.t);
+    const float* wp = ptr<float>(w);
     Tensor y = like_rows(x, v.cols, x.scalar_type());
-    void* st = stream();
-    call("el_prelinear_rows", [&] {
-        return g_lib.el_prelinear_rows(v.t.data_ptr(), gated ? u.t.data_ptr() : nullptr, code_of(x.scalar_type()), v.ld,
-                                 w.defined() ? (const float*)w.data_ptr() : nullptr, neps, y.data_ptr(), (int)v.M, (int)v.cols, st);
-    });
+    call("el_prelinear_rows", g_lib.el_prelinear_rows, xp, up_p, code_of(x.scalar_type()), v.ld, wp, neps, ptr(y), v.M, v.cols, stream());
     return wrap(y);
 }
 
@@ -404,13 +400,12 @@ PyObject* gemm_fwd(PyObject* const* a) {
     const int64_t M = K ? Xf.numel() / K : Xf.reshape({-1, K}).size(0);
     EL_REQUIRE(stride == 0 || amax.numel() == M, "one absmax per token expected");
     const int dt = code_of(out_dt);
+    const int8_t* xp = ptr<int8_t>(Xf);
+    const uint8_t* wp = ptr<uint8_t>(Wc);
+    const float* ap = ptr<float>(amax);
     Tensor Y = like_rows(Xq, N, out_dt), ws = gemm_scratch(Xq, 0, M, N, K, path);
-    int32_t* word = status_word(Xq);
-    void* st = stream();
-    call("el_gemm_fwd_ws", [&] {
-        return g_lib.el_gemm_fwd_ws((const int8_t*)Xf.data_ptr(), (const uint8_t*)Wc.data_ptr(), Y.data_ptr(), dt, (const float*)amax.data_ptr(), stride,
-                              gamma, (int)M, (int)N, (int)K, path, ws.defined() ? ws.data_ptr() : nullptr, ws.defined() ? (size_t)ws.numel() : 0, word, st);
-    });
+    call("el_gemm_fwd_ws", g_lib.el_gemm_fwd_ws, xp, wp, ptr(Y), dt, ap, stride, gamma, M, N, K, path, ptr(ws), ws.defined() ? ws.numel() : 0,
+         status_word(Xq), stream());
     maybe_check(Xq);
     return wrap(Y);
 }
@@ -435,13 +430,12 @@ PyObject* gemm_dx(PyObject* const* a) {
     const int64_t M = N ? Yf.numel() / N : Yf.reshape({-1, N}).size(0);
     EL_REQUIRE(stride == 0 || amax.numel() == M, "one absmax per token expected");
     const int dt = code_of(out_dt);
+    const int8_t* yp = ptr<int8_t>(Yf);
+    const uint8_t* wp = ptr<uint8_t>(Wc);
+    const float* ap = ptr<float>(amax);
     Tensor dX = like_rows(dYq, K, out_dt), ws = gemm_scratch(dYq, 1, M, N, K, path);
-    int32_t* word = status_word(dYq);
-    void* st = stream();
-    call("el_gemm_dx_ws", [&] {
-        return g_lib.el_gemm_dx_ws((const int8_t*)Yf.data_ptr(), (const uint8_t*)Wc.data_ptr(), dX.data_ptr(), dt, (const float*)amax.data_ptr(), stride,
-                             gamma, (int)M, (int)N, (int)K, path, ws.defined() ? ws.data_ptr() : nullptr, ws.defined() ? (size_t)ws.numel() : 0, word, st);
-    });
+    call("el_gemm_dx_ws", g_lib.el_gemm_dx_ws, yp, wp, ptr(dX), dt, ap, stride, gamma, M, N, K, path, ptr(ws), ws.defined() ? ws.numel() : 0,
+         status_word(dYq), stream());
     maybe_check(dYq);
     return wrap(dX);
 }
@@ -461,12 +455,11 @@ PyObject* dw_hysteresis(PyObject* const* a) {
     const int threshold = (int)int_arg(a[7]);
     const int step = (int)(uint32_t)int_arg(a[9]);
     const uint32_t idx_base = (uint32_t)int_arg(a[10]);
-    int32_t* word = status_word(Gq);
-    void* st = stream();
-    call("el_dw_hysteresis", [&] {
-        return g_lib.el_dw_hysteresis((const int8_t*)G2.data_ptr(), (const int8_t*)X2.data_ptr(), (const float*)ga.data_ptr(), (uint8_t*)W.data_ptr(),
-                                (uint8_t*)H.data_ptr(), lr, lr_scale, threshold, decay, step, idx_base, (int)M, (int)N, (int)K, word, st);
-    });
+    const int8_t *gp = ptr<int8_t>(G2), *xp = ptr<int8_t>(X2);
+    const float* gap = ptr<float>(ga);
+    uint8_t *wp = ptr<uint8_t>(W), *hp = ptr<uint8_t>(H);
+    call("el_dw_hysteresis", g_lib.el_dw_hysteresis, gp, xp, gap, wp, hp, lr, lr_scale, threshold, decay, step, idx_base, M, N, K, status_word(Gq),
+         stream());
     maybe_check(Gq);
     return none();
 }
@@ -519,6 +512,9 @@ PyObject* linear_decode(PyObject* const* a) {
     EL_REQUIRE(M >= 1 && M <= 64, "linear_decode takes 1..64 tokens; use quantize_rows + matmul_rows beyond that");
     const at::ScalarType out_dt = is_none(a[3]) ? x.scalar_type() : dtype_arg(a[3]);
     const int dt = code_of(out_dt);
+    const void *xp = ptr(v.t), *up_p = ptr(u.t);
+    const float* nwp = ptr<float>(w);
+    const uint8_t* wp = ptr<uint8_t>(Wc);
     const size_t need = g_lib.el_decode_workspace_bytes((int)N);
     void* st = stream();
     Tensor ws = is_none(a[4]) ? decode_workspace(x, st, N, need) : tensor_arg(a[4], "workspace");
@@ -527,20 +523,14 @@ PyObject* linear_decode(PyObject* const* a) {
     // one allocation for the quantised tokens and, on a 16-byte boundary behind them, their maxima
     const int64_t xq_bytes = (M * K + 15) & ~(int64_t)15;
     Tensor scratch = new_empty(x, {xq_bytes + M * 4}, at::kByte), Y = like_rows(x, N, out_dt);
-    int8_t* xq = (int8_t*)scratch.data_ptr();
-    float* amax = (float*)((char*)scratch.data_ptr() + xq_bytes);
+    int8_t* xq = ptr<int8_t>(scratch);
+    float* amax = reinterpret_cast<float*>(xq + xq_bytes);
     int32_t* word = status_word(x);
     if (gated || normed)
-        call("el_prelinear_decode", [&] {
-            return g_lib.el_prelinear_decode(v.t.data_ptr(), gated ? u.t.data_ptr() : nullptr, code_of(x.scalar_type()), v.ld,
-                                             normed ? (const float*)w.data_ptr() : nullptr, neps, (const uint8_t*)Wc.data_ptr(), Y.data_ptr(), dt,
-                                             gamma, xq, amax, ws.data_ptr(), have, (int)M, (int)N, (int)K, word, st);
-        });
+        call("el_prelinear_decode", g_lib.el_prelinear_decode, xp, up_p, code_of(x.scalar_type()), v.ld, nwp, neps, wp, ptr(Y), dt, gamma, xq, amax,
+             ptr(ws), have, M, N, K, word, st);
     else
-        call("el_linear_decode", [&] {
-            return g_lib.el_linear_decode(v.t.data_ptr(), code_of(x.scalar_type()), (const uint8_t*)Wc.data_ptr(), Y.data_ptr(), dt, gamma, xq, amax,
-                                          ws.data_ptr(), have, (int)M, (int)N, (int)K, word, st);
-        });
+        call("el_linear_decode", g_lib.el_linear_decode, xp, code_of(x.scalar_type()), wp, ptr(Y), dt, gamma, xq, amax, ptr(ws), have, M, N, K, word, st);
     maybe_check(x);
     return wrap(Y);
 }

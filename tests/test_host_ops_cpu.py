@@ -47,3 +47,47 @@ def test_arguments_that_are_no_cuda_tensors_are_refused(pkg, call, message):
 def test_a_wrong_number_of_arguments_is_a_type_error(pkg):
     with pytest.raises(TypeError):
         pkg._lib.host_ops().quantize_rows(torch.zeros(2, 8))
+
+
+def _refused_calls(o, t):
+    """Every native operator on arguments that pass its checks; `t(shape, dtype)` makes them."""
+    f, i8, u8 = torch.float32, torch.int8, torch.uint8
+    x, row, one, w = t((4, 64), torch.bfloat16), t((4,), f), t((1,), f), t((64,), f)
+    xq, gq, W, H = t((4, 64), i8), t((4, 32), i8), t((32, 16), u8), t((32, 32), u8)
+    return {
+        "quantize_rows": lambda: o.quantize_rows(x),
+        "quantize_rows_fold": lambda: o.quantize_rows(x, fold_absmax=row),
+        "quantize_grad": lambda: o.quantize_grad(x, row, one),
+        "quantize_tensor": lambda: o.quantize_activation_async(x, one),
+        "rmsnorm_quantize_rows": lambda: o.rmsnorm_quantize_rows(x, w),
+        "rmsnorm_backward": lambda: o.rmsnorm_backward(x, x, w, row),
+        "swiglu_quantize_rows": lambda: o.swiglu_quantize_rows(x, x, w),
+        "swiglu_backward": lambda: o.swiglu_backward(x, x, x, w, row),
+        "prelinear_rows": lambda: o.prelinear_rows(x, x, w),
+        "gemm_fwd": lambda: o.matmul_rows(xq, W, row, 1.0),
+        "gemm_dx": lambda: o.backward_input_rows(gq, W, row, 1.0, 64),
+        "dw_hysteresis": lambda: o.dw_hysteresis(gq, xq, one, W, H, 0.1, 5.0, 3, 0.0, 1),
+        "linear_decode": lambda: o.linear_decode(x, W, 1.0),
+        "linear_decode_norm": lambda: o.linear_decode(x, W, 1.0, norm_weight=w),
+    }
+
+
+NATIVE_CALLS = sorted(_refused_calls(None, lambda s, d: torch.zeros(s, dtype=d)))
+
+
+@pytest.mark.parametrize("name", NATIVE_CALLS)
+def test_a_tensor_without_storage_is_refused_before_anything_is_cached(pkg, name):
+    """Under vmap a tensor passes every check but has no data pointer.  Reading it raises, as it did in the Python functions: with the GIL
+    held, before an output is allocated or a status word or decode workspace is created.  (The CUDA tensors are fake ones.)"""
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    o = pkg.int2_tc_ops
+    status, decode = dict(o._status_bufs), dict(o._decode_ws)
+
+    def call(batched):
+        def make(shape, dtype):
+            return (batched + torch.zeros(shape, device="cuda:0")).to(dtype)
+        return _refused_calls(o, make)[name]()
+
+    with FakeTensorMode(), pytest.raises(RuntimeError, match="Cannot access data pointer of Tensor that doesn't have storage"):
+        torch.func.vmap(call)(torch.zeros(3, 1, device="cuda:0"))
+    assert o._status_bufs == status and o._decode_ws == decode
