@@ -139,7 +139,8 @@ PyObject* tuple_of(A... items) {
     return t;
 }
 
-// The status word of x's device: created by the Python function once, kept for the life of the process there and here.
+// The status word of x's device: the one tensor that the Python function hands to every caller, kept here for the life of the
+// process (the reference is never given back, so the address stays good whatever becomes of the Python module's dict).
 int32_t* status_word(const Tensor& x) {
     static int32_t* words[64] = {};
     const int dev = x.device().index();
@@ -147,8 +148,8 @@ int32_t* status_word(const Tensor& x) {
     if (words[dev] == nullptr) {
         PyObject* d = PyObject_CallFunction(g_status_of, "N", THPDevice_New(x.device()));
         if (d == nullptr) throw PyError();
-        words[dev] = THPVariable_Unpack(d).data_ptr<int32_t>();
-        Py_DECREF(d);           // the Python module's dict keeps it
+        int32_t* word = THPVariable_Unpack(d).data_ptr<int32_t>();
+        if (words[dev] == nullptr) words[dev] = word;       // another thread may have come first; it holds the same tensor
     }
     return words[dev];
 }

@@ -49,8 +49,8 @@ def device_status(device: torch.device) -> torch.Tensor:
     key = (device.type, device.index if device.index is not None else torch.cuda.current_device())
     buf = _status_bufs.get(key)
     if buf is None:
-        buf = torch.zeros(1, dtype=torch.int32, device=device)
-        _status_bufs[key] = buf
+        # two threads may both come here: the first word stored is everybody's, the native calls keep its address
+        buf = _status_bufs.setdefault(key, torch.zeros(1, dtype=torch.int32, device=device))
     return buf
 
 

@@ -91,3 +91,20 @@ def test_a_tensor_without_storage_is_refused_before_anything_is_cached(pkg, name
     with FakeTensorMode(), pytest.raises(RuntimeError, match="Cannot access data pointer of Tensor that doesn't have storage"):
         torch.func.vmap(call)(torch.zeros(3, 1, device="cuda:0"))
     assert o._status_bufs == status and o._decode_ws == decode
+
+
+def test_threads_that_meet_in_the_first_call_share_one_status_word(pkg, monkeypatch):
+    """The native calls keep the address of a device's status word, so a second thread's first call must not replace it: here the
+    other thread's whole call runs while this one is still creating its tensor."""
+    o, dev = pkg.int2_tc_ops, torch.device("cpu", 0)
+    zeros, other = torch.zeros, []
+
+    def zeros_with_another_thread(*args, **kw):
+        if not other:
+            other.append(None)
+            other[0] = o.device_status(dev)
+        return zeros(*args, **kw)
+
+    monkeypatch.setattr(o, "_status_bufs", {})
+    monkeypatch.setattr(torch, "zeros", zeros_with_another_thread)
+    assert o.device_status(dev) is other[0] and o.device_status(dev) is other[0]
