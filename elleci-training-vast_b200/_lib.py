@@ -13,7 +13,6 @@ import os
 _HERE = os.path.dirname(os.path.abspath(__file__))
 # ELLECI_INT2_LIB points at another build of the same library (a debug or experimental build)
 LIB_PATH = os.environ.get("ELLECI_INT2_LIB") or os.path.join(_HERE, "lib", "libelleci_int2.so")
-HOST_PATH = os.path.join(_HERE, "lib", "elleci_host_ops.so")
 
 EL_OK = 0
 EL_ERR_INVALID_ARG, EL_ERR_NULL_PTR, EL_ERR_ALIGNMENT, EL_ERR_UNSUPPORTED_SHAPE = -1, -2, -3, -4
@@ -111,16 +110,18 @@ _host = None
 
 def host_ops():
     """The extension module with the operators that every layer step goes through (csrc/host_ops.cpp); raises if it has not
-    been built."""
+    been built for the running Python and torch."""
     global _host
     if _host is None:
-        if not os.path.exists(HOST_PATH):
+        from .build import host_path
+        path = host_path()
+        if not os.path.exists(path):
             raise ElleciError("load", EL_ERR_DEVICE,
-                              f"{HOST_PATH} is missing: build it with `python elleci-training-vast_b200/build.py` "
+                              f"{path} is missing: build it with `python elleci-training-vast_b200/build.py` "
                               "(there is no fallback path)")
         lib()
-        loader = importlib.machinery.ExtensionFileLoader("elleci_host_ops", HOST_PATH)
-        module = importlib.util.module_from_spec(importlib.machinery.ModuleSpec("elleci_host_ops", loader, origin=HOST_PATH))
+        loader = importlib.machinery.ExtensionFileLoader("elleci_host_ops", path)
+        module = importlib.util.module_from_spec(importlib.machinery.ModuleSpec("elleci_host_ops", loader, origin=path))
         loader.exec_module(module)
         from . import int2_tc_ops as ops
         module.set_hooks(check, ops.device_status, ops.check_device_status, ops._decode_ws, LIB_PATH)

@@ -3,7 +3,8 @@ side, against the installed torch) with the C++ compiler.
 
     python elleci-training-vast_b200/build.py [--force]
 
-The outputs, lib/libelleci_int2.so and lib/elleci_host_ops.so, are git-ignored; they are rebuilt when a source file is newer.
+The outputs, lib/libelleci_int2.so and lib/elleci_host_ops.<python>.torch-<version>.so, are git-ignored; they are rebuilt when a
+source file is newer, and the second one when Python or torch is another one.
 """
 from __future__ import annotations
 
@@ -16,7 +17,6 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB_DIR = os.path.join(HERE, "lib")
 LIB_PATH = os.path.join(LIB_DIR, "libelleci_int2.so")
-HOST_PATH = os.path.join(LIB_DIR, "elleci_host_ops.so")
 SOURCES = ["api.cu", "pack_quant.cu", "hysteresis.cu", "gemm_simple.cu", "gemm_skinny.cu", "gemm_tc.cu", "gemm_tc2.cu", "decode_tc.cu", "gemv_small.cu", "gemv_mma.cu", "rmsnorm.cu", "swiglu.cu", "peer_sync.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -25,15 +25,22 @@ NVCC_FLAGS = [
 ]
 
 
+def host_path() -> str:
+    """The extension module of csrc/host_ops.cpp for the running Python and torch.  It is compiled against their headers and holds for
+    no other version, so its name carries both: after an upgrade the file is missing (and built again), not loaded and wrong."""
+    import torch
+    return os.path.join(LIB_DIR, f"elleci_host_ops.{sys.implementation.cache_tag}.torch-{torch.__version__}.so")
+
+
 def _nvcc() -> str:
     cand = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "bin", "nvcc")
     return cand if os.path.exists(cand) else "nvcc"
 
 
 def _stale() -> bool:
-    if not os.path.exists(LIB_PATH) or not os.path.exists(HOST_PATH):
+    if not os.path.exists(LIB_PATH) or not os.path.exists(host_path()):
         return True
-    t = min(os.path.getmtime(LIB_PATH), os.path.getmtime(HOST_PATH))
+    t = min(os.path.getmtime(LIB_PATH), os.path.getmtime(host_path()))
     deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC)] + [os.path.join(HERE, "..", "include", "elleci_int2.h"),
                                                                  os.path.abspath(__file__)]
     return any(os.path.getmtime(d) > t for d in deps)
@@ -77,12 +84,12 @@ def build_host_ops() -> str:
     cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f"-I{root}/include",
            f"-I{root}/include/torch/csrc/api/include", f"-I{sysconfig.get_paths()['include']}", f"-I{cuda}/include",
-           os.path.join(CSRC, "host_ops.cpp"), "-o", HOST_PATH, f"-L{root}/lib", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch",
+           os.path.join(CSRC, "host_ops.cpp"), "-o", host_path(), f"-L{root}/lib", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch",
            "-ltorch_python", "-ldl"]
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"building host_ops.cpp failed:\n{r.stderr}")
-    return HOST_PATH
+    return host_path()
 
 
 if __name__ == "__main__":

@@ -1,8 +1,8 @@
 """The native operator calls (csrc/host_ops.cpp): the module loads, names every operator that int2_tc_ops forwards to, and refuses
 what the Python checks refused, with the same exception type and message.  No call here reaches a GPU."""
-import re
-
+import importlib.util
 import os
+import re
 
 import pytest
 import torch
@@ -108,3 +108,17 @@ def test_threads_that_meet_in_the_first_call_share_one_status_word(pkg, monkeypa
     monkeypatch.setattr(o, "_status_bufs", {})
     monkeypatch.setattr(torch, "zeros", zeros_with_another_thread)
     assert o.device_status(dev) is other[0] and o.device_status(dev) is other[0]
+
+
+def test_a_module_built_for_another_torch_is_not_loaded(pkg, monkeypatch):
+    """The extension module is compiled against one torch: under another one it counts as not built, to the loader and to the build."""
+    spec = importlib.util.spec_from_file_location("_elleci_build", os.path.join(ROOT, "elleci-training-vast_b200", "build.py"))
+    build = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(build)
+    built = build.host_path()
+    assert os.path.exists(built)
+    monkeypatch.setattr(torch, "__version__", "0.0.0+other")
+    assert build.host_path() != built and build._stale()
+    monkeypatch.setattr(pkg._lib, "_host", None)
+    with pytest.raises(pkg.ElleciError, match="is missing: build it with"):
+        pkg._lib.host_ops()
