@@ -21,6 +21,7 @@ pkg = load_package()
 layer = pkg.BitLinearInt2(64, 128, use_extra_rmsnorm=False).to("cuda").eval()
 x = torch.randn(3, 4, 64, device="cuda", dtype=torch.bfloat16)
 with torch.no_grad():
+    layer(x)                    # the first call draws the weights
     try:
         torch.func.vmap(layer)(x)
     except RuntimeError as e:
