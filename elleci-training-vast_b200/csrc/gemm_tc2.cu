@@ -95,7 +95,8 @@ __device__ __forceinline__ void item_coords(int w, int num_tiles, const Params& 
 // 160 registers per thread: the CTA fills the SM's register file.  LEAN = true: one image, the next block's loads issued
 // right after the current one has been expanded, at most 128 registers: a quarter of the register file stays free and a
 // kernel that needs no shared memory (the peer pushes of a multi-GPU step, on a side stream) can run beside this
-// persistent one.  The lean form is about 9 % slower on its own (2140 against 2350 TOP/s at 4096 -> 11008).
+// persistent one.  On its own it runs at the same speed at the sizes measured (4096 tokens 4096 -> 11008 and 11008 -> 4096, forward / dX:
+// 138 / 140 and 142 / 136 us against 138 / 142 and 142 / 138; before the handshakes got shorter it was 9 % slower).
 template <int MODE, bool LEAN>
 __global__ void __maxnreg__(LEAN ? 128 : 168)
 gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ OutMaps outs, const Params p) {
@@ -110,13 +111,14 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     //   full   (leader's copy is used) one phase = both CTAs' A tiles landed (transaction bytes) + both halves expanded
     //          (one arrival per CTA's transform warp) + the leader producer's expect-arrival
     //   empty  (local) the MMAs that read stage s have completed
-    // The kernel is bound by the latency of this handshake chain, so the MMA-issuing thread waits on ONE barrier and makes
-    // ONE commit per block, which arrives on both CTAs' "empty" barriers, and arrivals across the pair carry no wider memory
-    // ordering than they need (tc_ptx.cuh).  Passing the peer's release through the leader's producer was tried and lost a
-    // third of the throughput: the relay added a hop to the chain.
-    // 4096 tokens, 4096 -> 11008 / 11008 -> 4096, bf16 out, L2 flushed: forward 157 / 173 us with two commits, cluster-scope
-    // arrivals and block coordinates divided out per block; 137 / 140 us now
-    // (2700 / 2640 TOP/s); dX 169 / 155 -> 138 / 134 us.  (Two boxes; the faster one gave 133 / 136 and 136 / 131.)
+    // The latency of this handshake chain was the kernel's bound, so the MMA-issuing thread waits on ONE barrier and makes ONE
+    // commit per block, which arrives on both CTAs' "empty" barriers, and the arrivals of the transform warps release their
+    // shared-memory writes and nothing else (tc_ptx.cuh).  Passing the peer's release through the leader's producer was tried and
+    // lost a third of the throughput: the relay added a hop to the chain.  What is left above the MMAs now is the shared memory
+    // that the expansion and the epilogue share with them (without both, 111 us).
+    // 4096 tokens, 4096 -> 11008 / 11008 -> 4096, bf16 out, L2 flushed, events around the call: forward 157 / 173 us with two
+    // commits, full cluster-scope releases and block coordinates divided out per block, 138 / 142 us now (2670 / 2600 TOP/s); dX
+    // 169 / 155 -> 142 / 138 us.  Boxes differ: 133 / 136 forward on the fastest seen, 146 / 145 on the slowest.
     auto bar_full = [&](int s) { return bars + 8u * s; };
     auto bar_empty = [&](int s) { return bars + 8u * (DA + s); };
     static_assert(DA == DB, "the A and B rings advance in lockstep");
@@ -392,7 +394,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             }
             fence_async_smem();
             __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(mapa_u32(bar_full(sb_i), 0));
+            if (lane == 0) mbar_arrive_cluster_smem(mapa_u32(bar_full(sb_i), 0));
             if (!LEAN && more) {
 #pragma unroll
                 for (int j = 0; j < 8; ++j) cur[j] = nxt[j];

@@ -151,14 +151,19 @@ __device__ __forceinline__ uint32_t mapa_u32(uint32_t addr, uint32_t rank) {
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
     return r;
 }
-// Arrive on a barrier given by its cluster-wide address; works for the own CTA too.  The arrival hands nothing to generic
-// reads of the other CTA: what it announces are writes to the OWN shared memory that only the async proxy reads (ordered by
-// the fence.proxy.async before it) and finished tensor-memory reads (ordered by tcgen05.wait::ld and the tcgen05 fences).  So
-// it takes the instruction's default scope.  With .release.cluster the arriving thread waited until all its earlier memory
-// operations were visible to the whole cluster, the packed weights of its NEXT block still on their way from L2 among
-// them: forward 4096 x 11008 x 4096 156 us, dX 169 us; with the default scope 146 and 145 us.
+// Arrive on a barrier given by its cluster-wide address; works for the own CTA too.  The waiter may be in the other CTA, so the
+// release has cluster scope (the instruction's default covers the own CTA only).
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+// The same, announcing only what this thread (and its warp, after __syncwarp) has written to its own shared memory: the fence
+// releases those writes at cluster scope and the arrival itself orders nothing.  A full release waits until all earlier memory
+// operations of the thread are visible to the cluster, the packed weights of its NEXT block still on their way from L2 among them.
+// Pair GEMM, 4096 tokens 4096 -> 11008 with one arrival per expanded block: a full release 149 us forward, 157 us dX (with the loads
+// issued after the arrival, 156 / 169 before it), this form 138 / 142 us.
+__device__ __forceinline__ void mbar_arrive_cluster_smem(uint32_t cluster_addr) {
+    asm volatile("fence.release.sync_restrict::shared::cta.cluster;\n\t"
+                 "mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 __device__ __forceinline__ bool mbar_try_cluster(uint32_t bar, uint32_t parity) {
     uint32_t ok;
