@@ -1,4 +1,5 @@
-// Decode GEMV for a few to 32 tokens, one launch: Y[m,n] = (sum_k Q(x)[m,k]*Wq[n,k]) * (absmax[m]/127) * gamma.
+// Decode GEMV on the warp-level int8 MMA: Y[m,n] = (sum_k Q(x)[m,k]*Wq[n,k]) * (absmax[m]/127) * gamma.  Up to 8 tokens that fit
+// in shared memory as one launch that quantises them itself; up to 64 tokens that arrive quantised, one launch per 32 of them.
 //
 // The call is bound by streaming W_packed once and by the 2-bit -> int8 expansion of the weights; the products themselves
 // are few.  With more than a handful of tokens the dp4a of the CUDA-core GEMV (one per token and 4 weights) outgrow the
@@ -315,16 +316,9 @@ int launch_gemv_mma_t(const T* x, const int8_t* xq, const float* amax, const uin
     return EL_ERR_UNSUPPORTED_SHAPE;
 }
 
-template <typename T>
-int launch_gemv_mma_m(const T* x, const uint8_t* Wp, const EpiParams& epi, int M, int N, int K, cudaStream_t st, bool overlap) {
-    if (M <= 8) return launch_gemv_mma_t<T, 1, false>(x, nullptr, nullptr, Wp, epi, M, N, K, st, overlap);
-    if (M <= 16) return launch_gemv_mma_t<T, 2, false>(x, nullptr, nullptr, Wp, epi, M, N, K, st, overlap);
-    return launch_gemv_mma_t<T, 4, false>(x, nullptr, nullptr, Wp, epi, M, N, K, st, overlap);
-}
-
 }  // namespace
 
-// Whether launch_gemv_mma takes the problem: up to 32 tokens whose int8 image fits in shared memory.
+// Whether the int8 image of up to 32 tokens fits in shared memory at once.
 bool gemv_mma_fits(int M, int K) {
     if (M < 1 || M > 32 || K <= 0 || K % 64 != 0) return false;
     const int mt = M <= 8 ? 8 : (M <= 16 ? 16 : 32);
@@ -332,15 +326,16 @@ bool gemv_mma_fits(int M, int K) {
     return 256 + kblocks * 16 * mt * sizeof(uint4) + 2 * 16 * mt * sizeof(int) <= GM_SMEM_MAX;
 }
 
-// x [M,K] float (16-byte aligned rows), K % 64 == 0.  epi.absmax is not read: the scales are computed here.
+// One launch that quantises the tokens itself, for up to 8 of them (gemv_mma_fits).  x [M,K] float (16-byte aligned rows),
+// K % 64 == 0.  epi.absmax is not read: the scales are computed here.
 int launch_gemv_mma(const void* x, int x_dtype, const uint8_t* Wp, const EpiParams& epi, int M, int N, int K, cudaStream_t st,
                     bool overlap) {
-    if (!gemv_mma_fits(M, K)) return EL_ERR_UNSUPPORTED_SHAPE;
+    if (M > DECODE_MMA_SINGLE_MAX || !gemv_mma_fits(M, K)) return EL_ERR_UNSUPPORTED_SHAPE;
     if ((reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(Wp) & 15)) return EL_ERR_ALIGNMENT;
     switch (x_dtype) {
-        case EL_BF16: return launch_gemv_mma_m((const __nv_bfloat16*)x, Wp, epi, M, N, K, st, overlap);
-        case EL_F16: return launch_gemv_mma_m((const __half*)x, Wp, epi, M, N, K, st, overlap);
-        case EL_F32: return launch_gemv_mma_m((const float*)x, Wp, epi, M, N, K, st, overlap);
+        case EL_BF16: return launch_gemv_mma_t<__nv_bfloat16, 1, false>((const __nv_bfloat16*)x, nullptr, nullptr, Wp, epi, M, N, K, st, overlap);
+        case EL_F16: return launch_gemv_mma_t<__half, 1, false>((const __half*)x, nullptr, nullptr, Wp, epi, M, N, K, st, overlap);
+        case EL_F32: return launch_gemv_mma_t<float, 1, false>((const float*)x, nullptr, nullptr, Wp, epi, M, N, K, st, overlap);
         default: return EL_ERR_INVALID_ARG;
     }
 }
@@ -352,8 +347,9 @@ int launch_gemv_mma(const void* x, int x_dtype, const uint8_t* Wp, const EpiPara
 // is safe whatever else the stream holds, because the quantiser itself started after all earlier work had finished.
 // Any number of tokens: they are taken 32 (or 16, or 8) at a time, one launch each; the weights of the later launches
 // come from L2.  Rows whose tokens do not fit in shared memory are taken in chunks of the reduction, as long as the row groups'
-// sums leave room for one round of blocks (N up to about 84000 at 32 tokens); a second launch of three or more chunks is
-// slower than the tcgen05 stream-K kernel (decode_tc.cu), which keeps those.  Whole call on that kernel / here, us: 11008 -> 4096 24
+// sums leave room for one round of blocks (at 17-32 tokens: 35 row groups per CTA, N up to 35*148*16 = 82880).  With more than 32
+// tokens, rows beyond 12288 (four or more chunks for every 32 tokens) are faster on the tcgen05 stream-K kernel (decode_tc.cu), which
+// keeps those.  Whole call on that kernel / here, us: 11008 -> 4096 24
 // tokens 25.6 / 19.7, 32 tokens 27.2 / 20.2, 48 tokens 34.5 / 29.4, 64 tokens 37.3 / 36.5; 16384 -> 4096 16 tokens 28.5 / 18.8, 32 tokens
 // 31.8 / 27.4, 48 tokens 39.2 / 40.8, 64 tokens 42.0 / 50.8.
 bool gemv_mma_preq_fits(int M, int N, int K) {

@@ -366,7 +366,7 @@ EL_API int el_set_decode_gemv_max_tokens(int max_tokens);
  * the tokens itself and touches no scratch; others as the row quantiser (into xq_scratch and absmax) followed by one launch
  * per 32 tokens on the quantised tokens (longer rows a chunk of the reduction at a time), each a programmatic dependent of
  * the launch before it.  Calls with more tokens than the limit, more than 32 tokens of rows beyond 12288, and very wide
- * outputs of long rows (N beyond about 84000) take the tcgen05 stream-K kernel.  Process-wide. */
+ * outputs of long rows (N beyond 82880 on 148 SMs, 17 to 32 tokens) take the tcgen05 stream-K kernel.  Process-wide. */
 EL_API int el_set_decode_mma_max_tokens(int max_tokens);
 /* Tuning, off by default: with `enable` != 0 the single-launch GEMV of el_linear_decode is issued as a programmatic
  * dependent launch.  It may then start while earlier work of the stream still runs; until that work has completed it
