@@ -12,8 +12,6 @@
 
 namespace el {
 
-int device_sm_count(int* out);
-
 namespace {
 
 using namespace rowio;
@@ -446,35 +444,6 @@ rmsnorm_backward_stream_kernel(const T* __restrict__ g, const T* __restrict__ x,
     }
 }
 
-// dweight[k] = float(sum of the CTAs' partial sums).  A CTA covers 32 columns (one per lane); its W warps (8 or 32) each add
-// every W-th partial in order, and warp 0 adds their results in order: a fixed order of additions for a given width.
-// Few columns take 32 warps: 592 partials of 16 columns on 8 warps are a chain of dependent loads (10.9 us, 3.8 us with 32); where
-// the columns fill the SMs, 8 warps per CTA are enough and start sooner.
-__global__ void __launch_bounds__(1024)
-rmsnorm_dweight_kernel(const double* __restrict__ partial, int n_parts, float* __restrict__ dweight, int K) {
-    __shared__ double part[32][32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
-    const int k = blockIdx.x * 32 + lane;
-    double s = 0.0;
-    if (k < K) {
-#pragma unroll 8
-        for (int p = warp; p < n_parts; p += warps) s += partial[(size_t)p * K + k];
-    }
-    part[warp][lane] = s;
-    __syncthreads();
-    if (warp == 0 && k < K) {
-        double t = 0.0;
-        for (int w = 0; w < warps; ++w) t += part[w][lane];
-        dweight[k] = (float)t;
-    }
-}
-
-int dweight_threads(int columns) {
-    int sms = 148;
-    device_sm_count(&sms);
-    return (columns + 31) / 32 <= sms ? 1024 : 256;
-}
-
 int backward_grid(int M, int K) {
     int sms = 148;
     device_sm_count(&sms);
@@ -581,8 +550,7 @@ static int launch_rmsnorm_backward_t(const T* g, const T* x, const float* weight
         if (stream_threads(K, 2) <= MAX_V2) rc = launch_backward_stream<T, 2, MAX_V2>(g, x, weight, rstd, dx, partial, M, K, &grid, st);
         else if constexpr (sizeof(T) == 2) rc = launch_backward_stream<T, 4, 512>(g, x, weight, rstd, dx, partial, M, K, &grid, st);
         if (rc != EL_OK) return rc;
-        rmsnorm_dweight_kernel<<<(K + 31) / 32, dweight_threads(K), 0, st>>>(partial, grid, dweight, K);
-        return check_launch();
+        return launch_dweight(partial, grid, dweight, K, st);
     }
     const size_t smem = (size_t)K * sizeof(double);
     static DeviceOnce attr_once;
@@ -595,8 +563,7 @@ static int launch_rmsnorm_backward_t(const T* g, const T* x, const float* weight
     rmsnorm_backward_kernel<T><<<grid, RN_THREADS, smem, st>>>(g, x, weight, rstd, dx, partial, M, K);
     rc = check_launch();
     if (rc != EL_OK) return rc;
-    rmsnorm_dweight_kernel<<<(K + 31) / 32, dweight_threads(K), 0, st>>>(partial, grid, dweight, K);
-    return check_launch();
+    return launch_dweight(partial, grid, dweight, K, st);
 }
 
 int launch_rmsnorm_backward(const void* g, const void* x, int dt, const float* weight, const float* rstd, void* dx,

@@ -8,6 +8,9 @@
 #include "row_io.cuh"
 
 namespace el {
+
+int device_sm_count(int* out);
+
 namespace rowio {
 
 __device__ __forceinline__ void cp_async16(void* dst_smem, const void* src) {
@@ -227,7 +230,6 @@ __device__ __forceinline__ uint32_t max_red(const uint32_t* red) {
 // Threads of a streaming CTA for rows of K elements, VECS vectors of 8 per thread: whole warps.
 inline int stream_threads(int K, int vecs) { return ((K + 8 * vecs - 1) / (8 * vecs) + 31) & ~31; }
 
-
 }  // namespace rowio
 
 // The int8 row of a token, 8 elements.  FAST, for a row whose largest magnitude gives s = 127/absmax: adding 1.5*2^23 rounds
@@ -254,6 +256,36 @@ __device__ __forceinline__ uint2 quantise8(const typename rowio::Io<T>::Raw& raw
         for (int i = 0; i < 8; ++i) qi[i] = q8_sat(__fmul_rn(finite_or_nan(y[i]), s));
     }
     return make_uint2(pack4_s8(qi[0], qi[1], qi[2], qi[3]), pack4_s8(qi[4], qi[5], qi[6], qi[7]));
+}
+
+// dweight[k] = float(sum of the CTAs' partial sums).  A CTA covers 32 columns (one per lane); its W warps (8 or 32) each add
+// every W-th partial in order, and warp 0 adds their results in order: a fixed order of additions for a given width.
+// Few columns take 32 warps: 592 partials of 16 columns on 8 warps are a chain of dependent loads (10.9 us, 3.8 us with 32); where
+// the columns fill the SMs, 8 warps per CTA are enough and start sooner.
+static __global__ void __launch_bounds__(1024)
+dweight_kernel(const double* __restrict__ partial, int n_parts, float* __restrict__ dweight, int K) {
+    __shared__ double part[32][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    const int k = blockIdx.x * 32 + lane;
+    double s = 0.0;
+    if (k < K) {
+#pragma unroll 8
+        for (int p = warp; p < n_parts; p += warps) s += partial[(size_t)p * K + k];
+    }
+    part[warp][lane] = s;
+    __syncthreads();
+    if (warp == 0 && k < K) {
+        double t = 0.0;
+        for (int w = 0; w < warps; ++w) t += part[w][lane];
+        dweight[k] = (float)t;
+    }
+}
+
+static int launch_dweight(const double* partial, int n_parts, float* dweight, int K, cudaStream_t st) {
+    int sms = 148;
+    device_sm_count(&sms);
+    dweight_kernel<<<(K + 31) / 32, (K + 31) / 32 <= sms ? 1024 : 256, 0, st>>>(partial, n_parts, dweight, K);
+    return check_launch();
 }
 
 }  // namespace el

@@ -641,35 +641,6 @@ swiglu_backward_stream_kernel(const T* __restrict__ gy, const T* __restrict__ ga
     }
 }
 
-// dweight[k] = float(sum of the CTAs' partial sums).  A CTA covers 32 columns (one per lane); its W warps (8 or 32) each add
-// every W-th partial in order, and warp 0 adds their results in order: a fixed order of additions for a given width.
-// Few columns take 32 warps: 592 partials of 16 columns on 8 warps are a chain of dependent loads (10.9 us, 3.8 us with 32); where
-// the columns fill the SMs, 8 warps per CTA are enough and start sooner.
-__global__ void __launch_bounds__(1024)
-swiglu_dweight_kernel(const double* __restrict__ partial, int n_parts, float* __restrict__ dweight, int H) {
-    __shared__ double part[32][32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
-    const int k = blockIdx.x * 32 + lane;
-    double s = 0.0;
-    if (k < H) {
-#pragma unroll 8
-        for (int p = warp; p < n_parts; p += warps) s += partial[(size_t)p * H + k];
-    }
-    part[warp][lane] = s;
-    __syncthreads();
-    if (warp == 0 && k < H) {
-        double t = 0.0;
-        for (int w = 0; w < warps; ++w) t += part[w][lane];
-        dweight[k] = (float)t;
-    }
-}
-
-int dweight_threads(int columns) {
-    int sms = 148;
-    device_sm_count(&sms);
-    return (columns + 31) / 32 <= sms ? 1024 : 256;
-}
-
 int backward_grid(int M, int H, bool norm) {
     int sms = 148;
     device_sm_count(&sms);
@@ -976,8 +947,7 @@ static int launch_swiglu_backward_norm(const T* gy, const T* gate, const T* up, 
                                                                                partial, M, H);
     int rc = check_launch();
     if (rc != EL_OK) return rc;
-    swiglu_dweight_kernel<<<(H + 31) / 32, dweight_threads(H), 0, st>>>(partial, grid, dweight, H);
-    return check_launch();
+    return launch_dweight(partial, grid, dweight, H, st);
 }
 
 template <typename T, int THREADS>
@@ -1004,8 +974,7 @@ static int launch_backward_stream(const T* gy, const T* gate, const T* up, long 
     swiglu_backward_stream_kernel<T, 2, THREADS><<<grid, threads, smem, st>>>(gy, gate, up, ld, weight, rstd, d_gate, d_up, ld_d, partial, M, H);
     rc = check_launch();
     if (rc != EL_OK) return rc;
-    swiglu_dweight_kernel<<<(H + 31) / 32, dweight_threads(H), 0, st>>>(partial, grid, dweight, H);
-    return check_launch();
+    return launch_dweight(partial, grid, dweight, H, st);
 }
 
 template <typename T>
