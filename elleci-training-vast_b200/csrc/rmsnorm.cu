@@ -16,11 +16,12 @@ namespace {
 
 using namespace rowio;
 
-// One CTA per token.  K % 8 == 0; x rows, weight and q rows 16-byte (q: 8-byte) aligned.  ROW_CACHE: vectors of 8
-// elements a thread keeps in registers between the passes (2 for rows up to 4096 elements: fewer registers, more CTAs
-// per SM, more bytes in flight; 6 for rows up to 12288).
-template <typename T, int ROW_CACHE>
-__global__ void __launch_bounds__(RN_THREADS, ROW_CACHE == 2 ? 6 : 3)
+// One CTA per token, for rows beyond the streaming form's 16384 elements.  K % 8 == 0; x rows, weight and q rows 16-byte (q:
+// 8-byte) aligned.  A thread keeps ROW_CACHE vectors of 8 elements, the row's first 12288, in registers between the passes;
+// the rest of the row is read again by every pass.
+constexpr int ROW_CACHE = 6;
+template <typename T>
+__global__ void __launch_bounds__(RN_THREADS, 3)
 rmsnorm_quantize_rows_kernel(const T* __restrict__ x, long long ldx, const float* __restrict__ weight, int8_t* __restrict__ q,
                              float* __restrict__ row_absmax, float* __restrict__ rstd_out, int K, float norm_eps,
                              float quant_eps) {
@@ -30,8 +31,6 @@ rmsnorm_quantize_rows_kernel(const T* __restrict__ x, long long ldx, const float
     const T* xr = x + (size_t)m * ldx;
     int8_t* qr = q + (size_t)m * K;
 
-    // The row is read from memory once: up to ROW_CACHE vectors of 8 elements per thread stay in registers for the two
-    // later passes; longer rows re-read their tail.
     typename Io<T>::Raw cache[ROW_CACHE];
     const int k_tail = (threadIdx.x + ROW_CACHE * RN_THREADS) * 8;
 
@@ -471,7 +470,7 @@ template <typename T>
 static int launch_quantize_t(const T* x, long long ldx, const float* weight, float norm_eps, int8_t* q, float* row_absmax, float* rstd,
                              int M, int K, float quant_eps, cudaStream_t st) {
     if (K > 16384) {
-        rmsnorm_quantize_rows_kernel<T, 6><<<M, RN_THREADS, 0, st>>>(x, ldx, weight, q, row_absmax, rstd, K, norm_eps, quant_eps);
+        rmsnorm_quantize_rows_kernel<T><<<M, RN_THREADS, 0, st>>>(x, ldx, weight, q, row_absmax, rstd, K, norm_eps, quant_eps);
         return check_launch();
     }
     static DeviceOnce attr_once;
