@@ -127,7 +127,9 @@ template <typename T> __device__ __forceinline__ typename Io<T>::Raw raw_zero() 
 }
 
 // io(a*b) for 8 elements of the I/O type.  The product of two 16-bit values is exact in float32, so one packed multiply with
-// a single rounding gives what a float32 product rounded to the I/O type gives, in a quarter of the instructions.
+// a single rounding gives what a float32 product rounded to the I/O type gives, in a quarter of the instructions.  A bfloat16
+// product (16 significant bits) with a bit below float32's last place, 2^-149, is no exception: it is below 2^-134, half of the
+// smallest bfloat16, and both ways give a zero of its sign.
 __device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {
     const __nv_bfloat162 r = __hmul2(*reinterpret_cast<const __nv_bfloat162*>(&a), *reinterpret_cast<const __nv_bfloat162*>(&b));
     return *reinterpret_cast<const uint32_t*>(&r);
