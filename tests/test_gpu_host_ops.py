@@ -2,8 +2,10 @@
 import os
 import subprocess
 import sys
+import threading
 
 import pytest
+import torch
 
 from conftest import ROOT
 
@@ -34,3 +36,59 @@ print("alive")
 """.format(tests=os.path.join(ROOT, "tests"), root=ROOT)
     r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and r.stdout.strip() == "alive", (r.returncode, r.stdout, r.stderr)
+
+
+def test_a_call_that_the_library_refuses_raises_and_leaves_the_next_one_alone(pkg):
+    """A status other than 0 comes back as ElleciError with the call's name, from each kind of entry point."""
+    o, dev = pkg.int2_tc_ops, "cuda"
+    x, w, W = torch.randn(4, 64, device=dev), torch.ones(64, device=dev), torch.zeros(32, 16, dtype=torch.uint8, device=dev)
+    odd, wide = torch.randn(4, 60, device=dev), torch.randn(4, 60, device=dev, dtype=torch.bfloat16)
+    refused = [
+        ("el_rmsnorm_quantize_rows", lambda: o.rmsnorm_quantize_rows(wide, torch.ones(60, device=dev))),
+        ("el_rmsnorm_backward", lambda: o.rmsnorm_backward(wide, wide, torch.ones(60, device=dev), w[:4])),
+        ("el_swiglu_quantize_rows", lambda: o.swiglu_quantize_rows(wide, wide)),
+        ("el_linear_decode", lambda: o.linear_decode(odd, W[:, :15], 1.0)),
+        ("el_prelinear_decode", lambda: o.linear_decode(odd, W[:, :15], 1.0, norm_weight=torch.ones(60, device=dev))),
+        ("el_gemm_fwd_ws", lambda: o.matmul_rows(torch.zeros(4, 60, dtype=torch.int8, device=dev), W[:, :15], w[:4], 1.0, path=pkg._lib.EL_PATH_TC)),
+    ]
+    good = o.linear_decode(x, W, 1.0, norm_weight=w)
+    for name, call in refused:
+        with pytest.raises(pkg.ElleciError, match=name):
+            call()
+        assert torch.equal(o.linear_decode(x, W, 1.0, norm_weight=w), good)
+    o.check_device_status(torch.device(dev, torch.cuda.current_device()))
+
+
+# 64 x 16384: the stream-K kernel, whose partial sums meet in the cached workspace; 5 and 64 x 1024: kernels without one
+@pytest.mark.parametrize("M,K,norm", [(64, 16384, False), (64, 16384, True), (64, 1024, True), (5, 1024, False)])
+def test_decode_from_several_threads_on_their_own_streams(pkg, M, K, norm):
+    """Threads that decode at the same time, each on its own stream and weights, each from its first call on (the call that creates the
+    stream's workspace): every output is that of the call alone."""
+    o, N, threads, calls = pkg.int2_tc_ops, 2048, 4, 25
+    g = torch.Generator(device="cuda").manual_seed(M + K)
+    W = [torch.randint(0, 256, (N, K // 4), generator=g, device="cuda", dtype=torch.uint8) for _ in range(threads)]
+    x = [torch.randn(M, K, generator=g, device="cuda").to(torch.bfloat16) for _ in range(threads)]
+    w = torch.rand(K, generator=g, device="cuda") + 0.5 if norm else None
+    want = []
+    for i in range(threads):
+        q, a = o.quantize_rows(x[i]) if w is None else o.rmsnorm_quantize_rows(x[i], w)[:2]
+        want.append(o.matmul_rows(q, W[i], a, 0.01))
+    torch.cuda.synchronize()
+    wrong, errors, start = [0] * threads, [], threading.Barrier(threads)
+
+    def decode(i):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                start.wait(timeout=60)
+                outs = [o.linear_decode(x[i], W[i], 0.01, norm_weight=w) for _ in range(calls)]
+                wrong[i] = sum(int((y != want[i]).sum()) for y in outs)
+        except BaseException as e:          # reported by the main thread
+            errors.append(e)
+
+    pool = [threading.Thread(target=decode, args=(i,)) for i in range(threads)]
+    for t in pool:
+        t.start()
+    for t in pool:
+        t.join(timeout=120)
+    assert not errors and wrong == [0] * threads, (errors, wrong)
+    o.check_device_status(torch.device("cuda", torch.cuda.current_device()))

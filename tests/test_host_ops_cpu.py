@@ -122,3 +122,107 @@ def test_a_module_built_for_another_torch_is_not_loaded(pkg, monkeypatch):
     monkeypatch.setattr(pkg._lib, "_host", None)
     with pytest.raises(pkg.ElleciError, match="is missing: build it with"):
         pkg._lib.host_ops()
+
+
+def _refusals(o, t):
+    """(call, exception, message) for the checks of every native operator behind the first one; `t(shape, dtype)` makes the tensors.
+    x [4,64], two weight matrices of 32 rows, and what a caller may get wrong about each argument."""
+    f, i8, u8, b16 = torch.float32, torch.int8, torch.uint8, torch.bfloat16
+    x, row, one, w = t((4, 64), b16), t((4,), f), t((1,), f), t((64,), f)
+    xq, gq, W, H = t((4, 64), i8), t((4, 32), i8), t((32, 16), u8), t((32, 32), u8)
+    row5, w2, h64 = t((5,), f), t((64, 2), f)[:, 0], t((4, 64), torch.float16)
+    cpu = torch.zeros(1)
+    R, K, V, T = RuntimeError, KeyError, ValueError, TypeError
+    floats = "must be float16, bfloat16 or float32"
+    upd = (0.1, 5.0, 3, 0.0, 1)
+    return {
+        "quantize_rows": [
+            (lambda: o.quantize_rows(xq), R, "x " + floats),
+            (lambda: o.quantize_rows(x, "eps"), T, "real number"),
+            (lambda: o.quantize_rows(x, fold_absmax=row5), R, r"fold_absmax must be float32 \[M\]"),
+            (lambda: o.quantize_rows(x, fold_absmax=row.to(b16)), R, r"fold_absmax must be float32 \[M\]"),
+            (lambda: o.quantize_rows(x, fold_absmax=3), T, "fold_absmax must be a tensor"),
+            (lambda: o.quantize_rows(x, raw_absmax=row5), R, r"raw_absmax must be a contiguous float32 \[M\]"),
+            (lambda: o.quantize_rows(x, raw_absmax=t((4, 2), f)[:, 0]), R, r"raw_absmax must be a contiguous float32 \[M\]"),
+            (lambda: o.quantize_rows(x, out=x), R, r"out must be a contiguous int8 CUDA tensor of M\*K elements"),
+            (lambda: o.quantize_rows(x, out=gq), R, r"out must be a contiguous int8 CUDA tensor of M\*K elements"),
+            (lambda: o.quantize_rows(x, out=t((4, 128), i8)[:, ::2]), R, r"out must be a contiguous int8 CUDA tensor of M\*K elements")],
+        "quantize_grad": [
+            (lambda: o.quantize_grad(x, row5, one), R, r"x_absmax must be float32 \[M\]"),
+            (lambda: o.quantize_grad(x, row, row), R, r"g_absmax must be float32 \[1\]"),
+            (lambda: o.quantize_grad(xq, row, one), K, "torch")],
+        "quantize_tensor": [
+            (lambda: o.quantize_activation_async(x, cpu), R, "d_global_max must be a CUDA tensor"),
+            (lambda: o.quantize_activation_async(xq, one), R, "Input must be float16")],
+        "rmsnorm_quantize_rows": [
+            (lambda: o.rmsnorm_quantize_rows(x, None), R, "weight must be a CUDA tensor"),
+            (lambda: o.rmsnorm_quantize_rows(xq, w), R, "x " + floats),
+            (lambda: o.rmsnorm_quantize_rows(x, row), R, r"weight must be a contiguous float32 \[K\]"),
+            (lambda: o.rmsnorm_quantize_rows(x, w.to(b16)), R, r"weight must be a contiguous float32 \[K\]"),
+            (lambda: o.rmsnorm_quantize_rows(x, w2), R, r"weight must be a contiguous float32 \[K\]")],
+        "rmsnorm_backward": [
+            (lambda: o.rmsnorm_backward(x, h64, w, row), R, "g and x must have the same shape and dtype"),
+            (lambda: o.rmsnorm_backward(x[:2], x, w, row), R, "g and x must have the same shape and dtype"),
+            (lambda: o.rmsnorm_backward(x, x, row, row), R, r"weight must be float32 \[K\]"),
+            (lambda: o.rmsnorm_backward(x, x, w, row5), R, r"rstd must be float32 \[M\]")],
+        "swiglu_quantize_rows": [
+            (lambda: o.swiglu_quantize_rows(x, h64), R, "gate and up must have the same shape and dtype"),
+            (lambda: o.swiglu_quantize_rows(xq, xq), R, "gate and up " + floats),
+            (lambda: o.swiglu_quantize_rows(x, x, w2), R, r"norm_weight must be a contiguous float32 \[H\]")],
+        "swiglu_backward": [
+            (lambda: o.swiglu_backward(x, x, x[:2]), R, "gate and up must have the same shape and dtype"),
+            (lambda: o.swiglu_backward(h64, x, x), R, "gy must have the shape and dtype of gate"),
+            (lambda: o.swiglu_backward(x, x, x, out=x), R, r"out must be a contiguous \[M, 2H\] tensor"),
+            (lambda: o.swiglu_backward(x, x, x, row, row), R, r"norm_weight must be float32 \[H\]"),
+            (lambda: o.swiglu_backward(x, x, x, w), R, r"rstd must be float32 \[M\]"),
+            (lambda: o.swiglu_backward(x, x, x, w, row5), R, r"rstd must be float32 \[M\]")],
+        "prelinear_rows": [
+            (lambda: o.prelinear_rows(xq), R, "x " + floats),
+            (lambda: o.prelinear_rows(x, cpu), R, "up must be a CUDA tensor"),
+            (lambda: o.prelinear_rows(x, h64), R, "gate and up must have the same shape and dtype"),
+            (lambda: o.prelinear_rows(x, None, w2), R, r"norm_weight must be a contiguous float32 \[K\]")],
+        "gemm_fwd": [
+            (lambda: o.matmul_rows(x, W, row, 1.0), R, "X_int8 must be int8"),
+            (lambda: o.matmul_rows(xq, xq, row, 1.0), R, "W_packed must be uint8"),
+            (lambda: o.matmul_rows(xq, W, row.to(b16), 1.0), R, "d_scale_x must be float32"),
+            (lambda: o.matmul_rows(xq, W[0], row, 1.0), R, "W_packed must be 2-D"),
+            (lambda: o.matmul_rows(gq, W, row, 1.0), R, "Dimension mismatch: X has 32 features but W_packed has packed_K=16"),
+            (lambda: o.matmul_rows(xq, W, row5, 1.0), R, "one absmax per token expected"),
+            (lambda: o.matmul_rows(xq, W, row, 1.0, torch.int64), K, "torch"),
+            (lambda: o.matmul_rows(xq, W, row, 1.0, "bf16"), T, "torch.dtype"),
+            (lambda: o.matmul_rows(xq, W, row, None), T, "real number")],
+        "gemm_dx": [
+            (lambda: o.backward_input_rows(x, W, row, 1.0, 64), R, "dY_int8 must be int8"),
+            (lambda: o.backward_input_rows(gq, gq, row, 1.0, 64), R, "W_packed must be uint8"),
+            (lambda: o.backward_input_rows(gq, W, row.to(b16), 1.0, 64), R, "d_scale_dy must be float32"),
+            (lambda: o.backward_input_rows(gq, W[0], row, 1.0, 64), V, "W_packed must be 2-D"),
+            (lambda: o.backward_input_rows(xq, W, row, 1.0, 64), R, "dY has 64 features but W_packed has 32 rows"),
+            (lambda: o.backward_input_rows(gq, W, row, 1.0, 60), R, "K=60 does not match W_packed's packed_K=16"),
+            (lambda: o.backward_input_rows(gq, W, row5, 1.0, 64), R, "one absmax per token expected")],
+        "dw_hysteresis": [
+            (lambda: o.dw_hysteresis(x, xq, one, W, H, *upd), R, "Gq and Xq must be int8"),
+            (lambda: o.dw_hysteresis(gq[:2], xq, one, W, H, *upd), R, "Gq and Xq must have the same number of tokens"),
+            (lambda: o.dw_hysteresis(gq, xq, one, W, W, *upd), R, "W_packed / H_packed shape mismatch"),
+            (lambda: o.dw_hysteresis(gq, xq, one, t((32, 32), u8)[:, ::2], H, *upd), R, "W_packed/H_packed must be contiguous")],
+        "linear_decode": [
+            (lambda: o.linear_decode(xq, W, 1.0), R, "x " + floats),
+            (lambda: o.linear_decode(x, W[0], 1.0), R, "W_packed must be uint8"),
+            (lambda: o.linear_decode(x[:, :32], W, 1.0), R, "x has 32 features but W_packed has packed_K=16"),
+            (lambda: o.linear_decode(t((65, 64), b16), W, 1.0), R, "linear_decode takes 1..64 tokens"),
+            (lambda: o.linear_decode(t((0, 64), b16), W, 1.0), R, "linear_decode takes 1..64 tokens"),
+            (lambda: o.linear_decode(x, W, 1.0, torch.int64), K, "torch"),
+            (lambda: o.linear_decode(x, W, 1.0, up=h64), R, "gate and up must have the same shape and dtype"),
+            (lambda: o.linear_decode(x, W, 1.0, norm_weight=w2), R, r"norm_weight must be a contiguous float32 \[K\]")],
+    }
+
+
+@pytest.mark.parametrize("name", sorted(_refusals(None, lambda s, d: torch.zeros(s, dtype=d))))
+def test_arguments_with_the_wrong_type_or_shape_are_refused(pkg, name):
+    """Each check of the native operators, on fake CUDA tensors: the exception type and the message that the caller sees."""
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    with FakeTensorMode():
+        cases = _refusals(pkg.int2_tc_ops, lambda shape, dtype: torch.zeros(shape, device="cuda:0").to(dtype))[name]
+        for i, (call, error, message) in enumerate(cases):
+            with pytest.raises(error, match=message):
+                call()
+                pytest.fail(f"{name}: case {i} was accepted")
