@@ -118,7 +118,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     // that the expansion and the epilogue share with them (without both, 111 us).
     // 4096 tokens, 4096 -> 11008 / 11008 -> 4096, bf16 out, L2 flushed, events around the call: forward 157 / 173 us with two
     // commits, full cluster-scope releases and block coordinates divided out per block, 138 / 142 us now (2670 / 2600 TOP/s); dX
-    // 169 / 155 -> 142 / 138 us.  Boxes differ: 133 / 136 forward on the fastest seen, 146 / 145 on the slowest.
+    // 169 / 155 -> 142 / 138 us.  GPUs differ: 133 / 136 forward on the fastest seen, 146 / 145 on the slowest.
     auto bar_full = [&](int s) { return bars + 8u * s; };
     auto bar_empty = [&](int s) { return bars + 8u * (DA + s); };
     static_assert(DA == DB, "the A and B rings advance in lockstep");
