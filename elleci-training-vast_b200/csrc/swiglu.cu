@@ -103,7 +103,8 @@ __device__ __forceinline__ void gated8(const float g[8], const float u[8], float
 }
 
 // One CTA per token.  H % 8 == 0, rows 16-byte aligned.  `weight` null: no normalisation (y = h, rstd is not written).
-// ROW_CACHE as in the RMSNorm kernel: vectors of 8 hidden values a thread keeps in registers between the passes.
+// ROW_CACHE: vectors of 8 hidden values a thread keeps in registers between the passes (2 for float32 rows up to 4096: fewer
+// registers, more CTAs per SM; 6 for the others, whose elements beyond 12288 are formed again by every pass).
 template <typename T, int ROW_CACHE>
 __global__ void __launch_bounds__(RN_THREADS, ROW_CACHE == 2 ? 4 : (sizeof(T) == 4 ? 2 : 3))
 swiglu_quantize_rows_kernel(const T* __restrict__ gate, const T* __restrict__ up, long long ld, const float* __restrict__ weight,
@@ -906,10 +907,13 @@ static int launch_quantize_t(const T* gate, const T* up, long long ld, const flo
             return launch_quantize_stream<T, false>(gate, up, ld, weight, norm_eps, q, row_absmax, rstd, M, H, quant_eps, st);
         }
     }
-    if (sizeof(T) == 4 && H <= 4096)
-        swiglu_quantize_rows_kernel<T, 2><<<M, RN_THREADS, 0, st>>>(gate, up, ld, weight, q, row_absmax, rstd, H, norm_eps, quant_eps);
-    else
-        swiglu_quantize_rows_kernel<T, 6><<<M, RN_THREADS, 0, st>>>(gate, up, ld, weight, q, row_absmax, rstd, H, norm_eps, quant_eps);
+    if constexpr (sizeof(T) == 4) {
+        if (H <= 4096) {
+            swiglu_quantize_rows_kernel<T, 2><<<M, RN_THREADS, 0, st>>>(gate, up, ld, weight, q, row_absmax, rstd, H, norm_eps, quant_eps);
+            return check_launch();
+        }
+    }
+    swiglu_quantize_rows_kernel<T, 6><<<M, RN_THREADS, 0, st>>>(gate, up, ld, weight, q, row_absmax, rstd, H, norm_eps, quant_eps);
     return check_launch();
 }
 
