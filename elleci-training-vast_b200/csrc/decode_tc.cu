@@ -69,7 +69,7 @@ decode_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
     auto bar_tempty = [&](int a) { return bars + 8u * (2 * DP + 2 * DA + 2 + a); };
     volatile uint32_t* tmem_holder = reinterpret_cast<volatile uint32_t*>(bars_gen + 8 * (2 * DP + 2 * DA + 4));
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const long long u_lo = p.units * blockIdx.x / gridDim.x, u_hi = p.units * (blockIdx.x + 1) / gridDim.x;
 
     if (threadIdx.x == 0) {
@@ -108,7 +108,7 @@ decode_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
         for (long long u = u_lo + lane; u < u_hi; u += 32)
             tma_prefetch_2d(&tmW, (int)(u % p.k_blocks) * (BK / 4), (int)(u / p.k_blocks) * TILE_N);
         __syncwarp();
-        if (lane == 0) {
+        if (elect_one()) {
             int sp = 0;
             uint32_t php = 0;
             for (long long u = u_lo; u < u_hi; ++u) {
@@ -123,7 +123,7 @@ decode_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
         }
     } else if (warp == WARP_MMA) {
         // ================= MMA issuer =================
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc = make_idesc(0, 0, NU);
             int sp = 0, sa = 0, it = 0;
             uint32_t php = 0, pha = 0;

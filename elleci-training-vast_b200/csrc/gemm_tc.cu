@@ -111,7 +111,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     auto bar_tempty = [&](int a) { return bars + 8u * (3 * STAGES + 2 + a); };
     volatile uint32_t* tmem_holder = reinterpret_cast<volatile uint32_t*>(bars_gen + 8 * (3 * STAGES + 4));
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const int num_tiles = p.tiles_r * p.tiles_c;
 
     if (threadIdx.x == 0) {
@@ -141,7 +141,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 
     if (warp == WARP_TMA) {
         // ================= producer =================
-        if (lane == 0) {
+        if (elect_one()) {
             int s = 0;
             uint32_t ph = 0;
             for (int t = blockIdx.x; t < num_tiles && !failed; t += gridDim.x) {
@@ -171,7 +171,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         }
     } else if (warp == WARP_MMA) {
         // ================= MMA issuer =================
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc = make_idesc(MODE == MODE_DW, MODE != MODE_FWD, BN);
             int s = 0;
             uint32_t ph = 0;

@@ -126,7 +126,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     auto bar_tempty = [&](int a) { return bars + 8u * (2 * DA + 2 + a); };   // leader: both epilogues done
     volatile uint32_t* tmem_holder = reinterpret_cast<volatile uint32_t*>(bars_gen + 8 * (2 * DA + 4));
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();            // 0 = leader
     const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
     const int num_tiles = p.tiles_r * p.tiles_c;
@@ -170,7 +170,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                 const int r0 = trow * (2 * BM) + (int)rank * BM;
                 for (int kb = kb0; kb < kb0 + p.kbp; ++kb) {
                     if (!mbar_wait_cluster_warp(bar_empty(s), ph ^ 1u, p.status, 21)) { failed = true; break; }
-                    if (lane == 0) {
+                    if (elect_one()) {
                         if (rank == 0) mbar_expect_tx(bar_full(s), 2 * A_BYTES);
                         tma_load_2d_pair(smem_base + s * A_BYTES, &tmA, mapa_u32(bar_full(s), 0), kb * BK, r0);
                     }
@@ -194,7 +194,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                 for (int kb = 0; kb < p.kbp; ++kb) {          // the item's own blocks: the first one starts the sums
                     if (!mbar_wait_cluster_warp(bar_full(s), ph, p.status, 23)) { failed = true; break; }
                     tcgen05_fence_after();
-                    if (lane == 0) {
+                    if (elect_one()) {
                         const uint32_t a_addr = smem_base + s * A_BYTES, b_addr = ring_b + s * B_BYTES;
 #pragma unroll
                         for (int k = 0; k < BK / 32; ++k) {
@@ -207,7 +207,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                     __syncwarp();
                     if (++s == DA) { s = 0; ph ^= 1u; }
                 }
-                if (!failed && lane == 0) umma_commit_pair(bar_tfull(acc));
+                if (!failed && elect_one()) umma_commit_pair(bar_tfull(acc));
                 __syncwarp();
             }
         }
