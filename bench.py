@@ -917,7 +917,7 @@ def run_ours(args, wl):
         "bound": "tensor", "achieved": achieved, "peak": int8_peak, "unit": "TFLOP/s", "frac": achieved / int8_peak,
         "traffic": traffic, "traffic_source": traffic_src,
         "algorithmic_bytes_per_launch": sum(wl["M"] * K + N * K // 4 + 2 * wl["M"] * N for K, N in wl["layers"]) / len(wl["layers"]),
-        "kernel": "gemm_tc2_kernel / gemm_tc_kernel (tcgen05 kind::i8; forward, dX and dW+hysteresis launches)",
+        "kernel": "gemm_wt_kernel / gemm_dw_kernel (tcgen05 kind::i8; forward, dX and dW+hysteresis launches)",
         "launches": gemm_launches, "avg_launch_ms": gemm_ms / max(gemm_launches, 1),
         "timing": ("CUDA event pair around every launch, " + ("inside the headline region" if args.inline_kernel_events else
                    "second pass of the same K steps right after the headline region (the headline has one pair per step)")),

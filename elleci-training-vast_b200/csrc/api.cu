@@ -23,13 +23,11 @@ int launch_gemm_simple(int mode, const int8_t* A, const void* B, int R, int C, i
 bool gemm_skinny_fits(int mode, const void* A, const void* B, int R, int C, int D, const EpiParams& epi);
 int launch_gemm_skinny(int mode, const int8_t* A, const void* B, int R, int C, int D, const EpiParams& epi, cudaStream_t st);
 int gemm_tc_eligible(int mode, const void* A, const void* B, int R, int C, int D);
-int launch_gemm_tc(int mode, const int8_t* A, const void* B, int R, int C, int D, const EpiParams& epi, int32_t* status,
-                   cudaStream_t st);
-int launch_gemm_tc2(int mode, const int8_t* A, const void* B, int R, int C, int D, const EpiParams& epi, int32_t* status,
-                    cudaStream_t st, void* const* dst, int n_dst, long long ld_total, long long col_offset, int rows_per_dst,
-                    int first_dst, void* workspace, size_t workspace_bytes, bool lean);
-int gemm_tc2_k_split(int R, int C, int D);
-bool gemm_tc_narrow(int R, int C);
+int launch_gemm_dw(const int8_t* Gq, const int8_t* Xq, int R, int C, int D, const EpiParams& epi, int32_t* status, cudaStream_t st);
+int launch_gemm_wt(int mode, const int8_t* A, const void* B, int R, int C, int D, const EpiParams& epi, int32_t* status,
+                   cudaStream_t st, void* const* dst, int n_dst, long long ld_total, long long col_offset, int rows_per_dst,
+                   int first_dst, void* workspace, size_t workspace_bytes, bool lean);
+int gemm_wt_split_max(int R, int C, int D);
 int launch_reduce_scale_gather(const int* parts, int n_parts, void* const* out_all, int n_ranks, long long row_offset,
                                long long rows_total, const EpiParams& epi, int Mr, int C, cudaStream_t st);
 int launch_dw_hysteresis_tc(const int8_t* Gq, const int8_t* Xq, const float* g_absmax, uint8_t* Wp, uint8_t* Hp,
@@ -135,15 +133,6 @@ int require_sm100() {
 static inline bool float_dtype(int dt) { return dt == EL_F16 || dt == EL_BF16 || dt == EL_F32; }
 static inline bool out_dtype_ok(int dt) { return dt == EL_F16 || dt == EL_BF16 || dt == EL_F32 || dt == EL_I32; }
 
-// Tensor-core launch: forward and dX run on CTA pairs unless the single-CTA kernel is asked for; dW has one kernel.
-static int launch_tc(int mode, bool single_cta, const int8_t* A, const void* B, int R, int C, int D, const EpiParams& epi,
-                     int32_t* status, cudaStream_t st, void* ws = nullptr, size_t ws_bytes = 0, bool lean = false) {
-    // The weight-gradient GEMM has one kernel: a CTA-pair version of it (half of the Xq columns per CTA) was built and
-    // measured 8-10 % slower than the single-CTA kernel at every size, and dropped.
-    if (single_cta || mode == MODE_DW) return launch_gemm_tc(mode, A, B, R, C, D, epi, status, st);
-    return launch_gemm_tc2(mode, A, B, R, C, D, epi, status, st, nullptr, 0, 0, 0, 0, 0, ws, ws_bytes, lean);
-}
-
 static int gemm_dispatch(int mode, const int8_t* A, const void* B, int R, int C, int D, const EpiParams& epi, int flags,
                          int32_t* status, cudaStream_t st, void* ws = nullptr, size_t ws_bytes = 0) {
     const bool lean = (flags & EL_FLAG_LEAN) != 0;
@@ -152,18 +141,15 @@ static int gemm_dispatch(int mode, const int8_t* A, const void* B, int R, int C,
     if (R == 0 || C == 0) return EL_OK;
     if (flags == EL_PATH_SIMPLE) return launch_gemm_simple(mode, A, B, R, C, D, epi, st);
     const int elig = (D > 0) ? gemm_tc_eligible(mode, A, B, R, C, D) : EL_ERR_UNSUPPORTED_SHAPE;
-    if (flags == EL_PATH_TC || flags == EL_PATH_TC_SINGLE)
-        return elig != EL_OK ? elig : launch_tc(mode, flags == EL_PATH_TC_SINGLE, A, B, R, C, D, epi, status, st, ws, ws_bytes, lean);
+    auto launch_tc = [&]() {
+        if (mode == MODE_DW) return launch_gemm_dw(A, static_cast<const int8_t*>(B), R, C, D, epi, status, st);
+        return launch_gemm_wt(mode, A, B, R, C, D, epi, status, st, nullptr, 0, 0, 0, 0, 0, ws, ws_bytes, lean);
+    };
+    if (flags == EL_PATH_TC || flags == EL_PATH_TC_SINGLE) return elig != EL_OK ? elig : launch_tc();
     // auto: the tensor-core tiles are 128 rows deep; very small problems go to the CUDA-core kernel.  A few rows against a
     // large weight matrix still belong on the tensor-core kernel: the call is then the time to stream the packed weights
     // once, which the CUDA-core kernel takes twenty times longer for.
-    if (elig == EL_OK && (R >= 32 || (long long)C * D >= (1ll << 18))) {
-        // Single CTAs for up to 128 rows and for problems with few tiles (figures at gemm_tc_narrow), unless the pair kernel splits
-        // the reduction of those (the caller's workspace) or is asked for in its register-lean form.
-        const bool split = mode != MODE_DW && ws != nullptr && gemm_tc2_k_split(R, C, D) > 1;
-        const bool single = R <= 128 || (!lean && !split && gemm_tc_narrow(R, C));
-        return launch_tc(mode, single, A, B, R, C, D, epi, status, st, ws, ws_bytes, lean);
-    }
+    if (elig == EL_OK && (R >= 32 || (long long)C * D >= (1ll << 18))) return launch_tc();
     // layers of 16, 32 or 48 inputs: streaming kernels (see gemm_skinny.cu for both sides' times); a column count that no vector
     // store takes, an odd reduction or unaligned operands stay with the CUDA-core kernel
     if (elig != EL_OK && gemm_skinny_fits(mode, A, B, R, C, D, epi)) return launch_gemm_skinny(mode, A, B, R, C, D, epi, st);
@@ -337,7 +323,7 @@ int el_gemm_fwd(const int8_t* Xq, const uint8_t* W_packed, void* Y, int out_dtyp
 size_t el_gemm_workspace_bytes(int mode, int M, int N, int K) {
     if (M <= 0 || N <= 0 || K <= 0 || (mode != 0 && mode != 1)) return 0;
     const int R = M, C = (mode == 0) ? N : K, D = (mode == 0) ? K : N;
-    const int q = gemm_tc2_k_split(R, C, D);
+    const int q = gemm_wt_split_max(R, C, D);
     return q > 1 ? (size_t)q * R * C * sizeof(int) : 0;
 }
 
@@ -368,7 +354,7 @@ int el_gemm_fwd_gather(const int8_t* Xq, const uint8_t* W_packed, void* const* Y
     if (M == 0 || N == 0) return EL_OK;
     if (!Y_all || !absmax || !Xq || !W_packed) return EL_ERR_NULL_PTR;
     const EpiParams epi{nullptr, ld_total, out_dtype, absmax, absmax_stride, gamma};
-    return launch_gemm_tc2(MODE_FWD, Xq, W_packed, M, N, K, epi, dev_status, (cudaStream_t)stream, Y_all, n_ranks, ld_total,
+    return launch_gemm_wt(MODE_FWD, Xq, W_packed, M, N, K, epi, dev_status, (cudaStream_t)stream, Y_all, n_ranks, ld_total,
                            col_offset, 0, 0, nullptr, 0, false);
 }
 
@@ -385,7 +371,7 @@ int el_gemm_dx_scatter(const int8_t* dYq, const uint8_t* W_packed, void* const* 
         dst[d] = static_cast<char*>(parts_all[d]) + (size_t)rank * Mr * K * sizeof(int);     // slot `rank` of owner d
     }
     const EpiParams epi{nullptr, (long long)K, EL_I32, nullptr, 0, 1.0f};
-    return launch_gemm_tc2(MODE_DX, dYq, W_packed, M, K, N, epi, dev_status, (cudaStream_t)stream, dst, n_ranks, 0, 0, Mr, rank,
+    return launch_gemm_wt(MODE_DX, dYq, W_packed, M, K, N, epi, dev_status, (cudaStream_t)stream, dst, n_ranks, 0, 0, Mr, rank,
                            nullptr, 0, false);
 }
 

@@ -298,7 +298,7 @@ static int launch_t(const CUtensorMap& tmW, const CUtensorMap& tmX, const Params
 
 namespace tc {
 int make_map(CUtensorMap* m, const void* base, uint64_t cols, uint64_t rows, uint64_t pitch, uint32_t box_cols,
-             uint32_t box_rows, bool swizzle128);
+             uint32_t box_rows, int swizzle_bytes);
 }
 
 size_t decode_workspace_bytes(int N) {
@@ -325,8 +325,8 @@ int launch_decode_tc(const int8_t* Xq, const uint8_t* Wp, const EpiParams& epi, 
     p.status = status;
     const int nu = M <= 16 ? 16 : (M <= 32 ? 32 : 64);
     CUtensorMap tmW, tmX;
-    if ((rc = tc::make_map(&tmW, Wp, K / 4, N, K / 4, 32, dec::TILE_N, false)) != EL_OK) return rc;
-    if ((rc = tc::make_map(&tmX, Xq, K, M, K, 128, nu, true)) != EL_OK) return rc;
+    if ((rc = tc::make_map(&tmW, Wp, K / 4, N, K / 4, 32, dec::TILE_N, 0)) != EL_OK) return rc;
+    if ((rc = tc::make_map(&tmX, Xq, K, M, K, 128, nu, 128)) != EL_OK) return rc;
     switch (nu) {
         case 16: return dec::launch_t<16>(tmW, tmX, p, st);
         case 32: return dec::launch_t<32>(tmW, tmX, p, st);

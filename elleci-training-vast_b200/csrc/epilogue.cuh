@@ -14,10 +14,11 @@ struct EpiParams {
     float alpha;
 };
 
+__device__ __forceinline__ float epi_scale(const EpiParams& e, float absmax) {
+    return e.absmax == nullptr ? e.alpha : __fmul_rn(__fdiv_rn(absmax, 127.0f), e.alpha);
+}
 __device__ __forceinline__ float epi_row_scale(const EpiParams& e, int row) {
-    if (e.absmax == nullptr) return e.alpha;
-    const float a = e.absmax[(size_t)row * e.absmax_stride];
-    return __fmul_rn(__fdiv_rn(a, 127.0f), e.alpha);
+    return epi_scale(e, e.absmax == nullptr ? 0.0f : e.absmax[(size_t)row * e.absmax_stride]);
 }
 
 __device__ __forceinline__ void epi_store_one(const EpiParams& e, int row, int col, int acc, float sc) {

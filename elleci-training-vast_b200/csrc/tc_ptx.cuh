@@ -179,6 +179,11 @@ __device__ __forceinline__ void mbar_arrive_cluster_smem(uint32_t cluster_addr) 
     asm volatile("fence.release.sync_restrict::shared::cta.cluster;\n\t"
                  "mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
+// The same with nothing to release: for a thread whose own accesses were to tensor memory only, ordered by tcgen05.wait and
+// tcgen05.fence::before_thread_sync.
+__device__ __forceinline__ void mbar_arrive_cluster_relaxed(uint32_t cluster_addr) {
+    asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
 __device__ __forceinline__ bool mbar_try_cluster(uint32_t bar, uint32_t parity) {
     uint32_t ok;
     asm volatile(
