@@ -33,6 +33,7 @@ SIGNATURES = {
     "el_ternarize_pack": [_vp, _f, _vp, _i, _i, _vp],
     "el_unpack_ternary": [_vp, _vp, _i, _i, _i, _vp],
     "el_quantize_rows": [_vp, _i, _ll, _vp, _vp, _i, _i, _f, _i, _vp, _vp, _vp],
+    "el_zero": [_vp, C.c_size_t, _vp],
     "el_quantize_tensor": [_vp, _i, _vp, _vp, _ll, _vp],
     "el_dequantize_tensor": [_vp, _vp, _vp, _i, _ll, _vp],
     "el_quantize_grad": [_vp, _i, _ll, _vp, _vp, _vp, _i, _i, _vp],

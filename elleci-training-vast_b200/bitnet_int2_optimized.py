@@ -72,21 +72,22 @@ class BitLinearInt2(nn.Module):
     def forward(self, x: torch.Tensor, up: Optional[torch.Tensor] = None) -> torch.Tensor:
         """`up`: x is the output of a gate projection and the layer's input is `silu(x) * up` (the reference's SwiGLU
         block, model/model.py:107-108); the product, the norm and the quantiser then run as one kernel."""
-        fusable = (self.int2_layer.quant_mode == "per_token"
-                   and (not self.use_extra_rmsnorm or self.extra_rmsnorm.weight.dtype == torch.float32))
+        inner = self.int2_layer
+        norm = self.extra_rmsnorm if self.use_extra_rmsnorm else None
+        fusable = inner.quant_mode == "per_token" and (norm is None or norm.weight.dtype == torch.float32)
         if up is not None:
             if self.fuse_swiglu and fusable and (self.fuse_rmsnorm or not self.use_extra_rmsnorm) and int2_tc_ops.swiglu_supported(x) \
                     and up.dtype == x.dtype and up.shape == x.shape:
-                return self.int2_layer(x, pre_norm=self.extra_rmsnorm if self.use_extra_rmsnorm else None, up=up)
+                return inner(x, pre_norm=norm, up=up)
             x = torch.nn.functional.silu(x) * up
-        if self.use_extra_rmsnorm:
+        if norm is not None:
             if self.fuse_rmsnorm and fusable and int2_tc_ops.rmsnorm_supported(x):
                 # normalisation, quantisation (and their backward) as one kernel each instead of eight tensor passes
-                return self.int2_layer(x, pre_norm=self.extra_rmsnorm)
-            x = self.extra_rmsnorm(x)
-        if self.int2_layer.quant_mode == "per_tensor" and x.dtype != torch.float16:
+                return inner(x, pre_norm=norm)
+            x = norm(x)
+        if inner.quant_mode == "per_tensor" and x.dtype != torch.float16:
             x = x.half()
-        return self.int2_layer(x)
+        return inner(x)
 
     def set_lr(self, lr: float):
         if self._use_grad_hook and hasattr(self.int2_layer, "set_lr"):

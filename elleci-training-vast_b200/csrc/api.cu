@@ -212,6 +212,13 @@ int el_quantize_rows(const void* x, int x_dtype, long long ldx, int8_t* q, float
     return launch_quantize_rows(x, x_dtype, ldx, q, row_absmax, M, K, eps, mode, fold_absmax, fold_max, (cudaStream_t)stream);
 }
 
+int el_zero(void* ptr, size_t bytes, el_stream_t stream) {
+    if (bytes == 0) return EL_OK;
+    if (!ptr) return EL_ERR_NULL_PTR;
+    EL_CUDA_TRY(cudaMemsetAsync(ptr, 0, bytes, (cudaStream_t)stream));
+    return EL_OK;
+}
+
 int el_quantize_tensor(const void* x, int x_dtype, int8_t* q, float* absmax, long long size, el_stream_t stream) {
     if (size < 0 || !float_dtype(x_dtype)) return EL_ERR_INVALID_ARG;
     if (!absmax || (size > 0 && (!x || !q))) return EL_ERR_NULL_PTR;

@@ -31,6 +31,11 @@ HAS_INT2_OPS = True
 _FLOAT_IO = (torch.float16, torch.bfloat16, torch.float32)
 
 
+# nn.Module's own attribute assignment looks through parameters, buffers and submodules first (1.5 us each time); what a step
+# assigns here are plain values.
+_put = object.__setattr__
+
+
 class Int2LinearTCFunction(Function):
     """Y = Q(X) . W^T scaled by gamma; backward gives dX = Q(dY) . W scaled by gamma; gamma gets no gradient
     (core/bitnet/int2_linear_tc.py:255-305).  `layer`, when given, selects the quantisation mode, receives the
@@ -87,8 +92,8 @@ class Int2LinearTCFunction(Function):
                 Xq, ax = int2_tc_ops.quantize_rows(Xin, ACT_EPS)
                 ctx.save_for_backward(W_packed, gamma)
             if layer is not None and layer.training:
-                layer._saved_input = (Xq, ax)
-                layer._saved_input_shape = X.shape
+                _put(layer, "_saved_input", (Xq, ax))
+                _put(layer, "_saved_input_shape", X.shape)
             return int2_tc_ops.matmul_rows(Xq, W_packed, ax, gamma_val, out_dtype)
         if norm_weight is not None or up is not None:
             raise RuntimeError("the fused pre-linear RMSNorm and SwiGLU gate need quant_mode='per_token'")
@@ -98,8 +103,8 @@ class Int2LinearTCFunction(Function):
         X_int8, d_scale_x = int2_tc_ops.quantize_activation_async(X_half.contiguous(),
                                                                   Int2LinearTCFunction._get_absmax_buf(X.device))
         if layer is not None and layer.training:
-            layer._saved_input = (X_int8, d_scale_x)
-            layer._saved_input_shape = X_half.shape
+            _put(layer, "_saved_input", (X_int8, d_scale_x))
+            _put(layer, "_saved_input_shape", X_half.shape)
         return int2_tc_ops.matmul_int8(X_int8, W_packed, d_scale_x, gamma_val)
 
     @staticmethod
@@ -220,7 +225,7 @@ class Int2LinearTC(nn.Module):
             self.init_from_float(w_init)
         if self._gamma_cached is None:
             self._gamma_cached = self.gamma.detach().item()
-        out = self._decode_forward(x, pre_norm, up)
+        out = None if torch.is_grad_enabled() else self._decode_forward(x, pre_norm, up)
         if out is None:
             args = (x, self.W_packed, self.gamma, self.in_features, self._gamma_cached, self)
             if up is not None:
@@ -230,18 +235,19 @@ class Int2LinearTC(nn.Module):
                 out = Int2LinearTCFunction.apply(*args, pre_norm.weight, pre_norm.eps)
             else:
                 out = Int2LinearTCFunction.apply(*args)
-        if self.bias is not None:
-            out = out + self.bias.to(out.dtype)
+        bias = self.bias
+        if bias is not None:
+            out = out + bias.to(out.dtype)
         return out
 
     def _decode_forward(self, x: torch.Tensor, pre_norm: Optional[nn.Module], up: Optional[torch.Tensor]):
-        """Inference with a few tokens (no gradient recorded, 1..64 tokens, per-token mode): the layer input is formed by
+        """Inference with a few tokens (the caller has seen that no gradient is recorded; 1..64 tokens, per-token mode): the layer input is formed by
         one small kernel when a norm or a gate comes first, and the weight-streaming decode call does the rest - the
         path of the reference's `generate` (model/model.py:505-623), where its own kernels fall back to a scalar loop
         (kernels/int2/int2_matmul_int8_tc_v2.cu:452-473).  Same output as the training-time forward, bit for bit.
         Returns None when the call does not qualify."""
         K = self.in_features
-        if (torch.is_grad_enabled() or self.quant_mode != "per_token" or not x.is_cuda or x.dtype not in _FLOAT_IO or K % 64 != 0
+        if (self.quant_mode != "per_token" or not x.is_cuda or x.dtype not in _FLOAT_IO or K % 64 != 0
                 or x.shape[-1] != K):
             return None
         M = x.numel() // K
@@ -263,14 +269,18 @@ class Int2LinearTC(nn.Module):
 
     # ---- weight update -----------------------------------------------------------------------------------------
     def _take_dy_cache(self, dY: torch.Tensor):
-        c, self._dy_cache = self._dy_cache, None
-        if c is not None and c[0] == dY.data_ptr() and c[1] == tuple(dY.shape):
+        c = self._dy_cache
+        if c is None:
+            return None
+        _put(self, "_dy_cache", None)
+        if c[0] == dY.data_ptr() and c[1] == dY.shape:
             return c[2], c[3]
         return None
 
     def _run_pending_update(self):
-        p, self._pending_update = self._pending_update, None
+        p = self._pending_update
         if p is not None:
+            _put(self, "_pending_update", None)
             self.hysteresis_update(*p)
 
     def hysteresis_update(self, dY: torch.Tensor, lr: float):
@@ -278,32 +288,15 @@ class Int2LinearTC(nn.Module):
         (core/bitnet/int2_linear_tc.py:483-548).  The layer's own counter, pre-incremented, is the random step."""
         if self._saved_input is None:
             raise RuntimeError("No saved input. Call forward() first in training mode.")
-        self._step_py += 1
+        _put(self, "_step_py", self._step_py + 1)
         Xq, ax = self._saved_input
-        N, K = self.out_features, self.in_features
-        dY2 = dY.reshape(-1, N)
-        if dY2.dtype not in _FLOAT_IO:
-            dY2 = dY2.float()
-        if self.quant_mode == "per_tensor":
-            dY2 = dY2.half() if dY2.dtype != torch.float16 else dY2
-        dY2 = dY2.contiguous()
-        M = dY2.shape[0]
-        ax_rows = ax if ax.numel() == M else ax.expand(M).contiguous()
-        dYq, ady, gmax = int2_tc_ops.quantize_rows(dY2, GRAD_EPS, fold_absmax=ax_rows)
-        if self.quant_mode == "per_token":
-            self._dy_cache = (dY.data_ptr(), tuple(dY.shape), dYq.view(*dY.shape[:-1], N), ady)
-        Gq = int2_tc_ops.quantize_grad(dY2, ax_rows, gmax)
-        Xq2 = Xq.reshape(-1, K)
-        idx_base = self.row_offset * K
-        if int2_tc_ops.dw_hysteresis_supported(N, K):
-            int2_tc_ops.dw_hysteresis(Gq, Xq2, gmax, self.W_packed, self.H_packed, lr, self.lr_scale, self.threshold,
-                                      self.decay_rate, self._step_py, idx_base)
-        else:
-            dW = int2_tc_ops.weight_grad(Gq, Xq2, gmax)
-            int2_tc_ops.hysteresis_step_v2(dW, self.W_packed, self.H_packed, lr, self.lr_scale, self.threshold,
-                                           self.decay_rate, self._step_py, idx_base)
-        self._saved_input = None
-        self._saved_input_shape = None
+        per_token = self.quant_mode == "per_token"
+        dYq, ady = int2_tc_ops.weight_update(dY, ax, Xq, self.W_packed, self.H_packed, not per_token, lr, self.lr_scale,
+                                             self.threshold, self.decay_rate, self._step_py, self.row_offset * self.in_features)
+        if per_token:
+            _put(self, "_dy_cache", (dY.data_ptr(), dY.shape, dYq, ady))
+        _put(self, "_saved_input", None)
+        _put(self, "_saved_input_shape", None)
 
     def memory_footprint(self) -> Dict[str, Any]:
         total_weights = self.out_features * self.in_features
@@ -359,13 +352,13 @@ class Int2LinearTCWithGradHook(Int2LinearTC):
     def _grad_hook(self, grad: torch.Tensor):
         if not Int2LinearTCWithGradHook._hysteresis_enabled:
             # accumulation micro-batch: drop the saved activation, leave the weights alone
-            self._saved_input = None
-            self._saved_input_shape = None
+            _put(self, "_saved_input", None)
+            _put(self, "_saved_input_shape", None)
             return
         if self._saved_input is None:
             return
         if self.hysteresis_order == "after_dx":
-            self._pending_update = (grad, self._lr)     # runs at the end of Int2LinearTCFunction.backward
+            _put(self, "_pending_update", (grad, self._lr))     # runs at the end of Int2LinearTCFunction.backward
         else:
             self.hysteresis_update(grad, self._lr)
 

@@ -484,6 +484,15 @@ def dw_hysteresis(Gq: torch.Tensor, Xq: torch.Tensor, g_absmax: torch.Tensor, W_
          int(idx_base) & 0xFFFFFFFF, M, N, K, st.data_ptr(), _stream())
 
 
+def weight_update(dY: torch.Tensor, x_absmax: torch.Tensor, Xq: torch.Tensor, W_packed: torch.Tensor, H_packed: torch.Tensor,
+                  half: bool, lr: float, lr_scale: float, threshold: int, decay: float, step: int, idx_base: int = 0):
+    """A layer's weight update from its output gradient: quantize_rows (folded with x_absmax: [M], or [1] for one scale per
+    tensor), quantize_grad, then dw_hysteresis or, where that does not fit, weight_grad + hysteresis_step_v2.  dY is taken as
+    float16 when `half`.  Returns (dYq like dY, its row maxima [M]) for the dX GEMM."""
+    return host_ops().weight_update(dY, x_absmax, Xq, W_packed, H_packed, half, lr, lr_scale, int(threshold), decay,
+                                    int(step) & 0xFFFFFFFF, int(idx_base) & 0xFFFFFFFF)
+
+
 _decode_ws: dict = {}
 
 

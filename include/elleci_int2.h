@@ -108,6 +108,9 @@ EL_API int el_unpack_ternary(const uint8_t* W_packed, void* out, int out_dtype, 
 EL_API int el_quantize_rows(const void* x, int x_dtype, long long ldx, int8_t* q, float* row_absmax, int M, int K,
                             float eps, int mode, const float* fold_absmax, float* fold_max, el_stream_t stream);
 
+/* Queues the zeroing of `bytes` bytes (fold_max above, say) on the stream. */
+EL_API int el_zero(void* ptr, size_t bytes, el_stream_t stream);
+
 /* Per-tensor absmax int8 quantisation: absmax[0] = max finite |x| (the call zeroes it first),
  * q = clamp(roundf(x * (absmax > 1e-8 ? 127/absmax : 0)), -127, 127).  Replaces quantize_activation_async
  * (kernels/int2/int2_activation_quant.cu:313-343, binding kernels/int2/int2_tc_ops.cpp:343-371); the scratch
