@@ -35,9 +35,8 @@ int launch_dw_hysteresis_tc(const int8_t* Gq, const int8_t* Xq, const float* g_a
 
 int launch_quantize_rows_perm(const void* x, int dt, long long ldx, int8_t* q, float* a, int M, int K, float eps,
                               cudaStream_t st);
-size_t decode_workspace_bytes(int N);
-int launch_decode_tc(const int8_t* Xq, const uint8_t* Wp, const EpiParams& epi, void* workspace, int M, int N, int K,
-                     int32_t* status, cudaStream_t st);
+int launch_gemm_wt_decode(const int8_t* xq, const float* absmax, const uint8_t* Wp, const EpiParams& epi, int M, int N, int K, int32_t* status,
+                          cudaStream_t st);
 
 int launch_rmsnorm_quantize_rows(const void* x, int dt, long long ldx, const float* weight, float norm_eps, int8_t* q,
                                  float* row_absmax, float* rstd, int M, int K, float quant_eps, cudaStream_t st);
@@ -155,6 +154,27 @@ static int gemm_dispatch(int mode, const int8_t* A, const void* B, int R, int C,
     if (elig != EL_OK && gemm_skinny_fits(mode, A, B, R, C, D, epi)) return launch_gemm_skinny(mode, A, B, R, C, D, epi, st);
     return launch_gemm_simple(mode, A, B, R, C, D, epi, st);
 }
+
+// Second half of a decode call of several tokens: the kernel on tokens quantised by the launch before.  The warp-MMA kernel takes 32
+// tokens a launch and its time grows with N*K; the tcgen05 kernel's with K, hardly with the tokens or N, on top of a dearer
+// start.  Whole call, warp MMA / tcgen05, us: 64 tokens 4096 -> 11008 24.0 / 12.8, 4096 -> 4096 15.7 / 11.4, 1024 -> 1024 7.2 / 7.7; 40 tokens
+// 4096 -> 4096 12.6 / 11.4, 2048 -> 8192 12.1 / 9.4, 256 -> 16384 11.8 / 7.2, 2048 -> 2048 8.2 / 9.2, 4096 -> 1024 10.6 / 11.4; 32 tokens 4096 ->
+// 11008 13.2 / 12.5, 11008 -> 4096 20.6 / 19.0, 4096 -> 16384 16.6 / 12.9, 8192 -> 2048 12.8 / 15.4; 16 tokens 4096 -> 11008 10.4 / 12.3.
+static bool decode_tcgen05_wins(int M, int N, int K) {
+    const long long weights = (long long)N * K;
+    if (M > 48) return true;
+    if (M > 32) return weights >= 6000000 || N >= 8192;
+    return M > 16 && weights >= 32000000;
+}
+int launch_decode_preq(const int8_t* xq, const float* absmax, const uint8_t* Wp, const EpiParams& epi, int M, int N, int K, int32_t* status,
+                       cudaStream_t st) {
+    if (M <= decode_mma_max_tokens() && gemv_mma_preq_fits(M, N, K) && !decode_tcgen05_wins(M, N, K))
+        return launch_gemv_mma_preq(xq, absmax, Wp, epi, M, N, K, st);
+    return launch_gemm_wt_decode(xq, absmax, Wp, epi, M, N, K, status, st);
+}
+
+// The workspace that the decode calls ask for.  No kernel uses it any more; callers size and pass it as before.
+static size_t decode_workspace_bytes(int N) { return ((size_t)64 * (size_t)N + 4 * ((size_t)(N + 127) / 128)) * sizeof(int); }
 
 }  // namespace el
 
@@ -547,17 +567,10 @@ int el_linear_decode(const void* x, int x_dtype, const uint8_t* W_packed, void* 
         const EpiParams gepi{Y, (long long)N, out_dtype, nullptr, 0, gamma};
         return launch_gemv_mma(x, x_dtype, W_packed, gepi, M, N, K, (cudaStream_t)stream, decode_overlap());
     }
-    if (M <= decode_mma_max_tokens() && gemv_mma_preq_fits(M, N, K)) {
-        // more tokens: quantise them once, then the warp-MMA kernel on the quantised tokens, 32 at a time
-        int rc = launch_quantize_rows_perm(x, x_dtype, K, xq_scratch, absmax, M, K, 1e-5f, (cudaStream_t)stream);
-        if (rc != EL_OK) return rc;
-        const EpiParams gepi{Y, (long long)N, out_dtype, nullptr, 0, gamma};
-        return launch_gemv_mma_preq(xq_scratch, absmax, W_packed, gepi, M, N, K, (cudaStream_t)stream);
-    }
     int rc = launch_quantize_rows_perm(x, x_dtype, K, xq_scratch, absmax, M, K, 1e-5f, (cudaStream_t)stream);
     if (rc != EL_OK) return rc;
-    const EpiParams epi{Y, (long long)N, out_dtype, absmax, 1, gamma};
-    return launch_decode_tc(xq_scratch, W_packed, epi, workspace, M, N, K, dev_status, (cudaStream_t)stream);
+    const EpiParams epi{Y, (long long)N, out_dtype, nullptr, 0, gamma};
+    return launch_decode_preq(xq_scratch, absmax, W_packed, epi, M, N, K, dev_status, (cudaStream_t)stream);
 }
 
 int el_prelinear_decode(const void* x, const void* up, int x_dtype, long long ld, const float* norm_weight, float norm_eps,
@@ -572,12 +585,8 @@ int el_prelinear_decode(const void* x, const void* up, int x_dtype, long long ld
     if (rc != EL_OK) return rc;
     rc = launch_prelinear_quantize_perm(x, up, x_dtype, ld, norm_weight, norm_eps, xq_scratch, absmax, M, K, 1e-5f, (cudaStream_t)stream);
     if (rc != EL_OK) return rc;
-    if (M <= decode_mma_max_tokens() && gemv_mma_preq_fits(M, N, K)) {
-        const EpiParams gepi{Y, (long long)N, out_dtype, nullptr, 0, gamma};
-        return launch_gemv_mma_preq(xq_scratch, absmax, W_packed, gepi, M, N, K, (cudaStream_t)stream);
-    }
-    const EpiParams epi{Y, (long long)N, out_dtype, absmax, 1, gamma};
-    return launch_decode_tc(xq_scratch, W_packed, epi, workspace, M, N, K, dev_status, (cudaStream_t)stream);
+    const EpiParams epi{Y, (long long)N, out_dtype, nullptr, 0, gamma};
+    return launch_decode_preq(xq_scratch, absmax, W_packed, epi, M, N, K, dev_status, (cudaStream_t)stream);
 }
 
 }  // extern "C"

@@ -37,7 +37,7 @@
 
 namespace el {
 
-enum { MODE_FWD = 0, MODE_DX = 1, MODE_DW = 2 };
+enum { MODE_FWD = 0, MODE_DX = 1, MODE_DW = 2, MODE_FWD_PERM = 3 };      // FWD_PERM: tokens quantised in the order of decode16_deint
 
 namespace wt {
 
@@ -95,6 +95,7 @@ struct Params {
     int n_dst;                          // destinations that receive every output block (1 unless gathered over ranks)
     int rows_per_dst;                   // > 0: scatter instead - rows [d*rows_per_dst, (d+1)*rows_per_dst) go to destination d only
     int row_rotate;                     // scatter: token tiles are taken starting from this one (see tile_coords)
+    int weights_first;                  // the launch before this one does not write the weights: load them without waiting for it
     int32_t* status;
 };
 
@@ -243,7 +244,7 @@ __device__ __forceinline__ void scale_chunk(uint32_t (&v)[2][16], uint32_t scale
 template <int MODE, int OUT>
 __device__ __forceinline__ void stage_chunk(const uint32_t (&v)[2][16], uint32_t dst, int lane) {
     const int i = lane >> 2, q = lane & 3;
-    if (MODE == MODE_FWD && (OUT == EL_BF16 || OUT == EL_F16)) {
+    if (MODE != MODE_DX && (OUT == EL_BF16 || OUT == EL_F16)) {
         // matrix m = features 8 m to 8 m + 7; its row is token 8 c + lane % 8
         const uint32_t at = dst + (lane & 7) * 64 + (((lane >> 3) ^ ((lane >> 1) & 3)) << 4);
 #pragma unroll
@@ -303,7 +304,7 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmT, const __grid_constant__ 
     using G = Geo<NT, LEAN>;
     constexpr int DT = G::DT, SB = G::SB, T_BYTES = SB * G::TOK, PS_BYTES = SB * P_BYTES;       // of one stage
     constexpr int WCOLS = G::WCOLS, GCOLS = G::GCOLS;
-    constexpr bool OVERLAP = G::OVERLAP;
+    constexpr bool OVERLAP = G::OVERLAP, FWD = MODE != MODE_DX;
     constexpr int ACC1 = G::ACC1;
 
     extern __shared__ uint8_t smem_raw[];
@@ -359,6 +360,27 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmT, const __grid_constant__ 
         // ================= producer: this CTA's tokens and packed weights of every reduction block =================
         // The whole warp waits (a warp whose lanes all wait on the barrier is woken sooner than a single waiting lane);
         // lane 0 issues the copies.
+        auto load_packed = [&](int s, int kb, int f0) {
+            if (elect_one()) {
+                mbar_expect_tx(bar_pfull(s), PS_BYTES);
+                const uint32_t dst = smem_base + G::P + s * PS_BYTES;
+                if (FWD) {
+#pragma unroll
+                    for (int b = 0; b < SB; ++b) tma_load_2d(dst + b * P_BYTES, &tmP, bar_pfull(s), (kb + b) * (BK / 4), f0);
+                } else {
+                    tma_load_2d(dst, &tmP, bar_pfull(s), f0 / 4, kb * BK);            // a box of SB * 128 reduction rows
+                }
+            }
+            __syncwarp();
+        };
+        // Weights that the launch before this one does not write are on their way, a whole ring of them, before that launch has ended.
+        int ahead = 0;
+        if (p.weights_first && pair < num_items) {
+            int trow, tcol, part, kb0;
+            item_coords(pair, num_tiles, p, trow, tcol, part, kb0);
+            for (; ahead < DT && ahead < p.steps; ++ahead) load_packed(ahead, kb0 + ahead * SB, tcol * (2 * BF) + (int)rank * BF);
+        }
+        griddep_wait();
         int s = 0;
         uint32_t ph = 0;
         for (int w = pair; w < num_items && !failed; w += num_pairs) {
@@ -366,19 +388,13 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmT, const __grid_constant__ 
             item_coords(w, num_tiles, p, trow, tcol, part, kb0);
             const int t0 = trow * NT + (int)rank * (NT / 2), f0 = tcol * (2 * BF) + (int)rank * BF;
             for (int st = 0, kb = kb0; st < p.steps; ++st, kb += SB) {
-                // the packed slot is free long before the token slot (its blocks have been expanded before their MMAs run)
-                if (!mbar_wait_warp(bar_pempty(s), ph ^ 1u, p.status, 24)) { failed = true; break; }
-                if (elect_one()) {
-                    mbar_expect_tx(bar_pfull(s), PS_BYTES);
-                    const uint32_t dst = smem_base + G::P + s * PS_BYTES;
-                    if (MODE == MODE_FWD) {
-#pragma unroll
-                        for (int b = 0; b < SB; ++b) tma_load_2d(dst + b * P_BYTES, &tmP, bar_pfull(s), (kb + b) * (BK / 4), f0);
-                    } else {
-                        tma_load_2d(dst, &tmP, bar_pfull(s), f0 / 4, kb * BK);            // a box of SB * 128 reduction rows
-                    }
+                if (ahead > 0) {
+                    --ahead;
+                } else {
+                    // the packed slot is free long before the token slot (its blocks have been expanded before its MMAs run)
+                    if (!mbar_wait_warp(bar_pempty(s), ph ^ 1u, p.status, 24)) { failed = true; break; }
+                    load_packed(s, kb, f0);
                 }
-                __syncwarp();
                 if (!mbar_wait_cluster_warp(bar_empty(s), ph ^ 1u, p.status, 21)) { failed = true; break; }
                 if (elect_one()) {
                     if (rank == 0) mbar_expect_tx(bar_full(s), 2 * T_BYTES);
@@ -448,6 +464,7 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmT, const __grid_constant__ 
                 amax[i] = (p.epi.absmax != nullptr && row < p.R) ? p.epi.absmax[(size_t)row * p.epi.absmax_stride] : 0.0f;
             }
         };
+        griddep_wait();
         fetch(pair, 0);
         int it = 0;
         for (int w = pair; w < num_items && !failed; w += num_pairs, ++it) {
@@ -537,9 +554,9 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmT, const __grid_constant__ 
         const uint32_t a_base = tmem_base + ((uint32_t)(quarter * 32) << 16) + G::A_COL0;
         const uint32_t full0 = mapa_u32(bar_full(0), 0);
         // FWD: this lane's row of the packed tile; DX: this lane's row address for ldmatrix (lanes 0-15 give the first matrix)
-        const int row = MODE == MODE_FWD ? quarter * 32 + lane : lane;
+        const int row = FWD ? quarter * 32 + lane : lane;
         const int sw = (row >> 2) & 1;                          // the 32-byte swizzle exchanges the halves of a row
-        const uint32_t src0 = smem_base + G::P + row * 32 + (MODE == MODE_FWD ? 0 : (((quarter >> 1) ^ sw) << 4));
+        const uint32_t src0 = smem_base + G::P + row * 32 + (FWD ? 0 : (((quarter >> 1) ^ sw) << 4));
         uint32_t ph = 0;
         for (int g = set; g < total && !failed; ph ^= 1u) {
 #pragma unroll
@@ -552,11 +569,15 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmT, const __grid_constant__ 
                 for (int b = 0; b < SB; ++b) {
                     const uint32_t src = src0 + s * PS_BYTES + b * P_BYTES;
                     uint32_t o[32];
-                    if (MODE == MODE_FWD) {
+                    if (FWD) {
                         const uint4 lo = lds128(src + sw * 16), hi = lds128(src + (sw ^ 1) * 16);
                         const uint32_t px[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
 #pragma unroll
-                        for (int j = 0; j < 8; ++j) decode16(px[j], *reinterpret_cast<uint32_t(*)[4]>(&o[4 * j]));
+                        for (int j = 0; j < 8; ++j) {
+                            uint32_t(&d)[4] = *reinterpret_cast<uint32_t(*)[4]>(&o[4 * j]);
+                            if (MODE == MODE_FWD_PERM) decode16_deint(px[j], d);
+                            else decode16(px[j], d);
+                        }
                     } else {
 #pragma unroll
                         for (int j = 0; j < 8; j += 2) {       // two groups of 16 reduction indices; the warp's byte columns are one half of the 16
@@ -574,7 +595,7 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmT, const __grid_constant__ 
                         if (g >= DA && !mbar_wait_cluster_warp(bar_empty((s + DT - DA) % DT), G::SETS * i >= DA ? ph : (ph ^ 1u), p.status, 28)) { failed = true; break; }
                         tcgen05_fence_after();
                     }
-                    if (MODE == MODE_FWD) {
+                    if (FWD) {
                         tmem_st32(a_tmem + b * 32, o);
                     } else {
                         tmem_st16x128(a_tmem + b * 32, *reinterpret_cast<uint32_t(*)[16]>(&o[0]));
@@ -616,16 +637,20 @@ static int launch_t(const CUtensorMap& tmT, const CUtensorMap& tmP, const OutMap
     EL_CUDA_TRY(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64) return EL_ERR_DEVICE;
     cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr[1];
+    // A programmatic dependent launch: the set-up of its CTAs runs under the end of the launch before it; the warps that touch
+    // global memory wait for that launch to complete first (griddep_wait).
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.blockDim = dim3(Geo<NT>::THREADS, 1, 1);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 1;                    // the occupancy query below knows clusters only
     int dev_pairs = max_pairs[dev].load(std::memory_order_acquire);
     if (dev_pairs == 0) {       // host threads may race here: both then query and store the same number
         EL_CUDA_TRY(cudaFuncSetAttribute(gemm_wt_kernel<MODE, NT, LEAN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
@@ -656,6 +681,7 @@ static int launch_t(const CUtensorMap& tmT, const CUtensorMap& tmP, const OutMap
     const long long items = tiles * p.k_split;
     const int pairs = (int)(items < dev_pairs ? items : dev_pairs);
     cfg.gridDim = dim3((unsigned)(2 * pairs), 1, 1);
+    cfg.numAttrs = 2;
     EL_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_wt_kernel<MODE, NT, LEAN>, tmT, tmP, outs, p));
     return check_launch();
 }
@@ -800,6 +826,34 @@ int launch_gemm_wt(int mode, const int8_t* A, const void* B, int R, int C, int D
     if (rc != EL_OK || p.k_split == 1) return rc;
     void* out_one[1] = {epi.out};
     return launch_reduce_scale_gather(static_cast<const int*>(workspace), p.k_split, out_one, 1, 0, R, epi, R, C, st);
+}
+
+// Up to 64 tokens quantised by launch_quantize_rows_perm or launch_prelinear_quantize_perm, the launch right before this one.
+int launch_gemm_wt_decode(const int8_t* xq, const float* absmax, const uint8_t* Wp, const EpiParams& epi, int M, int N, int K, int32_t* status,
+                          cudaStream_t st) {
+    if (M < 1 || M > 64) return EL_ERR_UNSUPPORTED_SHAPE;
+    int rc = gemm_tc_eligible(MODE_FWD, xq, Wp, M, N, K);
+    if (rc != EL_OK) return rc;
+    rc = require_sm100();
+    if (rc != EL_OK) return rc;
+    wt::Params p{};
+    p.R = M; p.C = N; p.D = K;
+    p.epi = epi;
+    p.epi.absmax = absmax;
+    p.epi.absmax_stride = 1;
+    p.status = status;
+    p.k_split = 1;
+    p.n_dst = 1;
+    p.small_sums = K <= 32767;
+    p.weights_first = 1;
+    const int esz = (epi.out_dtype == EL_BF16 || epi.out_dtype == EL_F16) ? 2 : 4, nt = M <= 32 ? 32 : 64;
+    p.tma_store = ((reinterpret_cast<uintptr_t>(epi.out) & 15) == 0) && ((epi.ldo * esz) % 16 == 0);
+    wt::OutMaps outs{};
+    CUtensorMap tmT, tmP;
+    if (p.tma_store && (rc = tc::make_map_out(&outs.m[0], epi.out, N, M, (uint64_t)epi.ldo * esz, esz, 32)) != EL_OK) return rc;
+    if ((rc = tc::make_map(&tmT, xq, K, M, K, wt::BK, nt / 2, 128)) != EL_OK) return rc;
+    if ((rc = tc::make_map(&tmP, Wp, K / 4, N, K / 4, wt::BK / 4, wt::BF, 32)) != EL_OK) return rc;
+    return nt == 32 ? wt::launch_t<MODE_FWD_PERM, 32>(tmT, tmP, outs, p, st) : wt::launch_t<MODE_FWD_PERM, 64>(tmT, tmP, outs, p, st);
 }
 
 }  // namespace el

@@ -1,5 +1,6 @@
 // Decode GEMV on the warp-level int8 MMA: Y[m,n] = (sum_k Q(x)[m,k]*Wq[n,k]) * (absmax[m]/127) * gamma.  Up to 8 tokens that fit
-// in shared memory as one launch that quantises them itself; up to 64 tokens that arrive quantised, one launch per 32 of them.
+// in shared memory as one launch that quantises them itself; up to 48 tokens that arrive quantised, one launch per 32 of them
+// (more, and large matrices from 17 on, take gemm_wt.cu; the line and both sides' times are at its dispatch).
 //
 // The call is bound by streaming W_packed once and by the 2-bit -> int8 expansion of the weights; the products themselves
 // are few.  With more than a handful of tokens the dp4a of the CUDA-core GEMV (one per token and 4 weights) outgrow the
@@ -348,10 +349,7 @@ int launch_gemv_mma(const void* x, int x_dtype, const uint8_t* Wp, const EpiPara
 // Any number of tokens: they are taken 32 (or 16, or 8) at a time, one launch each; the weights of the later launches
 // come from L2.  Rows whose tokens do not fit in shared memory are taken in chunks of the reduction, as long as the row groups'
 // sums leave room for one round of blocks (at 17-32 tokens: 35 row groups per CTA, N up to 35*148*16 = 82880).  With more than 32
-// tokens, rows beyond 12288 (four or more chunks for every 32 tokens) are faster on the tcgen05 stream-K kernel (decode_tc.cu), which
-// keeps those.  Whole call on that kernel / here, us: 11008 -> 4096 24
-// tokens 25.6 / 19.7, 32 tokens 27.2 / 20.2, 48 tokens 34.5 / 29.4, 64 tokens 37.3 / 36.5; 16384 -> 4096 16 tokens 28.5 / 18.8, 32 tokens
-// 31.8 / 27.4, 48 tokens 39.2 / 40.8, 64 tokens 42.0 / 50.8.
+// tokens, rows beyond 12288 (four or more chunks for every 32 tokens) belong to the tcgen05 kernel.
 bool gemv_mma_preq_fits(int M, int N, int K) {
     if (M < 1 || N < 1 || K <= 0 || K % 64 != 0) return false;
     if (gemv_mma_fits(M < 32 ? M : 32, K)) return true;

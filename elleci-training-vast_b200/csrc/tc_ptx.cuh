@@ -87,6 +87,9 @@ __device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* map, int x, i
                  : "memory");
 }
 
+// Waits until the launch that this one is a programmatic dependent of has completed and its writes are visible; nothing where there is none.
+__device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 __device__ __forceinline__ void tcgen05_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tcgen05_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }

@@ -352,12 +352,11 @@ EL_API int el_dw_hysteresis_step_ptr(const int8_t* Gq, const int8_t* Xq, const f
 /* ---- small-M ("decode") layer -------------------------------------------------------------------------------- */
 
 /* Y[m,n] = out_dtype( float(sum_k Q(x)[m,k]*Wq[n,k]) * ((absmax[m]/127) * gamma) ) for 1 <= M <= 64 tokens: per-token
- * quantisation of x followed by a weight-streaming tensor-core kernel (operands swapped, stream-K over all SMs), the
+ * quantisation of x followed by a weight-streaming kernel (CUDA cores, warp MMA or tcgen05, by tokens and size), the
  * same integers and the same rounding as el_quantize_rows + el_gemm_fwd.  Needs K % 64 == 0 and 16-byte aligned x,
  * W_packed, xq_scratch and workspace.  Caller-owned scratch: xq_scratch int8 [M,K] and absmax float [M] (overwritten),
- * and `workspace` of el_decode_workspace_bytes(N) bytes, which must be all zero before its first use and is left
- * all zero by every call (partial sums of weight tiles that span several SMs meet there); calls that share a
- * workspace must not overlap on the GPU.  Replaces the scalar kernel the reference falls back to when M < 64
+ * and `workspace` of el_decode_workspace_bytes(N) bytes, which earlier versions kept partial sums in: it has to be given, and
+ * is neither read nor written.  Replaces the scalar kernel the reference falls back to when M < 64
  * (int2_matmul_int8_tc_v2_simple_kernel, kernels/int2/int2_matmul_int8_tc_v2.cu:452-473, dispatch :511-536), the
  * path of Elleci.generate (model/model.py:505-623). */
 EL_API size_t el_decode_workspace_bytes(int N);
@@ -369,7 +368,7 @@ EL_API int el_set_decode_gemv_max_tokens(int max_tokens);
  * the tokens itself and touches no scratch; others as the row quantiser (into xq_scratch and absmax) followed by one launch
  * per 32 tokens on the quantised tokens (longer rows a chunk of the reduction at a time), each a programmatic dependent of
  * the launch before it.  Calls with more tokens than the limit, more than 32 tokens of rows beyond 12288, and very wide
- * outputs of long rows (N beyond 82880 on 148 SMs, 17 to 32 tokens) take the tcgen05 stream-K kernel.  Process-wide. */
+ * outputs of long rows (N beyond 82880 on 148 SMs, 17 to 32 tokens) take the tcgen05 kernel.  Process-wide. */
 EL_API int el_set_decode_mma_max_tokens(int max_tokens);
 /* Tuning, off by default: with `enable` != 0 the single-launch GEMV of el_linear_decode is issued as a programmatic
  * dependent launch.  It may then start while earlier work of the stream still runs; until that work has completed it
@@ -392,14 +391,12 @@ EL_API int el_prelinear_decode(const void* x, const void* up, int x_dtype, long 
 /* el_linear_decode for callers that cannot give the library any device memory (no counterpart in the reference).
  * Serving processes that forbid cudaMalloc after start-up, runtimes that own the whole memory pool and hosts at
  * their memory budget cannot supply the scratch buffers of el_linear_decode; here the quantised tokens, their
- * scales and the partial-sum workspace live in one static device array inside the library (about 5.3 MB, held by
+ * scales live in one static device array inside the library (one megabyte, held by
  * every GPU that loads the library until the process exits).  The caller passes only x [M,K], W_packed and Y [M,N].
  * Limits: M <= 64, N <= 16384, K <= 16384, K % 64 == 0; larger sizes return EL_ERR_TOO_LARGE.  Same results as
  * el_linear_decode.  The call makes no cudaMalloc / cudaFree and uses no allocating library routine.
  * The first call on a device resolves the array's address (cudaGetSymbolAddress): make that first call with the
- * device current and before any stream capture.  All calls on a device share the one array, which keeps the
- * contents of the previous call; the parts that must start at zero are cleared on `stream` at the start of each
- * call.  Two calls whose GPU work overlaps (different streams, or threads) race on it: order them. */
+ * device current and before any stream capture.  All calls on a device share the one array.  Two calls whose GPU work overlaps (different streams, or threads) race on it: order them. */
 EL_API int el_linear_decode_static(const void* x, int x_dtype, const uint8_t* W_packed, void* Y, int out_dtype, float gamma,
                                    int M, int N, int K, int32_t* dev_status, el_stream_t stream);
 
