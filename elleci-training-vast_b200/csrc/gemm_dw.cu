@@ -7,12 +7,12 @@
 //   warp 1      allocates tensor memory; one lane (of the pair's leader) issues the MMAs and commits them to the ring's barriers
 //   warps 2-    epilogue: tcgen05.ld of one of two accumulators while the MMAs fill the other; twelve warps, three per quarter of
 //               the tensor-memory lanes, in the plain kernel; sixteen, four per quarter, in the fused one, which its
-//               integer instructions bind (two 32-column chunks a warp)
+//               integer instructions bind (two neighbouring 32-column chunks a warp)
 //
 // A pair's SM takes 32 KB of operands per block of 512 MMA cycles, a single CTA with a tile of 128 x 256 took 48 KB, which at 16 TB/s from
 // L2 was its bound.  Fused launch, cold L2, single CTAs / pairs, us: 4096 tokens 4096 -> 11008 137 / 130, 4096 -> 4096 67 / 61, 8192 tokens
-// 4096 -> 11008 261 / 229, 16384 tokens 4096 -> 16384 713 / 700.  What binds the fused kernel at 4096 tokens and below is the
-// update's integer instructions: 1024 tokens 4096 -> 4096 take 49 us where the plain sums of the same MMAs take 46 for their stores.
+// 4096 -> 11008 261 / 229, 16384 tokens 4096 -> 16384 713 / 700.  What binds the fused kernel below 4096 tokens is the
+// update's integer instructions (512 tokens 4096 -> 4096: 37 us for 33 us of them; common.cuh has what they took before).
 //
 // Every wait on an mbarrier is bounded: when it gives up, the kernel records a code in *status, lets its
 // outstanding copies land, frees tensor memory and returns.
@@ -204,6 +204,7 @@ gemm_dw_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         const int sub = (warp - 2) >> 2;              // 0 for warps 2-5, 1 for 6-9, 2 for 10-13, 3 for 14-17
         const int row_in_tile = quarter * 32 + lane;
         griddep_wait();
+        const float hyst_scale = EPI == EPI_HYST ? epi_row_scale(p.epi, 0) : 0.0f;      // g_absmax/127 (one scale for the tensor)
         HystParams hp;                                // with the step taken from device memory when the launch says so
         if (EPI == EPI_HYST) hp = hyst_resolve_step(p.hp);
         int it = 0;
@@ -217,15 +218,15 @@ gemm_dw_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             const bool row_ok = row < p.R;
             // Fused update: the packed weights and counters of this warp's chunks do not depend on the accumulator, so they
             // are requested before the wait for it and arrive while the tile's MMAs still run.
-            constexpr int HYST_CHUNKS = (BN / 32 + EPI_SPLIT - 1) / EPI_SPLIT;
+            constexpr int HYST_CHUNKS = EPI == EPI_HYST ? BN / 32 / EPI_SPLIT : 1;      // 2, or 1 for narrow tiles: neighbours
             uint2 w_pre[HYST_CHUNKS];
             uint4 h_pre[HYST_CHUNKS];
             if (EPI == EPI_HYST) {
 #pragma unroll
                 for (int i = 0; i < HYST_CHUNKS; ++i) {
-                    const int c = sub + i * EPI_SPLIT;
+                    const int c = sub * HYST_CHUNKS + i;
                     const int col0 = c0 + c * 32;
-                    if (c < BN / 32 && row_ok && col0 < p.C) {     // K % 32 == 0: a chunk is inside or outside as a whole
+                    if (row_ok && col0 < p.C) {     // K % 32 == 0: a chunk is inside or outside as a whole
                         w_pre[i] = *reinterpret_cast<const uint2*>(p.Wp + (size_t)row * p.pK + (col0 >> 2));
                         h_pre[i] = *reinterpret_cast<const uint4*>(p.Hp + (size_t)row * p.pH + (col0 >> 1));
                     }
@@ -246,24 +247,25 @@ gemm_dw_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 }
             } else {
                 // weight-gradient tile -> hysteresis update of 32 weights of row `row` per chunk
-                const float sc = epi_row_scale(p.epi, 0);   // g_absmax/127 (one scale for the tensor)
-#pragma unroll
+                // (not unrolled: the update is 17 KB of code, and two copies of it ran out of the instruction cache)
+#pragma unroll 1
                 for (int i = 0; i < HYST_CHUNKS; ++i) {
-                    const int c = sub + i * EPI_SPLIT;
-                    if (c >= BN / 32) break;
+                    const int c = sub * HYST_CHUNKS + i;
                     uint32_t v[32];
                     tmem_ld32(taddr + c * 32, v);
                     tmem_ld_wait();
                     const int col0 = c0 + c * 32;
                     if (row_ok && col0 < p.C) {
-                        uint32_t w[2] = {w_pre[i].x, w_pre[i].y};
-                        uint32_t h[4] = {h_pre[i].x, h_pre[i].y, h_pre[i].z, h_pre[i].w};
+                        uint32_t w[2] = {w_pre[0].x, w_pre[0].y};
+                        uint32_t h[4] = {h_pre[0].x, h_pre[0].y, h_pre[0].z, h_pre[0].w};
                         const uint32_t idx0 = p.idx_base + (uint32_t)row * (uint32_t)p.C + (uint32_t)col0;
-                        if ((p.idx_base & 31u) == 0) hyst_update_chunk32<true, true>(v, sc, w, h, idx0, hp);     // C % 32 == 0
-                        else hyst_update_chunk32<true, false>(v, sc, w, h, idx0, hp);
+                        if ((p.idx_base & 31u) == 0) hyst_update_chunk32<true, true>(v, hyst_scale, w, h, idx0, hp);     // C % 32 == 0
+                        else hyst_update_chunk32<true, false>(v, hyst_scale, w, h, idx0, hp);
                         *reinterpret_cast<uint2*>(p.Wp + (size_t)row * p.pK + (col0 >> 2)) = make_uint2(w[0], w[1]);
                         *reinterpret_cast<uint4*>(p.Hp + (size_t)row * p.pH + (col0 >> 1)) = make_uint4(h[0], h[1], h[2], h[3]);
                     }
+#pragma unroll
+                    for (int k = 0; k + 1 < HYST_CHUNKS; ++k) w_pre[k] = w_pre[k + 1], h_pre[k] = h_pre[k + 1];
                 }
             }
             tcgen05_fence_before();
