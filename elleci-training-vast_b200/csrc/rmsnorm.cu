@@ -148,13 +148,15 @@ rmsnorm_quantize_rows_kernel(const T* __restrict__ x, long long ldx, const float
 // others' work.  Products of two values of a 16-bit I/O type are taken packed (one rounding, the same result), and the
 // quantiser rounds by adding 1.5*2^23 instead of converting.  What bounds it: about 20 instructions per element and one
 // float64 conversion; memory 3 bytes per element (bf16).
-// 4096 tokens x 11008, bf16: 76 us in the one-CTA-per-row form, 47 us in this one; x 4096: 27 -> 20.5 us (events around
-// the call, L2 flushed).
+// 4096 tokens x 11008, bf16: 76 us in the one-CTA-per-row form, 47 us in this one at 64 registers a thread; x 4096: 27 -> 20.5 us (events
+// around the call, L2 flushed).  At 80 registers (in a CUDA graph): 44.2 -> 38.8 and 17.0 -> 15.8 us, 16384 x 2048 30.0 -> 27.2; 8192 x
+// 16384, where an SM then holds one CTA instead of two, 104.6 -> 110.6.  (Tried: the next row's squares before this row's maximum, so that
+// a row has one barrier: 41.0 us at 11008, the reads of the row from its slots cost more than the barrier.)
 constexpr int FW_STAGES = 2;
 template <typename T> constexpr int FW_VECS = 8 / (int)sizeof(T);        // vectors of 8 per thread: 4, float32: 2
 
-template <typename T>
-__global__ void __launch_bounds__(sizeof(T) == 2 ? 512 : 1024, sizeof(T) == 2 ? 2 : 1)
+template <typename T, int REGS>
+__global__ void __maxnreg__(REGS)
 rmsnorm_quantize_stream_kernel(const T* __restrict__ x, long long ldx, const float* __restrict__ weight, int8_t* __restrict__ q,
                                float* __restrict__ row_absmax, float* __restrict__ rstd_out, int M, int K, float norm_eps,
                                float quant_eps) {
@@ -464,6 +466,28 @@ size_t rmsnorm_backward_workspace_bytes(int K) {
     return (size_t)sms * 4 * (size_t)K * sizeof(double);
 }
 
+template <typename T, int REGS>
+static int launch_quantize_stream(const T* x, long long ldx, const float* weight, float norm_eps, int8_t* q, float* row_absmax, float* rstd,
+                                  int M, int K, float quant_eps, int threads, cudaStream_t st) {
+    static DeviceOnce attr_once;
+    int dev = 0, sms = 0;
+    EL_CUDA_TRY(cudaGetDevice(&dev));
+    const int rc = device_sm_count(&sms);
+    if (rc != EL_OK) return rc;
+    if (!attr_once.is_done(dev)) {
+        EL_CUDA_TRY(cudaFuncSetAttribute(rmsnorm_quantize_stream_kernel<T, REGS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+        attr_once.mark(dev);
+    }
+    const size_t smem = (size_t)FW_STAGES * 64 * threads;
+    int per_sm = resident_threads(REGS) / threads;
+    const int by_smem = (int)((200u * 1024u) / (smem + 1024));
+    per_sm = per_sm < by_smem ? per_sm : by_smem;
+    per_sm = per_sm < 1 ? 1 : (per_sm > 32 ? 32 : per_sm);
+    const int grid = M < sms * per_sm ? M : sms * per_sm;
+    rmsnorm_quantize_stream_kernel<T, REGS><<<grid, threads, smem, st>>>(x, ldx, weight, q, row_absmax, rstd, M, K, norm_eps, quant_eps);
+    return check_launch();
+}
+
 // Rows of up to 16384 elements stream (64 bytes of a row per thread, sixteen warps: 32 for float32); longer ones take the
 // one-CTA-per-row kernel.
 template <typename T>
@@ -473,24 +497,12 @@ static int launch_quantize_t(const T* x, long long ldx, const float* weight, flo
         rmsnorm_quantize_rows_kernel<T><<<M, RN_THREADS, 0, st>>>(x, ldx, weight, q, row_absmax, rstd, K, norm_eps, quant_eps);
         return check_launch();
     }
-    static DeviceOnce attr_once;
-    int dev = 0, sms = 0;
-    EL_CUDA_TRY(cudaGetDevice(&dev));
-    const int rc = device_sm_count(&sms);
-    if (rc != EL_OK) return rc;
-    if (!attr_once.is_done(dev)) {
-        EL_CUDA_TRY(cudaFuncSetAttribute(rmsnorm_quantize_stream_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-        attr_once.mark(dev);
-    }
     const int threads = stream_threads(K, FW_VECS<T>);
-    const size_t smem = (size_t)FW_STAGES * 64 * threads;
-    int per_sm = 1024 / threads;                     // 64 registers per thread
-    const int by_smem = (int)((200u * 1024u) / (smem + 1024));
-    per_sm = per_sm < by_smem ? per_sm : by_smem;
-    per_sm = per_sm < 1 ? 1 : (per_sm > 32 ? 32 : per_sm);
-    const int grid = M < sms * per_sm ? M : sms * per_sm;
-    rmsnorm_quantize_stream_kernel<T><<<grid, threads, smem, st>>>(x, ldx, weight, q, row_absmax, rstd, M, K, norm_eps, quant_eps);
-    return check_launch();
+    // 80 registers per thread, or 64 where an SM would hold one CTA of 80 but two of 64
+    const int wide = resident_threads(80) / threads, narrow = resident_threads(64) / threads;
+    if (wide == 0 || (wide == 1 && narrow == 2))
+        return launch_quantize_stream<T, 64>(x, ldx, weight, norm_eps, q, row_absmax, rstd, M, K, quant_eps, threads, st);
+    return launch_quantize_stream<T, 80>(x, ldx, weight, norm_eps, q, row_absmax, rstd, M, K, quant_eps, threads, st);
 }
 
 int launch_rmsnorm_quantize_rows(const void* x, int dt, long long ldx, const float* weight, float norm_eps, int8_t* q,

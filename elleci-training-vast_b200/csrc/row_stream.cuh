@@ -229,6 +229,9 @@ __device__ __forceinline__ uint32_t max_red(const uint32_t* red) {
     return __reduce_max_sync(0xffffffffu, lane < (int)(blockDim.x >> 5) ? red[lane] : 0u);
 }
 
+// Threads that an SM holds at `regs` registers each: 16384 registers in each of its four parts.
+constexpr int resident_threads(int regs) { return 512 / regs * 128; }
+
 // Threads of a streaming CTA for rows of K elements, VECS vectors of 8 per thread: whole warps.
 inline int stream_threads(int K, int vecs) { return ((K + 8 * vecs - 1) / (8 * vecs) + 31) & ~31; }
 
