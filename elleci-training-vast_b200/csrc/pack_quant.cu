@@ -225,6 +225,34 @@ __device__ __forceinline__ void raw_unpack(const Raw8<float>& r, float v[8]) {
     v[4] = __uint_as_float(r.b.x); v[5] = __uint_as_float(r.b.y); v[6] = __uint_as_float(r.b.z); v[7] = __uint_as_float(r.b.w);
 }
 
+// Running maximum of |value| on bit patterns, whose order is that of the finite values, with infinities and then NaN on top: one
+// operation for two 16-bit values (both halves of a word carry a maximum until top_bits joins them, as a float32's bits).
+template <typename T> __device__ __forceinline__ uint32_t raw_max(uint32_t m, const Raw8<T>& r) {
+    m = __vmaxu2(m, __vmaxu2(r.a.x & 0x7fff7fffu, r.a.y & 0x7fff7fffu));
+    return __vmaxu2(m, __vmaxu2(r.a.z & 0x7fff7fffu, r.a.w & 0x7fff7fffu));
+}
+template <> __device__ __forceinline__ uint32_t raw_max<float>(uint32_t m, const Raw8<float>& r) {
+    const uint32_t v[8] = {r.a.x, r.a.y, r.a.z, r.a.w, r.b.x, r.b.y, r.b.z, r.b.w};
+#pragma unroll
+    for (int i = 0; i < 8; ++i) m = max(m, v[i] & 0x7fffffffu);
+    return m;
+}
+template <typename T> __device__ __forceinline__ uint32_t top_bits(uint32_t m);
+template <> __device__ __forceinline__ uint32_t top_bits<__nv_bfloat16>(uint32_t m) { return max(m << 16, m & 0xffff0000u); }
+template <> __device__ __forceinline__ uint32_t top_bits<__half>(uint32_t m) {
+    return __float_as_uint(__half2float(__ushort_as_half((unsigned short)max(m & 0xffffu, m >> 16))));
+}
+template <> __device__ __forceinline__ uint32_t top_bits<float>(uint32_t m) { return m; }
+__device__ __forceinline__ uint32_t block_max_bits(uint32_t v, float* red) {
+    v = __reduce_max_sync(0xffffffffu, v);
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    if (l == 0) red[w] = __uint_as_float(v);
+    __syncthreads();
+    v = __reduce_max_sync(0xffffffffu, l < (int)((blockDim.x + 31) >> 5) ? __float_as_uint(red[l]) : 0u);
+    __syncthreads();
+    return v;
+}
+
 __device__ __forceinline__ int quant_half_even(float x, float s) {
     float r = rintf(__fmul_rn(x, s));
     r = fminf(127.0f, fmaxf(-128.0f, r));
@@ -234,9 +262,14 @@ __device__ __forceinline__ int quant_half_even(float x, float s) {
 // VEC: the row pitch and base allow 8-element vector loads and 8-byte stores.
 // MODE 0: absmax + quantise; 1: raw absmax only; 2: quantise with the raw absmax found in row_absmax.
 // ROW_CACHE: vectors of 8 elements a thread keeps in registers between the passes (2 for rows up to 4096 elements: fewer
-// registers, more resident CTAs; 6 for rows up to 12288; longer rows re-read their tail).
+// registers, more resident CTAs; 6 for rows up to 12288, 8 beyond for two-byte types; longer rows re-read their tail).
+// What bounds it: memory, 3 bytes per element (bf16), and at two bytes the instructions beside it.  With a cold L2 and events around the
+// call, us, before the maximum on bits, the rounding by addition, the cache of 8 and the bounds on registers / with them: bf16 4096 x 4096
+// 15.5 / 14.8, 4096 x 11008 29.6 / 27.8, 16384 x 16384 152.8 / 121.8 (6.6 TB/s), 65536 x 1536 98.3 / 84.5; float32 4096 x 4096 20.8 / 20.1,
+// 4096 x 11008 41.9 / 41.5, 16384 x 16384 229.9 / 210.0, 65536 x 1536 123.4 / 111.3.  A float32 cache of 8 takes 106 registers: 16384 x
+// 16384 got slower by 4 %, so float32 stays at 6.  A row of the cache of 2 has no tail, and without one float32 fits six CTAs on an SM.
 template <typename T, bool VEC, int MODE, int ROW_CACHE>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, sizeof(T) == 2 ? (ROW_CACHE == 2 ? 8 : 4) : (ROW_CACHE == 2 ? 6 : 3))
 quantize_rows_kernel(const T* __restrict__ x, long long ldx, int8_t* __restrict__ q, float* __restrict__ row_absmax, int K,
                      float eps, const float* __restrict__ fold_absmax, float* __restrict__ fold_max) {
     __shared__ float red[8];
@@ -252,26 +285,20 @@ quantize_rows_kernel(const T* __restrict__ x, long long ldx, int8_t* __restrict_
     } else {
         if (VEC) {
             // The row is read from memory once: up to ROW_CACHE vectors per thread stay in registers for the second pass.
-            // fmaxf drops NaN operands and keeps infinities: only a row that holds an infinity needs the checked pass
+            // Only a row that holds an infinity or a NaN needs the checked pass.
+            uint32_t top = 0u;
 #pragma unroll
             for (int c = 0; c < ROW_CACHE; ++c) {
                 const int k = (threadIdx.x + c * 256) * 8;
                 if (k < K) {
                     cache[c] = raw_load<T>(xr + k);
-                    float v[8];
-                    raw_unpack(cache[c], v);
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(v[i]));
+                    top = raw_max<T>(top, cache[c]);
                 }
             }
-            for (int k = (threadIdx.x + ROW_CACHE * 256) * 8; k < K; k += 256 * 8) {
-                float v[8];
-                load8<T>(xr + k, v);
-#pragma unroll
-                for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(v[i]));
-            }
-            amax = block_max(amax, red);
-            if (!(amax <= 3.402823466e38f)) {          // same value in every thread of the CTA
+            for (int k = (threadIdx.x + ROW_CACHE * 256) * 8; ROW_CACHE > 2 && k < K; k += 256 * 8) top = raw_max<T>(top, raw_load<T>(xr + k));
+            top = block_max_bits(top_bits<T>(top), red);
+            amax = __uint_as_float(top);
+            if (top >= 0x7f800000u) {          // same value in every thread of the CTA
                 amax = 0.0f;
                 for (int k = threadIdx.x * 8; k < K; k += blockDim.x * 8) {
                     float v[8];
@@ -301,8 +328,10 @@ quantize_rows_kernel(const T* __restrict__ x, long long ldx, int8_t* __restrict_
         }
     }
     if (VEC) {
-        // second read of the row: served by L1/L2.  q8_sat rounds, clamps and turns NaN into 0.
-        if (row_finite) {           // MODE 0 only: the cached vectors are valid
+        // Finite rows (MODE 0 only: the cached vectors are valid): |v*s| <= 127 rounds by adding 1.5*2^23, which leaves the integer in the low
+        // mantissa bits, without the conversion unit.  Others: q8_sat rounds, clamps and turns NaN into 0.
+        if (row_finite && s <= 3.402823466e38f) {
+            auto round8 = [s](float v) { return __float_as_int(__fadd_rn(__fmul_rn(v, s), 12582912.0f)); };
 #pragma unroll
             for (int c = 0; c < ROW_CACHE; ++c) {
                 const int k = (threadIdx.x + c * 256) * 8;
@@ -311,16 +340,16 @@ quantize_rows_kernel(const T* __restrict__ x, long long ldx, int8_t* __restrict_
                     raw_unpack(cache[c], v);
                     int qi[8];
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) qi[i] = q8_sat(__fmul_rn(v[i], s));
+                    for (int i = 0; i < 8; ++i) qi[i] = round8(v[i]);
                     *reinterpret_cast<uint2*>(qr + k) = make_uint2(pack4_s8(qi[0], qi[1], qi[2], qi[3]), pack4_s8(qi[4], qi[5], qi[6], qi[7]));
                 }
             }
-            for (int k = (threadIdx.x + ROW_CACHE * 256) * 8; k < K; k += 256 * 8) {
+            for (int k = (threadIdx.x + ROW_CACHE * 256) * 8; ROW_CACHE > 2 && k < K; k += 256 * 8) {
                 float v[8];
                 load8<T>(xr + k, v);
                 int qi[8];
 #pragma unroll
-                for (int i = 0; i < 8; ++i) qi[i] = q8_sat(__fmul_rn(v[i], s));
+                for (int i = 0; i < 8; ++i) qi[i] = round8(v[i]);
                 *reinterpret_cast<uint2*>(qr + k) = make_uint2(pack4_s8(qi[0], qi[1], qi[2], qi[3]), pack4_s8(qi[4], qi[5], qi[6], qi[7]));
             }
         } else {
@@ -645,7 +674,8 @@ static int launch_quantize_rows_t(const T* x, long long ldx, int8_t* q, float* a
     const bool vec = (K % 8 == 0) && (ldx % 8 == 0) && ((reinterpret_cast<uintptr_t>(x) & 15) == 0) &&
                      ((reinterpret_cast<uintptr_t>(q) & 7) == 0);
 #define EL_QR(V, MD) do { if (K <= 4096) quantize_rows_kernel<T, V, MD, 2><<<M, 256, 0, st>>>(x, ldx, q, a, K, eps, fold_absmax, fold_max); \
-                         else quantize_rows_kernel<T, V, MD, 6><<<M, 256, 0, st>>>(x, ldx, q, a, K, eps, fold_absmax, fold_max); } while (0)
+                         else if (K <= 12288 || sizeof(T) == 4) quantize_rows_kernel<T, V, MD, 6><<<M, 256, 0, st>>>(x, ldx, q, a, K, eps, fold_absmax, fold_max); \
+                         else quantize_rows_kernel<T, V, MD, sizeof(T) == 4 ? 6 : 8><<<M, 256, 0, st>>>(x, ldx, q, a, K, eps, fold_absmax, fold_max); } while (0)
     if (mode == 0) { if (vec) EL_QR(true, 0); else EL_QR(false, 0); }
     else if (mode == 1) { if (vec) EL_QR(true, 1); else EL_QR(false, 1); }
     else { if (vec) EL_QR(true, 2); else EL_QR(false, 2); }
