@@ -471,7 +471,8 @@ PyObject* dw_hysteresis(PyObject* const* a) {
 // checks that the layer made around them.  Host time of the update, separate calls -> this one: 34 -> 17 us (1024 tokens, 1536 -> 1536),
 // 68 -> 20 us where the fused kernel does not fit (2048 tokens, 16 -> 8192); of the whole step 152 -> 120 and 229 -> 154 us, in both the
 // attribute writes that went through nn.Module among it.
-// weight_update(dY, x_absmax, Xq, W_packed, H_packed, half, lr, lr_scale, threshold, decay, step, idx_base) -> (dYq like dY, its row maxima)
+// weight_update(dY, x_absmax, Xq, W_packed, H_packed, half, lr, lr_scale, threshold, decay, step, idx_base) -> (dYq, its row maxima)
+// dY is any shape of M*N elements when `half`; else its last dimension has to be N, as the dX GEMM takes dYq in dY's shape.
 PyObject* weight_update(PyObject* const* a) {
     const Tensor& dY = cuda_arg(a[0], "dY");
     const Tensor &ax = tensor_arg(a[1], "x_absmax"), &Xq = cuda_arg(a[2], "Xq");
@@ -490,6 +491,16 @@ PyObject* weight_update(PyObject* const* a) {
     if (half && d.scalar_type() != at::kHalf) d = d.to(at::kHalf);
     d = d.contiguous();
     const int64_t M = d.size(0);
+    // dYq has dY's leading dimensions where these count the M rows, and [M, N] where not
+    auto q_sizes = dY.sizes().vec();
+    if (q_sizes.empty()) q_sizes.push_back(N);
+    q_sizes.back() = N;
+    int64_t q_rows = 1;
+    for (size_t i = 0; i + 1 < q_sizes.size(); ++i) q_rows *= q_sizes[i];
+    if (q_rows != M) {
+        EL_REQUIRE(half, "dY's last dimension must be the number of rows of W_packed");
+        q_sizes = {M, N};
+    }
     Tensor X2 = Xq.contiguous();
     EL_REQUIRE((K ? X2.numel() / K : 0) == M, "Gq and Xq must have the same number of tokens");
     EL_REQUIRE(W.size(1) == (K + 3) / 4 && H.dim() == 2 && H.size(0) == N && H.size(1) == (K + 1) / 2, "W_packed / H_packed shape mismatch");
@@ -505,7 +516,7 @@ PyObject* weight_update(PyObject* const* a) {
     uint8_t *wp = ptr<uint8_t>(W), *hp = ptr<uint8_t>(H);
     // dYq and its maxima go back to the caller (the dX GEMM reads them); the folded gradient, its maximum and, unfused, the weight
     // gradient are this call's own, in one block, each on a 256-byte boundary
-    Tensor dYq = like_rows(dY, N, at::kChar), ady = new_empty(d, {M}, at::kFloat);
+    Tensor dYq = new_empty(d, q_sizes, at::kChar), ady = new_empty(d, {M}, at::kFloat);
     const int64_t g_bytes = (M * N + 255) & ~(int64_t)255;
     Tensor own = new_empty(d, {256 + g_bytes + (fused ? 0 : N * K * 4)}, at::kByte);
     float* gmax = ptr<float>(own);

@@ -58,3 +58,40 @@ def test_refusals(ops):
                       ((dY, ax, Xq, W.char(), H), "must be uint8"), ((dY, ax, Xq, W.cpu(), H), "must be uint8")]:
         with pytest.raises(RuntimeError, match=msg):
             ops.weight_update(*args, *upd)
+
+
+@pytest.mark.parametrize("shape", ["flat", "rows joined", "rows cut in two"])
+@pytest.mark.parametrize("N,K", [(96, 64), (40, 48)])
+def test_gradient_of_another_shape(ops, pkg, shape, N, K):
+    """M*N gradient elements whose last dimension is not N: one scale per tensor takes them as [M, N], one per token refuses them before
+    anything changes."""
+    B, T = 3, 10
+    M = B * T
+    g = torch.Generator(device=DEV).manual_seed(N)
+    rows = torch.randn(M, N, generator=g, device=DEV).mul_(1e-3).half()
+    dY = {"flat": rows.flatten(), "rows joined": rows.view(B, T * N), "rows cut in two": rows.view(2 * M, N // 2)}[shape]
+    Xq = torch.randint(-127, 128, (M, K), generator=g, device=DEV, dtype=torch.int8)
+    ax = torch.rand(1, generator=g, device=DEV) + 0.5
+    W = torch.randint(0, 256, (N, (K + 3) // 4), generator=g, device=DEV, dtype=torch.uint8)
+    H = torch.randint(0, 256, (N, (K + 1) // 2), generator=g, device=DEV, dtype=torch.uint8)
+    W1, H1, W2, H2 = W.clone(), H.clone(), W.clone(), H.clone()
+    q1, a1 = ops.weight_update(rows, ax, Xq, W1, H1, True, 0.5, 5.0, 3, 0.01, 7)
+    q2, a2 = ops.weight_update(dY, ax, Xq, W2, H2, True, 0.5, 5.0, 3, 0.01, 7)
+    assert q2.shape == (M, N) and torch.equal(q1, q2) and torch.equal(a1, a2)
+    assert not torch.equal(W1, W) and torch.equal(W1, W2) and torch.equal(H1, H2)
+    W0, H0 = W.clone(), H.clone()
+    with pytest.raises(RuntimeError, match="last dimension"):
+        ops.weight_update(dY, ax.expand(M).contiguous(), Xq, W, H, False, 0.5, 5.0, 3, 0.01, 7)
+    assert torch.equal(W, W0) and torch.equal(H, H0)
+    for mode in ("per_token", "per_tensor"):                 # the same through a layer
+        layer = pkg.Int2LinearTC(K, N, threshold=3, quant_mode=mode).to(DEV)
+        layer.init_from_float(torch.randn(N, K, generator=g, device=DEV))
+        before, counters = layer.W_packed.clone(), layer.H_packed.clone()
+        layer(torch.randn(B, T, K, generator=g, device=DEV).half())
+        if mode == "per_tensor":
+            layer.hysteresis_update(dY, 0.5)
+            assert not torch.equal(layer.H_packed, counters)
+        else:
+            with pytest.raises(RuntimeError, match="last dimension"):
+                layer.hysteresis_update(dY, 0.5)
+            assert torch.equal(layer.W_packed, before) and torch.equal(layer.H_packed, counters)
