@@ -471,7 +471,8 @@ PyObject* dw_hysteresis(PyObject* const* a) {
 // checks that the layer made around them.  Host time of the update, separate calls -> this one: 34 -> 17 us (1024 tokens, 1536 -> 1536),
 // 68 -> 20 us where the fused kernel does not fit (2048 tokens, 16 -> 8192); of the whole step 152 -> 120 and 229 -> 154 us, in both the
 // attribute writes that went through nn.Module among it.
-// weight_update(dY, x_absmax, Xq, W_packed, H_packed, half, lr, lr_scale, threshold, decay, step, idx_base) -> (dYq, its row maxima)
+// weight_update(dY, x_absmax, Xq, W_packed, H_packed, half, lr, lr_scale, threshold, decay, step, idx_base, g_absmax) -> (dYq, its row
+// maxima), or None where the caller has the folded maximum already (g_absmax): quantise_rows is then left out.
 // dY is any shape of M*N elements when `half`; else its last dimension has to be N, as the dX GEMM takes dYq in dY's shape.
 PyObject* weight_update(PyObject* const* a) {
     const Tensor& dY = cuda_arg(a[0], "dY");
@@ -514,18 +515,27 @@ PyObject* weight_update(PyObject* const* a) {
     const int8_t* xp = ptr<int8_t>(X2);
     const float* ap = ptr<float>(rows);
     uint8_t *wp = ptr<uint8_t>(W), *hp = ptr<uint8_t>(H);
+    Tensor dYq, ady, folded;
+    if (!is_none(a[12])) {
+        folded = cuda_arg(a[12], "g_absmax");
+        EL_REQUIRE(folded.scalar_type() == at::kFloat && folded.numel() == 1, "g_absmax must be float32 [1]");
+    } else {
+        dYq = new_empty(d, q_sizes, at::kChar);
+        ady = new_empty(d, {M}, at::kFloat);
+    }
     // dYq and its maxima go back to the caller (the dX GEMM reads them); the folded gradient, its maximum and, unfused, the weight
     // gradient are this call's own, in one block, each on a 256-byte boundary
-    Tensor dYq = new_empty(d, q_sizes, at::kChar), ady = new_empty(d, {M}, at::kFloat);
     const int64_t g_bytes = (M * N + 255) & ~(int64_t)255;
     Tensor own = new_empty(d, {256 + g_bytes + (fused ? 0 : N * K * 4)}, at::kByte);
-    float* gmax = ptr<float>(own);
+    float* gmax = folded.defined() ? ptr<float>(folded) : ptr<float>(own);
     int8_t* gq = ptr<int8_t>(own) + 256;
     float* dw = reinterpret_cast<float*>(gq + g_bytes);
     int32_t* word = status_word(d);
     void* st = stream();
-    call("el_zero", g_lib.el_zero, gmax, sizeof(float), st);
-    call("el_quantize_rows", g_lib.el_quantize_rows, dp, dt, N, ptr<int8_t>(dYq), ptr<float>(ady), M, N, 1e-30f, EL_QUANT_FULL, ap, gmax, st);
+    if (!folded.defined()) {
+        call("el_zero", g_lib.el_zero, gmax, sizeof(float), st);
+        call("el_quantize_rows", g_lib.el_quantize_rows, dp, dt, N, ptr<int8_t>(dYq), ptr<float>(ady), M, N, 1e-30f, EL_QUANT_FULL, ap, gmax, st);
+    }
     call("el_quantize_grad", g_lib.el_quantize_grad, dp, dt, N, ap, gmax, gq, M, N, st);
     if (fused) {
         call("el_dw_hysteresis", g_lib.el_dw_hysteresis, gq, xp, gmax, wp, hp, lr, lr_scale, threshold, decay, step, idx_base, M, N, K, word, st);
@@ -534,6 +544,7 @@ PyObject* weight_update(PyObject* const* a) {
         call("el_hysteresis_from_dw", g_lib.el_hysteresis_from_dw, dw, wp, hp, lr, lr_scale, threshold, decay, step, N, K, idx_base, 1, st);
     }
     maybe_check(d);
+    if (folded.defined()) return none();
     return tuple_of(wrap(dYq), wrap(ady));
 }
 
@@ -647,7 +658,7 @@ PyObject* set_hooks(PyObject* const* a) {
 PyMethodDef methods[] = {
     EL_ENTRY(quantize_rows, 5), EL_ENTRY(quantize_grad, 3), EL_ENTRY(quantize_tensor, 2), EL_ENTRY(rmsnorm_quantize_rows, 4),
     EL_ENTRY(rmsnorm_backward, 4), EL_ENTRY(swiglu_quantize_rows, 5), EL_ENTRY(swiglu_backward, 6), EL_ENTRY(prelinear_rows, 4),
-    EL_ENTRY(gemm_fwd, 7), EL_ENTRY(gemm_dx, 8), EL_ENTRY(dw_hysteresis, 11), EL_ENTRY(weight_update, 12), EL_ENTRY(linear_decode, 8), EL_ENTRY(set_hooks, 5),
+    EL_ENTRY(gemm_fwd, 7), EL_ENTRY(gemm_dx, 8), EL_ENTRY(dw_hysteresis, 11), EL_ENTRY(weight_update, 13), EL_ENTRY(linear_decode, 8), EL_ENTRY(set_hooks, 5),
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "elleci_host_ops", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 

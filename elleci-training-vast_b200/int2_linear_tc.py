@@ -36,6 +36,17 @@ _FLOAT_IO = (torch.float16, torch.bfloat16, torch.float32)
 _put = object.__setattr__
 
 
+def _stamp(t: torch.Tensor):
+    """A tensor and the version of its content, to be compared later with `_same`.  The pair keeps the tensor alive, so nothing else can
+    come to lie at its address in between."""
+    return t, -1 if t.is_inference() else t._version
+
+
+def _same(stamp, t: torch.Tensor) -> bool:
+    """t is the stamped tensor, unwritten since (inference tensors, whose writes are not counted, never are)."""
+    return stamp is not None and stamp[0] is t and stamp[1] >= 0 and stamp[1] == t._version
+
+
 class Int2LinearTCFunction(Function):
     """Y = Q(X) . W^T scaled by gamma; backward gives dX = Q(dY) . W scaled by gamma; gamma gets no gradient
     (core/bitnet/int2_linear_tc.py:255-305).  `layer`, when given, selects the quantisation mode, receives the
@@ -92,6 +103,7 @@ class Int2LinearTCFunction(Function):
                 Xq, ax = int2_tc_ops.quantize_rows(Xin, ACT_EPS)
                 ctx.save_for_backward(W_packed, gamma)
             if layer is not None and layer.training:
+                _put(layer, "_dy_handed", None)
                 _put(layer, "_saved_input", (Xq, ax))
                 _put(layer, "_saved_input_shape", X.shape)
             return int2_tc_ops.matmul_rows(Xq, W_packed, ax, gamma_val, out_dtype)
@@ -109,21 +121,27 @@ class Int2LinearTCFunction(Function):
 
     @staticmethod
     def backward(ctx, dY: torch.Tensor) -> Tuple[Optional[torch.Tensor], ...]:
+        layer = ctx.layer
+        # what the output's hook has quantised for this pass; before the saved tensors are read, which under activation
+        # checkpointing runs the forward pass again
+        handed = layer._take_dy_handed(dY) if layer is not None else None
         saved = ctx.saved_tensors        # read once: under activation checkpointing a second read is an error
         W_packed, gamma = saved[:2]
-        layer = ctx.layer
         dX = None
         d_norm_weight = None
         d_up = None
         if ctx.needs_input_grad[0] or (ctx.has_norm and ctx.needs_input_grad[6]) or (ctx.has_gate and ctx.needs_input_grad[8]):
             gamma_val = ctx.gamma_cached if ctx.gamma_cached is not None else gamma.item()
             if ctx.mode == "per_token":
-                cached = layer._take_dy_cache(dY) if layer is not None else None
-                if cached is None:
+                fold = layer._pending_fold(dY) if layer is not None and handed is None else None
+                if handed is not None:
+                    dYq, ady = handed
+                elif fold is not None:
+                    dYq, ady, gmax = int2_tc_ops.quantize_rows(dY, GRAD_EPS, fold_absmax=fold)
+                    _put(layer, "_folded", (_stamp(dY), fold, gmax))
+                else:
                     dYc = dY if dY.dtype in _FLOAT_IO else dY.to(ctx.io_dtype)
                     dYq, ady = int2_tc_ops.quantize_rows(dYc, GRAD_EPS)
-                else:
-                    dYq, ady = cached
                 dX = int2_tc_ops.backward_input_rows(dYq, W_packed, ady, gamma_val, ctx.K, ctx.io_dtype)
             else:
                 dY_half = dY.half() if dY.dtype != torch.float16 else dY
@@ -145,6 +163,13 @@ class Int2LinearTCFunction(Function):
 class Int2LinearTC(nn.Module):
     """Linear layer over 2-bit packed ternary weights with int4 hysteresis counters
     (core/bitnet/int2_linear_tc.py:308-649): 0.25 + 0.5 bytes per weight."""
+
+    # What the hook of the output's gradient, the update and the backward pass of one step hand to one another; each is taken, or
+    # dropped, within that step.  (Class defaults, so that a layer pickled without them has them.)
+    _hooked = None              # the gradient whose hook is running
+    _dy_handed = None           # reference order: (stamp of dY, dYq, its row maxima), from the update to the dX that follows it
+    _pending_update = None      # after_dx: (dY, lr), from the hook to the end of backward
+    _folded = None              # after_dx: (stamp of dY, x_absmax, folded maximum), from dX to the update that follows it
 
     def __init__(self, in_features: int, out_features: int, bias: bool = False, threshold: int = 7,
                  lr_scale: float = 5.0, decay_rate: float = 0.001, compress_activations: bool = True,
@@ -183,8 +208,6 @@ class Int2LinearTC(nn.Module):
         self._saved_input_shape = None
         self._initialized = False
         self._gamma_cached: Optional[float] = None
-        self._dy_cache = None
-        self._pending_update = None
         # row offset of this layer's rows inside a larger (sharded) weight matrix: keeps the per-weight random
         # numbers of a shard equal to those of the unsharded layer
         self.row_offset = 0
@@ -268,14 +291,21 @@ class Int2LinearTC(nn.Module):
         return int2_tc_ops.linear_decode(y, self.W_packed, self._gamma_cached, x.dtype)
 
     # ---- weight update -----------------------------------------------------------------------------------------
-    def _take_dy_cache(self, dY: torch.Tensor):
-        c = self._dy_cache
+    def _take_dy_handed(self, dY: torch.Tensor):
+        c = self._dy_handed
         if c is None:
             return None
-        _put(self, "_dy_cache", None)
-        if c[0] == dY.data_ptr() and c[1] == dY.shape:
-            return c[2], c[3]
-        return None
+        _put(self, "_dy_handed", None)
+        return c[1:] if _same(c[0], dY) else None
+
+    def _pending_fold(self, dY: torch.Tensor):
+        """The row maxima of the saved input, if the update that waits for the end of this backward pass is of this very gradient: the
+        pass that quantises dY for dX then finds the update's folded maximum too."""
+        p = self._pending_update
+        if p is None or p[0] is not dY or self._saved_input is None or dY.dtype not in _FLOAT_IO:
+            return None
+        ax = self._saved_input[1]
+        return ax if ax.numel() * self.out_features == dY.numel() else None
 
     def _run_pending_update(self):
         p = self._pending_update
@@ -291,10 +321,14 @@ class Int2LinearTC(nn.Module):
         _put(self, "_step_py", self._step_py + 1)
         Xq, ax = self._saved_input
         per_token = self.quant_mode == "per_token"
-        dYq, ady = int2_tc_ops.weight_update(dY, ax, Xq, self.W_packed, self.H_packed, not per_token, lr, self.lr_scale,
-                                             self.threshold, self.decay_rate, self._step_py, self.row_offset * self.in_features)
-        if per_token:
-            _put(self, "_dy_cache", (dY.data_ptr(), dY.shape, dYq, ady))
+        f = self._folded
+        if f is not None:
+            _put(self, "_folded", None)
+            f = f[2] if f[1] is ax and _same(f[0], dY) else None
+        quantised = int2_tc_ops.weight_update(dY, ax, Xq, self.W_packed, self.H_packed, not per_token, lr, self.lr_scale, self.threshold,
+                                              self.decay_rate, self._step_py, self.row_offset * self.in_features, f)
+        if per_token and self._hooked is dY:        # dX of this gradient comes next
+            _put(self, "_dy_handed", (_stamp(dY), *quantised))
         _put(self, "_saved_input", None)
         _put(self, "_saved_input_shape", None)
 
@@ -350,6 +384,10 @@ class Int2LinearTCWithGradHook(Int2LinearTC):
         return out
 
     def _grad_hook(self, grad: torch.Tensor):
+        # what an earlier pass that formed no dX has left
+        _put(self, "_dy_handed", None)
+        _put(self, "_folded", None)
+        _put(self, "_pending_update", None)
         if not Int2LinearTCWithGradHook._hysteresis_enabled:
             # accumulation micro-batch: drop the saved activation, leave the weights alone
             _put(self, "_saved_input", None)
@@ -360,7 +398,11 @@ class Int2LinearTCWithGradHook(Int2LinearTC):
         if self.hysteresis_order == "after_dx":
             _put(self, "_pending_update", (grad, self._lr))     # runs at the end of Int2LinearTCFunction.backward
         else:
-            self.hysteresis_update(grad, self._lr)
+            _put(self, "_hooked", grad)
+            try:
+                self.hysteresis_update(grad, self._lr)
+            finally:
+                _put(self, "_hooked", None)
 
 
 # Names under which the reference instantiates the layer (core/bitnet/int2_linear_tc_offload.py:31,289).

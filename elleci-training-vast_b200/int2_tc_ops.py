@@ -485,12 +485,14 @@ def dw_hysteresis(Gq: torch.Tensor, Xq: torch.Tensor, g_absmax: torch.Tensor, W_
 
 
 def weight_update(dY: torch.Tensor, x_absmax: torch.Tensor, Xq: torch.Tensor, W_packed: torch.Tensor, H_packed: torch.Tensor,
-                  half: bool, lr: float, lr_scale: float, threshold: int, decay: float, step: int, idx_base: int = 0):
+                  half: bool, lr: float, lr_scale: float, threshold: int, decay: float, step: int, idx_base: int = 0,
+                  g_absmax: Optional[torch.Tensor] = None):
     """A layer's weight update from its output gradient: quantize_rows (folded with x_absmax: [M], or [1] for one scale per
     tensor), quantize_grad, then dw_hysteresis or, where that does not fit, weight_grad + hysteresis_step_v2.  dY is taken as
-    float16 when `half`.  Returns (dYq like dY, its row maxima [M]) for the dX GEMM."""
+    float16 when `half`.  Returns (dYq like dY, its row maxima [M]) for the dX GEMM.  `g_absmax` [1]: the folded maximum that
+    quantize_rows has given for the same dY and x_absmax; the update then starts with quantize_grad and returns None."""
     return host_ops().weight_update(dY, x_absmax, Xq, W_packed, H_packed, half, lr, lr_scale, int(threshold), decay,
-                                    int(step) & 0xFFFFFFFF, int(idx_base) & 0xFFFFFFFF)
+                                    int(step) & 0xFFFFFFFF, int(idx_base) & 0xFFFFFFFF, g_absmax)
 
 
 _decode_ws: dict = {}
