@@ -156,15 +156,22 @@ static int gemm_dispatch(int mode, const int8_t* A, const void* B, int R, int C,
 }
 
 // Second half of a decode call of several tokens: the kernel on tokens quantised by the launch before.  The warp-MMA kernel takes 32
-// tokens a launch and its time grows with N*K; the tcgen05 kernel's with K, hardly with the tokens or N, on top of a dearer
-// start.  Whole call, warp MMA / tcgen05, us: 64 tokens 4096 -> 11008 24.0 / 12.8, 4096 -> 4096 15.7 / 11.4, 1024 -> 1024 7.2 / 7.7; 40 tokens
-// 4096 -> 4096 12.6 / 11.4, 2048 -> 8192 12.1 / 9.4, 256 -> 16384 11.8 / 7.2, 2048 -> 2048 8.2 / 9.2, 4096 -> 1024 10.6 / 11.4; 32 tokens 4096 ->
-// 11008 13.2 / 12.5, 11008 -> 4096 20.6 / 19.0, 4096 -> 16384 16.6 / 12.9, 8192 -> 2048 12.8 / 15.4; 16 tokens 4096 -> 11008 10.4 / 12.3.
+// tokens a launch; its time grows with K and, in rounds of 16 output features per SM, with N.  The tcgen05 kernel's grows with K
+// alone (7.5 us + 1.05 us per 1000 of it), hardly with tokens or N.  Whole call in a CUDA graph over 192 MB of weight matrices, warp MMA /
+// tcgen05, us:
+//   64 tokens   1024 -> 1024 7.5 / 8.5, 2048 -> 2048 9.6 / 10.1, 2048 -> 4096 11.2 / 10.2, 4096 -> 256 12.7 / 11.6, 4096 -> 11008 24.1 / 12.8
+//   56 tokens   1024 -> 2048 7.4 / 8.9, 1024 -> 2560 8.4 / 9.0, 1536 -> 256 8.8 / 8.2 (the line is off by a few per cent at such sizes)
+//   40 tokens   2048 -> 4096 9.7 / 10.1, 4096 -> 2048 10.8 / 12.2, 4096 -> 4096 12.9 / 12.4, 8192 -> 256 16.7 / 16.3, 1024 -> 8192 10.2 / 9.2
+//   48 tokens   8192 -> 1024 18.5 / 16.3
+//   32 tokens   4096 -> 4096 9.7 / 11.8, 4096 -> 11008 13.9 / 12.4, 11008 -> 4096 20.6 / 19.0, 2048 -> 16384 11.5 / 10.6, 256 -> 32000 12.9 / 8.9
+//   24 tokens   16384 -> 2048 22.6 / 24.3, one round of features, however large the matrix
 static bool decode_tcgen05_wins(int M, int N, int K) {
     const long long weights = (long long)N * K;
-    if (M > 48) return true;
-    if (M > 32) return weights >= 6000000 || N >= 8192;
-    return M > 16 && weights >= 32000000;
+    if (M > 48) return K > 2048 || N > 2048;
+    if (M > 32) return weights >= 9000000 || N >= 8192 || K >= 7168;
+    int sms = 148;
+    device_sm_count(&sms);
+    return M > 16 && ((weights >= 32000000 && N > 16 * sms) || N >= 16384);
 }
 int launch_decode_preq(const int8_t* xq, const float* absmax, const uint8_t* Wp, const EpiParams& epi, int M, int N, int K, int32_t* status,
                        cudaStream_t st) {

@@ -1,6 +1,6 @@
 // Decode GEMV on the warp-level int8 MMA: Y[m,n] = (sum_k Q(x)[m,k]*Wq[n,k]) * (absmax[m]/127) * gamma.  Up to 8 tokens that fit
-// in shared memory as one launch that quantises them itself; up to 48 tokens that arrive quantised, one launch per 32 of them
-// (more, and large matrices from 17 on, take gemm_wt.cu; the line and both sides' times are at its dispatch).
+// in shared memory as one launch that quantises them itself; up to 64 tokens that arrive quantised, one launch per 32 of them
+// (from 17 on, large matrices take gemm_wt.cu; the line and both sides' times are at launch_decode_preq).
 //
 // The call is bound by streaming W_packed once and by the 2-bit -> int8 expansion of the weights; the products themselves
 // are few.  With more than a handful of tokens the dp4a of the CUDA-core GEMV (one per token and 4 weights) outgrow the

@@ -364,11 +364,13 @@ EL_API size_t el_decode_workspace_bytes(int N);
  * quantises the tokens itself and touches no scratch; larger ones take the tensor-core kernel.  Process-wide. */
 EL_API int el_set_decode_gemv_max_tokens(int max_tokens);
 /* Tuning: calls with more tokens than the limit above and at most `max_tokens` (0..64, default 64)
- * take the warp-level int8 MMA: up to 8 tokens that fit in shared memory (8*K of about 190 KB) as one launch that quantises
+ * may take the warp-level int8 MMA: up to 8 tokens that fit in shared memory (8*K of about 190 KB) as one launch that quantises
  * the tokens itself and touches no scratch; others as the row quantiser (into xq_scratch and absmax) followed by one launch
  * per 32 tokens on the quantised tokens (longer rows a chunk of the reduction at a time), each a programmatic dependent of
- * the launch before it.  Calls with more tokens than the limit, more than 32 tokens of rows beyond 12288, and very wide
- * outputs of long rows (N beyond 82880 on 148 SMs, 17 to 32 tokens) take the tcgen05 kernel.  Process-wide. */
+ * the launch before it.  Within the limit the tcgen05 kernel takes the quantised tokens where it is the faster one: 17 to 32
+ * tokens with N >= 16384, or N*K >= 32 million and N beyond 16 features per SM (2368 on 148 SMs); 33 to 48 tokens with N*K >= 9 million,
+ * N >= 8192 or K >= 7168; 49 to 64 tokens with N or K beyond 2048.  It also takes calls with more tokens than the limit and outputs
+ * too wide for the warp-MMA kernel's sums of rows beyond 12288.  Process-wide. */
 EL_API int el_set_decode_mma_max_tokens(int max_tokens);
 /* Tuning, off by default: with `enable` != 0 the single-launch GEMV of el_linear_decode is issued as a programmatic
  * dependent launch.  It may then start while earlier work of the stream still runs; until that work has completed it

@@ -33,6 +33,21 @@ def test_every_route_gives_the_forward_pass(ops, M, K, N, dtype):
     ops.check_device_status(torch.device(DEV))
 
 
+# both sides of the lines in matrix size: 2048 outputs or inputs (49 tokens up), 9 million weights, 8192 outputs and 7168 inputs (33 to 48),
+# 16384 outputs, 32 million weights and 2368 outputs (17 to 32)
+@pytest.mark.parametrize("M,K,N", [(49, 2048, 2048), (64, 2048, 2064), (64, 2112, 100), (40, 2944, 3056), (48, 2944, 3060), (33, 256, 8200), (40, 7168, 72),
+                                   (40, 7104, 72), (17, 64, 16384), (32, 64, 16380), (24, 13568, 2368), (24, 13568, 2376), (32, 13504, 2364)])
+def test_lines_in_matrix_size(ops, M, K, N):
+    g = torch.Generator(device=DEV).manual_seed(M + K + N)
+    x = torch.randn(M, K, generator=g, device=DEV).bfloat16()
+    W = torch.randint(0, 256, (N, K // 4), generator=g, device=DEV, dtype=torch.uint8)
+    nw = torch.rand(K, generator=g, device=DEV) + 0.5
+    for w in (None, nw):
+        q, a = ops.quantize_rows(x if w is None else ops.prelinear_rows(x, None, w))
+        assert torch.equal(ops.linear_decode(x, W, 0.02, None, None, None, w), ops.matmul_rows(q, W, a, 0.02, torch.bfloat16, 1))
+    ops.check_device_status(torch.device(DEV))
+
+
 def test_calls_in_a_chain_and_under_capture(ops):
     """Each call is a programmatic dependent launch behind its quantiser: a chain of layers that feed one another, eager and replayed."""
     g = torch.Generator(device=DEV).manual_seed(3)
