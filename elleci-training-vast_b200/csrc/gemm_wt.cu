@@ -828,7 +828,9 @@ int launch_gemm_wt(int mode, const int8_t* A, const void* B, int R, int C, int D
     return launch_reduce_scale_gather(static_cast<const int*>(workspace), p.k_split, out_one, 1, 0, R, epi, R, C, st);
 }
 
-// Up to 64 tokens quantised by launch_quantize_rows_perm or launch_prelinear_quantize_perm, the launch right before this one.
+// Up to 64 tokens quantised by launch_quantize_rows_perm or launch_prelinear_quantize_perm, the launch right before this one.  No other
+// may come in between, and that one has to be an ordinary launch (see there): the first packed weights are loaded while it runs
+// (weights_first), which races with a weight update queued earlier unless that has completed before the quantiser began.
 int launch_gemm_wt_decode(const int8_t* xq, const float* absmax, const uint8_t* Wp, const EpiParams& epi, int M, int N, int K, int32_t* status,
                           cudaStream_t st) {
     if (M < 1 || M > 64) return EL_ERR_UNSUPPORTED_SHAPE;

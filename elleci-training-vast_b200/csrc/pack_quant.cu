@@ -723,6 +723,9 @@ int launch_quantize_rows(const void* x, int dt, long long ldx, int8_t* q, float*
     }
 }
 
+// An ordinary launch, and it has to stay one: its kernel lets its dependents start in its first instruction, and these (gemv_mma.cu,
+// gemm_wt.cu) read packed weights before they wait for it.  That is safe because this launch itself begins after everything
+// queued before it, a weight update among that, has completed; as a programmatic dependent it would begin earlier.
 int launch_quantize_rows_perm(const void* x, int dt, long long ldx, int8_t* q, float* a, int M, int K, float eps,
                               cudaStream_t st) {
     if (M == 0) return EL_OK;

@@ -836,7 +836,8 @@ int launch_prelinear_rows(const void* x, const void* up, int dt, long long ld, c
     return check_launch();
 }
 
-// K % 16 == 0, K <= 16384; x, up and weight rows 16-byte aligned.  At least one of `up` and `weight`.
+// K % 16 == 0, K <= 16384; x, up and weight rows 16-byte aligned.  At least one of `up` and `weight`.  Has to stay an ordinary launch,
+// for the reason given at launch_quantize_rows_perm: the kernels behind it read packed weights before they wait for it.
 int launch_prelinear_quantize_perm(const void* x, const void* up, int dt, long long ld, const float* weight, float norm_eps, int8_t* q,
                                    float* row_absmax, int M, int K, float quant_eps, cudaStream_t st) {
     if (M == 0) return EL_OK;
