@@ -125,7 +125,7 @@ def host_ops():
         module = importlib.util.module_from_spec(importlib.machinery.ModuleSpec("elleci_host_ops", loader, origin=path))
         loader.exec_module(module)
         from . import int2_tc_ops as ops
-        module.set_hooks(check, ops.device_status, ops.check_device_status, ops._decode_ws, LIB_PATH)
+        module.set_hooks(check, ops.device_status, ops.check_device_status, LIB_PATH)
         _host = module
     return _host
 

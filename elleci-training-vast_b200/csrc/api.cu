@@ -180,7 +180,7 @@ int launch_decode_preq(const int8_t* xq, const float* absmax, const uint8_t* Wp,
     return launch_gemm_wt_decode(xq, absmax, Wp, epi, M, N, K, status, st);
 }
 
-// The workspace that the decode calls ask for.  No kernel uses it any more; callers size and pass it as before.
+// The workspace that the decode calls used to need.  No kernel reads or writes it; callers may size and pass it as before, or none.
 static size_t decode_workspace_bytes(int N) { return ((size_t)64 * (size_t)N + 4 * ((size_t)(N + 127) / 128)) * sizeof(int); }
 
 }  // namespace el
@@ -563,8 +563,8 @@ int el_linear_decode(const void* x, int x_dtype, const uint8_t* W_packed, void* 
     if (M < 0 || N < 0 || K < 0 || !float_dtype(x_dtype) || !float_dtype(out_dtype)) return EL_ERR_INVALID_ARG;
     if (M == 0 || N == 0) return EL_OK;
     if (M > 64 || K == 0 || K % 64 != 0) return EL_ERR_UNSUPPORTED_SHAPE;
-    if (!x || !W_packed || !Y || !xq_scratch || !absmax || !workspace) return EL_ERR_NULL_PTR;
-    if (workspace_bytes < decode_workspace_bytes(N)) return EL_ERR_INVALID_ARG;
+    if (!x || !W_packed || !Y || !xq_scratch || !absmax) return EL_ERR_NULL_PTR;
+    if (workspace && workspace_bytes < decode_workspace_bytes(N)) return EL_ERR_INVALID_ARG;
     if (M <= decode_gemv_max_tokens()) {      // a handful of tokens: one CUDA-core launch, no scratch touched
         const EpiParams gepi{Y, (long long)N, out_dtype, nullptr, 0, gamma};
         return launch_gemv_small(x, x_dtype, W_packed, gepi, M, N, K, (cudaStream_t)stream, decode_overlap());
@@ -586,8 +586,8 @@ int el_prelinear_decode(const void* x, const void* up, int x_dtype, long long ld
     if (M < 0 || N < 0 || K < 0 || !float_dtype(x_dtype) || !float_dtype(out_dtype) || ld < K || (!up && !norm_weight)) return EL_ERR_INVALID_ARG;
     if (M == 0 || N == 0) return EL_OK;
     if (M > 64 || K == 0 || K % 64 != 0 || K > 16384) return EL_ERR_UNSUPPORTED_SHAPE;
-    if (!x || !W_packed || !Y || !xq_scratch || !absmax || !workspace) return EL_ERR_NULL_PTR;
-    if (workspace_bytes < decode_workspace_bytes(N)) return EL_ERR_INVALID_ARG;
+    if (!x || !W_packed || !Y || !xq_scratch || !absmax) return EL_ERR_NULL_PTR;
+    if (workspace && workspace_bytes < decode_workspace_bytes(N)) return EL_ERR_INVALID_ARG;
     int rc = require_sm100();
     if (rc != EL_OK) return rc;
     rc = launch_prelinear_quantize_perm(x, up, x_dtype, ld, norm_weight, norm_eps, xq_scratch, absmax, M, K, 1e-5f, (cudaStream_t)stream);

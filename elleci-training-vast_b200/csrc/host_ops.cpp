@@ -6,9 +6,8 @@
 // Host time of a pass through the module API, before -> now: training step of that layer 275 -> 145 us, decode of one token 57 -> 19 us,
 // feed-forward block with 4 tokens 177 -> 56 us.
 //
-// No state of its own but the handles that set_hooks hands over: the status word of each device, the decode workspaces
-// (a dict of the Python module, keyed by device, stream and width), the function that turns a status into an exception and
-// the one that checks the device's status word.  Scratch that a call needs and leaves is allocated per call.
+// No state of its own but the handles that set_hooks hands over: the status word of each device, the function that turns a status
+// into an exception and the one that checks the device's status word.  Scratch that a call needs and leaves is allocated per call.
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Dtype.h>
@@ -28,7 +27,6 @@ using at::Tensor;
 PyObject* g_check = nullptr;            // _lib.check(name, status): raises ElleciError
 PyObject* g_status_of = nullptr;        // int2_tc_ops.device_status(device) -> int32 tensor
 PyObject* g_check_status = nullptr;     // int2_tc_ops.check_device_status(device)
-PyObject* g_decode_ws = nullptr;        // dict (device index, stream, N) -> workspace tensor
 
 // The library's entry points, taken from the very file that the Python binding has loaded.
 #define EL_FUNCTIONS(X)                                                                                                   \
@@ -549,25 +547,6 @@ PyObject* weight_update(PyObject* const* a) {
 }
 
 // ---- decode -------------------------------------------------------------------------------------------------------------
-// Cached per device, stream and N: calls that share a workspace must be stream-ordered.
-Tensor decode_workspace(const Tensor& x, void* st, int64_t N, size_t need) {
-    PyObject* key = Py_BuildValue("(iKL)", (int)x.device().index(), (unsigned long long)(uintptr_t)st, (long long)N);
-    if (key == nullptr) throw PyError();
-    PyObject* hit = PyDict_GetItemWithError(g_decode_ws, key);
-    Tensor ws;
-    if (hit != nullptr) {
-        ws = THPVariable_Unpack(hit);
-    } else if (!PyErr_Occurred()) {
-        ws = at::zeros({(int64_t)need}, at::TensorOptions().device(x.device()).dtype(at::kByte));
-        PyObject* t = wrap(ws);
-        if (t != nullptr) PyDict_SetItem(g_decode_ws, key, t);
-        Py_XDECREF(t);
-    }
-    Py_DECREF(key);
-    if (PyErr_Occurred()) throw PyError();
-    return ws;
-}
-
 // linear_decode(x, W_packed, gamma, out_dtype, workspace, up, norm_weight, norm_eps)
 PyObject* linear_decode(PyObject* const* a) {
     const Tensor &x = cuda_arg(a[0], "x"), &W = cuda_arg(a[1], "W_packed");
@@ -599,11 +578,14 @@ PyObject* linear_decode(PyObject* const* a) {
     const void *xp = ptr(v.t), *up_p = ptr(u.t);
     const float* nwp = ptr<float>(w);
     const uint8_t* wp = ptr<uint8_t>(Wc);
-    const size_t need = g_lib.el_decode_workspace_bytes((int)N);
     void* st = stream();
-    Tensor ws = is_none(a[4]) ? decode_workspace(x, st, N, need) : tensor_arg(a[4], "workspace");
-    const size_t have = (size_t)ws.numel() * ws.element_size();
-    EL_REQUIRE(ws.is_cuda() && have >= need, "workspace too small");
+    Tensor ws;                      // the kernels need none; what a caller passes has to be large enough all the same
+    size_t have = 0;
+    if (!is_none(a[4])) {
+        ws = tensor_arg(a[4], "workspace");
+        have = (size_t)ws.numel() * ws.element_size();
+        EL_REQUIRE(ws.is_cuda() && have >= g_lib.el_decode_workspace_bytes((int)N), "workspace too small");
+    }
     // one allocation for the quantised tokens and, on a 16-byte boundary behind them, their maxima
     const int64_t xq_bytes = (M * K + 15) & ~(int64_t)15;
     Tensor scratch = new_empty(x, {xq_bytes + M * 4}, at::kByte), Y = like_rows(x, N, out_dt);
@@ -635,9 +617,9 @@ PyObject* entry(PyObject*, PyObject* const* args, Py_ssize_t n) {
     END_HANDLE_TH_ERRORS
 }
 
-// set_hooks(check, device_status, check_device_status, decode workspaces, path of the loaded library)
+// set_hooks(check, device_status, check_device_status, path of the loaded library)
 PyObject* set_hooks(PyObject* const* a) {
-    const char* path = PyUnicode_AsUTF8(a[4]);
+    const char* path = PyUnicode_AsUTF8(a[3]);
     if (path == nullptr) throw PyError();
     void* handle = dlopen(path, RTLD_NOW | RTLD_NOLOAD);
     EL_REQUIRE(handle != nullptr, "the library is not loaded");
@@ -646,8 +628,8 @@ PyObject* set_hooks(PyObject* const* a) {
     EL_FUNCTIONS(X)
 #undef X
     EL_REQUIRE(all, "the library lacks an entry point");
-    PyObject** dst[] = {&g_check, &g_status_of, &g_check_status, &g_decode_ws};
-    for (int i = 0; i < 4; ++i) {
+    PyObject** dst[] = {&g_check, &g_status_of, &g_check_status};
+    for (int i = 0; i < 3; ++i) {
         Py_INCREF(a[i]);
         Py_XSETREF(*dst[i], a[i]);
     }
@@ -658,7 +640,7 @@ PyObject* set_hooks(PyObject* const* a) {
 PyMethodDef methods[] = {
     EL_ENTRY(quantize_rows, 5), EL_ENTRY(quantize_grad, 3), EL_ENTRY(quantize_tensor, 2), EL_ENTRY(rmsnorm_quantize_rows, 4),
     EL_ENTRY(rmsnorm_backward, 4), EL_ENTRY(swiglu_quantize_rows, 5), EL_ENTRY(swiglu_backward, 6), EL_ENTRY(prelinear_rows, 4),
-    EL_ENTRY(gemm_fwd, 7), EL_ENTRY(gemm_dx, 8), EL_ENTRY(dw_hysteresis, 11), EL_ENTRY(weight_update, 13), EL_ENTRY(linear_decode, 8), EL_ENTRY(set_hooks, 5),
+    EL_ENTRY(gemm_fwd, 7), EL_ENTRY(gemm_dx, 8), EL_ENTRY(dw_hysteresis, 11), EL_ENTRY(weight_update, 13), EL_ENTRY(linear_decode, 8), EL_ENTRY(set_hooks, 4),
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "elleci_host_ops", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 

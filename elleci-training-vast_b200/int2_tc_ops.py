@@ -55,15 +55,10 @@ def device_status(device: torch.device) -> torch.Tensor:
 
 
 def check_device_status(device: torch.device) -> None:
-    """Synchronises and raises if a tensor-core kernel reported a failed wait.  A kernel that gave up may have left
-    partial sums in a decode workspace, which every call expects to find zeroed: the cached workspaces of the device are
-    dropped, so the next decode call starts from a fresh zeroed one."""
+    """Synchronises and raises if a tensor-core kernel reported a failed wait; the next call starts from a cleared status word."""
     code = int(device_status(device).item())
     if code != 0:
         device_status(device).zero_()
-        index = device.index if device.index is not None else torch.cuda.current_device()
-        for key in [k for k in _decode_ws if k[0] == index]:
-            del _decode_ws[key]
         raise ElleciError("tensor-core kernel", code, f"a bounded barrier wait gave up (code {code})")
 
 
@@ -495,15 +490,15 @@ def weight_update(dY: torch.Tensor, x_absmax: torch.Tensor, Xq: torch.Tensor, W_
                                     int(step) & 0xFFFFFFFF, int(idx_base) & 0xFFFFFFFF, g_absmax)
 
 
-_decode_ws: dict = {}
+_decode_ws: dict = {}        # workspaces of decode calls: none needs one any more, so it stays empty
 
 
 def linear_decode(x: torch.Tensor, W_packed: torch.Tensor, gamma: float, out_dtype: Optional[torch.dtype] = None,
                   workspace: Optional[torch.Tensor] = None, up: Optional[torch.Tensor] = None,
                   norm_weight: Optional[torch.Tensor] = None, norm_eps: float = NORM_EPS) -> torch.Tensor:
-    """Small-M layer call (1 <= M <= 64 tokens): per-token quantisation + the weight-streaming tensor-core kernel.
-    Same integers and rounding as quantize_rows + matmul_rows.  `workspace` (uint8, zero before first use, left
-    zero) defaults to a cached buffer per device, stream and N, so calls on different streams never share one.
+    """Small-M layer call (1 <= M <= 64 tokens): per-token quantisation + a weight-streaming kernel (CUDA cores, warp MMA or
+    tcgen05, by tokens and size).  Same integers and rounding as quantize_rows + matmul_rows.  `workspace` is not needed: it is
+    neither read nor written, only its size (el_decode_workspace_bytes) is checked if it is given.
     `up` and `norm_weight` as in prelinear_rows (K <= 16384): the layer input is formed from x first, without a tensor for it."""
     return host_ops().linear_decode(x, W_packed, gamma, out_dtype, workspace, up, norm_weight, norm_eps)
 

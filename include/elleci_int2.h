@@ -354,9 +354,8 @@ EL_API int el_dw_hysteresis_step_ptr(const int8_t* Gq, const int8_t* Xq, const f
 /* Y[m,n] = out_dtype( float(sum_k Q(x)[m,k]*Wq[n,k]) * ((absmax[m]/127) * gamma) ) for 1 <= M <= 64 tokens: per-token
  * quantisation of x followed by a weight-streaming kernel (CUDA cores, warp MMA or tcgen05, by tokens and size), the
  * same integers and the same rounding as el_quantize_rows + el_gemm_fwd.  Needs K % 64 == 0 and 16-byte aligned x,
- * W_packed, xq_scratch and workspace.  Caller-owned scratch: xq_scratch int8 [M,K] and absmax float [M] (overwritten),
- * and `workspace` of el_decode_workspace_bytes(N) bytes, which earlier versions kept partial sums in: it has to be given, and
- * is neither read nor written.  Replaces the scalar kernel the reference falls back to when M < 64
+ * W_packed and xq_scratch.  Caller-owned scratch: xq_scratch int8 [M,K] and absmax float [M] (overwritten).  `workspace`, which
+ * earlier versions kept partial sums in, is neither read nor written: NULL, or el_decode_workspace_bytes(N) bytes.  Replaces the scalar kernel the reference falls back to when M < 64
  * (int2_matmul_int8_tc_v2_simple_kernel, kernels/int2/int2_matmul_int8_tc_v2.cu:452-473, dispatch :511-536), the
  * path of Elleci.generate (model/model.py:505-623). */
 EL_API size_t el_decode_workspace_bytes(int N);

@@ -92,3 +92,23 @@ def test_decode_from_several_threads_on_their_own_streams(pkg, M, K, norm):
         t.join(timeout=120)
     assert not errors and wrong == [0] * threads, (errors, wrong)
     o.check_device_status(torch.device("cuda", torch.cuda.current_device()))
+
+
+@pytest.mark.parametrize("M,norm", [(1, False), (5, True), (24, False), (64, False), (64, True)])
+def test_decode_keeps_no_memory_and_needs_no_workspace(pkg, M, norm):
+    """A stream's first decode call holds nothing once its output is gone; a workspace that is given is still checked for its size."""
+    o, N, K = pkg.int2_tc_ops, 4096, 256
+    x, W = torch.randn(M, K, device="cuda"), torch.randint(0, 256, (N, K // 4), device="cuda", dtype=torch.uint8)
+    w = torch.ones(K, device="cuda") if norm else None
+    need = pkg._lib.lib().el_decode_workspace_bytes(N)
+    want = o.linear_decode(x, W, 0.01, workspace=torch.zeros(need, device="cuda", dtype=torch.uint8), norm_weight=w)
+    with pytest.raises(RuntimeError, match="workspace too small"):
+        o.linear_decode(x, W, 0.01, workspace=torch.zeros(need - 1, device="cuda", dtype=torch.uint8), norm_weight=w)
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    with torch.cuda.stream(torch.cuda.Stream()):
+        y = o.linear_decode(x, W, 0.01, norm_weight=w)
+        torch.cuda.synchronize()
+        assert torch.equal(y, want)
+        del y
+    assert torch.cuda.memory_allocated() == before
