@@ -52,3 +52,30 @@ def test_several_tiles_per_pair(ops, pkg, M, N, K):
 @pytest.mark.parametrize("M,N,K", [(20, 512, 40000), (60, 400, 40064), (128, 640, 40000), (2500, 1536, 4096), (5000, 256, 8256)])
 def test_several_tiles_per_pair_dx(ops, pkg, M, N, K):
     _check(ops, pkg, M, N, K, True)
+
+
+# Scaled outputs of sums up to the edge of 2^22 and beyond: tokens of -128 against weights of one sign, reductions of up to 32767 (the sums are
+# converted by an addition) and from 32768 on (by the conversion unit); some rows of ordinary tokens between them.
+@pytest.mark.parametrize("D", [32704, 32752, 32768, 65536])
+@pytest.mark.parametrize("dx", [False, True])
+@pytest.mark.parametrize("M", [40, 300])
+@pytest.mark.parametrize("byte", [0x00, 0xAA])       # all weights -1, all +1
+def test_large_sums(ops, pkg, D, dx, M, byte):
+    if not dx and D % 64:
+        pytest.skip("the forward reduction is a multiple of 64")
+    g = torch.Generator(device=DEV).manual_seed(D + M)
+    C = 192
+    W = torch.full((D, C // 4) if dx else (C, D // 4), byte, device=DEV, dtype=torch.uint8)
+    a = torch.rand(M, generator=g, device=DEV) + 0.5
+    q = torch.full((M, D), -128, device=DEV, dtype=torch.int8)
+    q[::3] = torch.randint(-128, 128, q[::3].shape, generator=g, device=DEV, dtype=torch.int8)
+
+    def call(dtype, path):
+        return ops.backward_input_rows(q, W, a, 0.02, C, dtype, path) if dx else ops.matmul_rows(q, W, a, 0.02, dtype, path)
+
+    assert int(call(torch.int32, pkg._lib.EL_PATH_SIMPLE).abs().max()) == 128 * D
+    for dtype in (torch.bfloat16, torch.float32):
+        want = call(dtype, pkg._lib.EL_PATH_SIMPLE)
+        for path in (pkg._lib.EL_PATH_TC, pkg._lib.EL_PATH_TC | pkg._lib.EL_FLAG_LEAN):
+            assert torch.equal(call(dtype, path), want), (dtype, path)
+    ops.check_device_status(torch.device(DEV))
