@@ -76,7 +76,6 @@ __device__ __forceinline__ void decode16_deint(uint32_t x, uint32_t out[4]) {
 }
 
 // ---- float helpers ----------------------------------------------------------------------------------------
-__device__ __forceinline__ float ftz32(float x) { return fabsf(x) < 1.17549435e-38f ? 0.0f : x; }
 __host__ inline float ftz32_host(float x) {
     return (x < 1.17549435e-38f && x > -1.17549435e-38f) ? 0.0f : x;
 }

@@ -79,14 +79,6 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
         : "memory");
 }
 
-// Asks for a tile to be brought into L2 without a shared-memory destination or a barrier: a kernel that streams a
-// matrix once can request all of its tiles up front, far deeper than its shared-memory ring could hold them.
-__device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* map, int x, int y) {
-    asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];"
-                 ::"l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y)
-                 : "memory");
-}
-
 // Waits until the launch that this one is a programmatic dependent of has completed and its writes are visible; nothing where there is none.
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
@@ -115,15 +107,6 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
           "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]),
           "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]),
           "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-        : "r"(taddr)
-        : "memory");
-}
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-          "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
         : "r"(taddr)
         : "memory");
 }
@@ -168,22 +151,8 @@ __device__ __forceinline__ uint32_t mapa_u32(uint32_t addr, uint32_t rank) {
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
     return r;
 }
-// Arrive on a barrier given by its cluster-wide address; works for the own CTA too.  The waiter may be in the other CTA, so the
-// release has cluster scope (the instruction's default covers the own CTA only).
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
-// The same, announcing only what this thread (and its warp, after __syncwarp) has written to its own shared memory: the fence
-// releases those writes at cluster scope and the arrival itself orders nothing.  A full release waits until all earlier memory
-// operations of the thread are visible to the cluster, the packed weights of its NEXT block still on their way from L2 among them.
-// Pair GEMM, 4096 tokens 4096 -> 11008 with one arrival per expanded block: a full release 149 us forward, 157 us dX (with the loads
-// issued after the arrival, 156 / 169 before it), this form 138 / 142 us.
-__device__ __forceinline__ void mbar_arrive_cluster_smem(uint32_t cluster_addr) {
-    asm volatile("fence.release.sync_restrict::shared::cta.cluster;\n\t"
-                 "mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
-// The same with nothing to release: for a thread whose own accesses were to tensor memory only, ordered by tcgen05.wait and
-// tcgen05.fence::before_thread_sync.
+// Arrive on a barrier given by its cluster-wide address (the own CTA's too), with nothing to release: for a thread whose own accesses
+// were to tensor memory only, ordered by tcgen05.wait and tcgen05.fence::before_thread_sync.
 __device__ __forceinline__ void mbar_arrive_cluster_relaxed(uint32_t cluster_addr) {
     asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
