@@ -1081,12 +1081,12 @@ def run_decode(args):
         del sgraph, dst
         # overlap: the GEMV issued as a programmatic dependent launch (weights constant, as at inference), so that a
         # call's weight loads start under the tail of the previous call
-        # columns: tokens, limit of the CUDA-core GEMV, limit of the warp-MMA kernel (tcgen05 stream-K above it), overlap
+        # columns: tokens, limit of the CUDA-core GEMV, limit of the warp-MMA kernel (tcgen05 above it), overlap.  Matrices of this
+        # size take the tcgen05 kernel from 17 tokens on, whatever that limit.
         for M, gemv_max, mma_max, overlap in ((1, 1, 64, False), (1, 1, 64, True), (1, 0, 64, True), (2, 2, 64, True),
                                               (2, 1, 64, True), (4, 4, 64, True), (4, 1, 64, False), (4, 1, 64, True),
                                               (8, 8, 64, True), (8, 1, 64, False), (8, 1, 64, True), (8, 0, 0, False),
-                                              (16, 1, 64, True), (16, 0, 0, False), (32, 1, 64, True), (32, 1, 0, False),
-                                              (64, 1, 64, False), (64, 1, 0, False)):
+                                              (16, 1, 64, True), (16, 0, 0, False), (32, 1, 64, True), (64, 1, 64, False)):
             pkg._lib.lib().el_set_decode_gemv_max_tokens(gemv_max)
             pkg._lib.lib().el_set_decode_mma_max_tokens(mma_max)
             ops.set_decode_overlap(overlap)
@@ -1112,7 +1112,7 @@ def run_decode(args):
             nbytes = N * K // 4 + 2 * M * K + 2 * M * N
             gbs = nbytes / (us * 1e-6) / 1e9
             mt = 8 if M <= 8 else (16 if M <= 16 else 32)      # tokens per launch of the warp-MMA kernel, padded
-            fits_mma = M <= mma_max and 256 + ((K + 255) // 256) * 16 * mt * 16 + 2 * 16 * mt * 4 <= 200 * 1024
+            fits_mma = M <= min(mma_max, 16) and 256 + ((K + 255) // 256) * 16 * mt * 16 + 2 * 16 * mt * 4 <= 200 * 1024
             kernel = "gemv" if M <= gemv_max else (("mma" if M <= 8 else "mma_preq") if fits_mma else "tcgen05")
             cases.append({"M": M, "K": K, "N": N, "kernel": kernel, "overlap": overlap, "us_per_call": us, "GBps": gbs, "frac_of_hbm": gbs / peaks["hbm_gbs"],
                           "algorithmic_bytes": nbytes})
