@@ -200,7 +200,7 @@ class TokenParallelInt2Linear(nn.Module):
         # How the pushes that run on a side stream beside the GEMMs move their bytes.  push_ctas > 0: a peer-store kernel of
         # that many CTAs.  It holds no shared memory, so it sits on the SMs next to the GEMM's CTAs; NVLink needs a few
         # megabytes of stores in flight to run at rate (32 CTAs moved 140-310 GB/s, a fifth of the link), and one CTA per
-        # SM is the most that fits: the register-lean GEMM leaves 16 K registers per SM, a push CTA takes 12 K, and with
+        # SM is the most that fits: the register-lean GEMM leaves 19 K registers per SM, a push CTA takes 12 K, and with
         # two per SM a GEMM CTA that arrives second finds no room and waits for the whole push.  push_ctas < 0: the copy
         # engines, one copy per destination (el_peer_put_dma): no SM takes part and the GEMM beside it keeps its faster
         # form, but the copies run one after the other at about 10 us each plus their bytes.  0 (default): by size -

@@ -391,13 +391,14 @@ EL_API int el_prelinear_decode(const void* x, const void* up, int x_dtype, long 
 
 /* el_linear_decode for callers that cannot give the library any device memory (no counterpart in the reference).
  * Serving processes that forbid cudaMalloc after start-up, runtimes that own the whole memory pool and hosts at
- * their memory budget cannot supply the scratch buffers of el_linear_decode; here the quantised tokens, their
+ * their memory budget cannot supply the scratch buffers of el_linear_decode; here the quantised tokens and their
  * scales live in one static device array inside the library (one megabyte, held by
  * every GPU that loads the library until the process exits).  The caller passes only x [M,K], W_packed and Y [M,N].
  * Limits: M <= 64, N <= 16384, K <= 16384, K % 64 == 0; larger sizes return EL_ERR_TOO_LARGE.  Same results as
  * el_linear_decode.  The call makes no cudaMalloc / cudaFree and uses no allocating library routine.
  * The first call on a device resolves the array's address (cudaGetSymbolAddress): make that first call with the
- * device current and before any stream capture.  All calls on a device share the one array.  Two calls whose GPU work overlaps (different streams, or threads) race on it: order them. */
+ * device current and before any stream capture.  All calls on a device share the one array.  Two calls whose GPU work
+ * overlaps (different streams, or threads) race on it: order them. */
 EL_API int el_linear_decode_static(const void* x, int x_dtype, const uint8_t* W_packed, void* Y, int out_dtype, float gamma,
                                    int M, int N, int K, int32_t* dev_status, el_stream_t stream);
 
